@@ -32,6 +32,7 @@
 #include "hp2d_fused.cuh"
 #include "hp2d_unfused.cuh"
 #include "hp2d_tb.cuh"
+#include "hp2d_tile.cuh"
 
 using namespace hp2d;
 
@@ -337,9 +338,18 @@ template <typename R> struct Impl : Base {
     RecordDesc<R> rec{};
     Dev<float> maps;
     RainDesc rain{};
-    Dev<StepScalars> sc;
+    // the launches' scalars (slot 0 is the host's; a batch's launches alternate), the steps' rain and
+    // sums (see StepAcc), and a sum for stored_volume: one allocation
+    struct Control {
+        StepScalars sc[2];
+        StepPrep<R> prep[2];
+        StepAcc acc[4];
+        double vol;
+    };
+    Dev<Control> ctl;
+    struct { StepScalars* p = nullptr; } sc;
+    struct { double* p = nullptr; } vol;
     StepScalars hs{};
-    Dev<double> vol;
     // host copies needed to rebuild records
     std::vector<uint32_t, NoInitAlloc<uint32_t>> host_meta;   // meta word per cell (host mirror)
     std::vector<uint8_t> host_soil;
@@ -380,6 +390,26 @@ template <typename R> struct Impl : Base {
         return best;
     }
     int cells_per_lane = 1;   // fused-step layout: 1 (32-column strips) or 2 (64-column strips)
+    // The tile step (hp2d_tile.cuh) instead of strips: -1 by the grid, 0 off (a layout or rows per warp
+    // were chosen), 1 or 2 rows per thread (chosen by hp2d_autotune).
+    int tile_mode = -1;
+    static constexpr unsigned int kWaitPolls = 1u << 22;
+    // rows per thread of the tile step, 0 for strips
+    int tile_rpt() const {
+        if (wait_polls != kWaitPolls) return 0;   // the caller bounds the row copies that strips have
+        if (tile_mode >= 0) return tile_mode;
+        // Up to where the tiles measured faster than the strips, us per step, strips / tiles.  FP32:
+        // 1000^2 56 / 29 wet, 54 / 22 valley, 103 / 50 Green-Ampt and rain maps; 1300^2 59 / 47, 58 / 30,
+        // 108 / 83; 1700^2 80 / 81, 80 / 51, 155 / 133; 2048^2 99 / 118, -, 203 / 200.  FP64: 1700^2 Green-Ampt
+        // and maps 291 / 259, wet 189 / 160.
+        const size_t most = sizeof(R) == 8 ? 4000000 : (inf_mode() || rain.n_maps) ? 4300000 : 2500000;
+        if (n > most) return 0;
+        // one row per thread while the grid gives the GPU little more than one wave of tiles (256^2 wet
+        // FP32 6.5 / 7.4 us with one / two rows, 400^2 9.7 / 9.5; FP64 Green-Ampt 600^2 43 / 46,
+        // 1000^2 103 / 103)
+        return n > (sizeof(R) == 8 ? 1000000u : 200000u) ? 2 : 1;
+    }
+    bool tile_on() const { return tile_rpt() != 0; }
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
 
@@ -395,8 +425,10 @@ template <typename R> struct Impl : Base {
         stat.alloc(n);
         for (int b = 0; b < 2; ++b) st4[b].alloc(n);
         arrival.alloc(n);
-        sc.alloc(1);
-        vol.alloc(1);
+        ctl.alloc(1);
+        HP_CK(cudaMemsetAsync(ctl.p, 0, sizeof(Control), ctx->stream));
+        sc.p = &ctl.p->sc[0];
+        vol.p = &ctl.p->vol;
         bit_words = (nx + 31) / 32;
         host_meta.resize(n);
         host_parallel(n, [&](size_t a, size_t b) { std::fill(host_meta.begin() + a, host_meta.begin() + b, 255u); });
@@ -1298,6 +1330,11 @@ template <typename R> struct Impl : Base {
         a.t_end = p.routing_time + p.min_time_step / 60.0;
         a.min_dt = p.min_time_step; a.max_dt = p.max_time_step; a.inc = p.time_step_increments;
         a.tsc = p.time_step_change; a.alfa_min = p.alfa_min; a.alfa_max = p.alfa_max;
+        a.inv_inc = 1.0 / a.inc; a.inv_tsc = 1.0 / a.tsc; a.inv_res = 1.0 / a.res;
+        a.map_sy = R(double(rain.my) / ny);
+        a.map_sx = R(double(rain.mx) / nx);
+        a.k_const[0] = R(a.inv_res); a.k_const[1] = R(kG); a.k_const[2] = R(a.tol_mm / 1000.0);
+        a.k_const[3] = R(a.thr_mm / 1000.0);
         a.flag_timestep = p.flag_timestep; a.adaptive = p.flag_adaptive_timestepping;
         a.flag_critical = p.flag_critical; a.outlet_type = p.outlet_type; a.ga = ga() ? 1 : 0;
         a.scheme = p.flag_numerical_scheme;
@@ -1326,9 +1363,23 @@ template <typename R> struct Impl : Base {
         a.strct = strct;
         a.dry_rows = dry_rows();
         a.dryflag = dry_usable(rpw) && tb_chosen <= 1 && !slab() ? dryf.p : nullptr;
+        a.tile_nx = 0;
+        if (tile_on()) {
+            if (!n_sms) HP_CK(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, ctx->device));
+            using T1 = TileShape<R, 1>;
+            using T2 = TileShape<R, 2>;
+            a.tile_rpt = tile_rpt();
+            const int rows = a.tile_rpt == 2 ? T2::OR : T1::OR;
+            a.tile_nx = (nx + T1::OC - 1) / T1::OC;
+            a.tile_grid = unsigned(n_sms * (a.tile_rpt == 2 ? T2::MINB : T1::MINB));
+            a.n_ctas = unsigned(a.tile_nx * ((ny + rows - 1) / rows));
+            a.dryflag = dry_enabled && tb_chosen <= 1 && !slab() ? dryf.p : nullptr;
+        }
         a.vmax = hz_on ? vmaxm.p : nullptr;
         a.hzmax = hz_on ? hzmaxm.p : nullptr;
         a.sc = sc.p;
+        a.prep = &ctl.p->prep[0];
+        a.acc = &ctl.p->acc[0];
         return a;
     }
 
@@ -1359,32 +1410,62 @@ template <typename R> struct Impl : Base {
     template <int CPL> void opt_in_t() { opt_in_i<0, CPL>(); opt_in_i<1, CPL>(); opt_in_i<2, CPL>(); }
     void opt_in() { opt_in_t<1>(); opt_in_t<2>(); }
 
-    template <int INF, bool MAP, int CPL, bool INFL, int SCH = 0> void launch_one(const FusedArgs<R>& a) {
+    template <int INF, bool MAP, int CPL, bool INFL, int SCH = 0> void launch_one(const FusedArgs<R>& a, int phase) {
         const size_t sm = fused_smem_bytes<R, CPL>(kThreads);
-        k_fused_step<R, kThreads, INF, MAP, CPL, INFL, SCH><<<a.n_ctas, kThreads, sm, st()>>>(a);
+        launch_step(k_fused_step<R, kThreads, INF, MAP, CPL, INFL, SCH>, a.n_ctas, kThreads, sm, st(), a, phase);
     }
-    template <int INF, int CPL> void launch_i(const FusedArgs<R>& a) {
+    template <int INF, int CPL> void launch_i(const FusedArgs<R>& a, int phase) {
         const bool map = rain.n_maps > 0, infl = bc_kernel();
         if (ctx->p.flag_numerical_scheme != 1) {   // schemes 2/3: the general (boundary-cell) variant
-            if (map) launch_one<INF, true, CPL, true, 1>(a); else launch_one<INF, false, CPL, true, 1>(a);
+            if (map) launch_one<INF, true, CPL, true, 1>(a, phase); else launch_one<INF, false, CPL, true, 1>(a, phase);
             return;
         }
         if (map) {
-            if (infl) launch_one<INF, true, CPL, true>(a); else launch_one<INF, true, CPL, false>(a);
+            if (infl) launch_one<INF, true, CPL, true>(a, phase); else launch_one<INF, true, CPL, false>(a, phase);
         } else {
-            if (infl) launch_one<INF, false, CPL, true>(a); else launch_one<INF, false, CPL, false>(a);
+            if (infl) launch_one<INF, false, CPL, true>(a, phase); else launch_one<INF, false, CPL, false>(a, phase);
         }
     }
-    template <int CPL> void launch_fused_t(const FusedArgs<R>& a) {
+    template <int CPL> void launch_fused_t(const FusedArgs<R>& a, int phase) {
         switch (inf_mode()) {
-            case 1: launch_i<1, CPL>(a); break;
-            case 2: launch_i<2, CPL>(a); break;
-            default: launch_i<0, CPL>(a);
+            case 1: launch_i<1, CPL>(a, phase); break;
+            case 2: launch_i<2, CPL>(a, phase); break;
+            default: launch_i<0, CPL>(a, phase);
         }
     }
-    void launch_fused(const FusedArgs<R>& a) {
-        if (cells_per_lane == 2) launch_fused_t<2>(a);
-        else launch_fused_t<1>(a);
+    // one step; `phase` is its number in the batch modulo 4 (0 after a flush)
+    void launch_fused(const FusedArgs<R>& a, int phase) {
+        if (a.tile_nx) {
+            launch_tile_step<R>(a, inf_mode(), rain.n_maps > 0, bc_kernel(), ctx->p.flag_numerical_scheme != 1,
+                                phase, st());
+            return;
+        }
+        if (cells_per_lane == 2) launch_fused_t<2>(a, phase);
+        else launch_fused_t<1>(a, phase);
+    }
+
+    // ends the step pending after `launched` steps since the last flush
+    template <int INF> void flush_i(const FusedArgs<R>& a, int phase) {
+        if (rain.n_maps > 0) k_step_flush<R, INF, true><<<1, 128, 0, st()>>>(a, phase);
+        else k_step_flush<R, INF, false><<<1, 128, 0, st()>>>(a, phase);
+    }
+    void launch_flush(const FusedArgs<R>& a, int64_t launched) {
+        const int phase = int(launched & 3);
+        switch (inf_mode()) {
+            case 1: flush_i<1>(a, phase); break;
+            case 2: flush_i<2>(a, phase); break;
+            default: flush_i<0>(a, phase);
+        }
+    }
+    // `count` steps in a row, the last one ended for the host.  Gauges, stages and control structures
+    // need the step's end before the next step's launch (its depths, stages and transfers).
+    void launch_row(const FusedArgs<R>& a, int64_t count) {
+        const bool each = a.inflow.n_gauges > 0 || a.inflow.n_stage > 0 || a.strct.n > 0;
+        for (int64_t s = 0; s < count; ++s) {
+            launch_fused(a, each ? 0 : int(s & 3));
+            if (each) launch_flush(a, 1);
+        }
+        if (!each && count > 0) launch_flush(a, count);
     }
 
     // the fused kernel variant with boundary-condition cells (inflow, stage, structures)
@@ -1439,6 +1520,7 @@ template <typename R> struct Impl : Base {
     bool dry_enabled = true;   // hp2d_set_dry_skip
     bool dry_usable(int rpw) const { return dry_enabled && rpw % 4 == 0 && rpw <= 128; }
     int dry_key(int cpl) {
+        if (const int t = tile_rpt()) return dry_enabled ? 64 * t : -64 * t;   // a flag per tile
         const int rpw = rpw_chosen ? rows_per_warp : default_rows(cpl);
         return dry_usable(rpw) ? cpl : -cpl;
     }
@@ -1456,6 +1538,7 @@ template <typename R> struct Impl : Base {
         dry_for_layout(cells_per_lane);
         if (!dirty) return;
         reset_dry();
+        HP_CK(cudaMemsetAsync(&ctl.p->prep[0], 0xff, 2 * sizeof(StepPrep<R>), st()));   // NaN keys: the first step makes its own
         pull_sc();
         hs.skip_clamp = 0;
         hs.counter = 0;
@@ -1496,7 +1579,7 @@ template <typename R> struct Impl : Base {
         if (graph) return;
         cudaGraph_t gr;
         HP_CK(cudaStreamBeginCapture(st(), cudaStreamCaptureModeThreadLocal));
-        for (int s = 0; s < kGraphChunk; ++s) launch_fused(a);
+        launch_row(a, kGraphChunk);
         HP_CK(cudaStreamEndCapture(st(), &gr));
         HP_CK(cudaGraphInstantiate(&graph, gr, 0));
         HP_CK(cudaGraphDestroy(gr));
@@ -1513,7 +1596,7 @@ template <typename R> struct Impl : Base {
                 remaining -= graph_steps;
             }
         }
-        for (int64_t s = 0; s < remaining; ++s) launch_fused(a);
+        launch_row(a, remaining);
         HP_CK(cudaGetLastError());
     }
 
@@ -1699,7 +1782,7 @@ template <typename R> struct Impl : Base {
                     tb_launch(a, K);
                     k += K;
                 } else {
-                    launch_fused(a);
+                    launch_row(a, 1);
                     k += 1;
                 }
             }
@@ -1720,7 +1803,7 @@ template <typename R> struct Impl : Base {
     // ---------------- failure handling (HydroPol2D_Main_While.m:926-993) ----------------
     int max_retries = 8;              // attempts of one step rejected before the call fails
     double factor_reduction = 2.0;    // running_control.factor_reduction (input_data_script.m:486)
-    unsigned int wait_polls = 1u << 22;
+    unsigned int wait_polls = kWaitPolls;
     int64_t rej_k = -1;               // step whose attempts were rejected last, and how often
     int rej_n = 0;
 
@@ -1892,7 +1975,7 @@ template <typename R> struct Impl : Base {
         }
         copy_dev(arrival.p, s.arr.p, n);
         if (n_out) { copy_dev(hf3.p, s.hf3s.p, n_out); copy_dev(qo.p, s.qos.p, n_out); }
-        copy_dev(sc.p, s.scs.p, 1);
+        copy_dev(sc.p, s.scs.p, 1);   // after a flush: nothing pending
         reset_dry();
         HP_CK(cudaStreamSynchronize(st()));
         pull_sc();
@@ -1910,6 +1993,7 @@ template <typename R> struct Impl : Base {
         const int cands[] = {16, 24, 32, 40, 44, 48, 56, 64, 96, 128};
         if (!rpw_chosen) rows_per_warp = default_rows(cells_per_lane);
         rpw_chosen = true;
+        tile_mode = 0;
         const int keep = rows_per_warp, keep_cpl = cells_per_lane;
         int best = keep, best_cpl = keep_cpl;
         float best_ms = std::numeric_limits<float>::infinity();
@@ -1923,9 +2007,9 @@ template <typename R> struct Impl : Base {
             rows_per_warp = c;
             cells_per_lane = cpl;
             const FusedArgs<R> a = fused_args();
-            launch_fused(a);   // warm-up
+            launch_row(a, 1);   // warm-up
             HP_CK(cudaEventRecord(e0, st()));
-            for (int s = 0; s < trial; ++s) launch_fused(a);
+            launch_row(a, trial);
             HP_CK(cudaEventRecord(e1, st()));
             HP_CK(cudaGetLastError());
             HP_CK(cudaEventSynchronize(e1));
@@ -1936,6 +2020,23 @@ template <typename R> struct Impl : Base {
             timed_out = timed_out || (hs.status & kStatusTimeout) != 0;
             put_back(snap);
         }
+        int best_tile = 0;
+        for (int t = 1; t <= 2 && wait_polls == kWaitPolls; ++t) {   // and the tile step
+            tile_mode = t;
+            const FusedArgs<R> a = fused_args();
+            launch_row(a, 1);   // warm-up
+            HP_CK(cudaEventRecord(e0, st()));
+            launch_row(a, trial);
+            HP_CK(cudaEventRecord(e1, st()));
+            HP_CK(cudaGetLastError());
+            HP_CK(cudaEventSynchronize(e1));
+            float ms = 0;
+            HP_CK(cudaEventElapsedTime(&ms, e0, e1));
+            if (ms < best_ms) { best_ms = ms; best_tile = t; }
+            pull_sc();
+            put_back(snap);
+        }
+        tile_mode = best_tile;
         rows_per_warp = best;
         cells_per_lane = best_cpl;
         // temporal blocking left to the tuner: blocks of 2, 3 and 4 steps against single steps,
@@ -2268,6 +2369,10 @@ struct hp2d_ensemble {
             if (im.rows_per_warp != rows_per_warp || !im.rpw_chosen) {
                 im.rows_per_warp = rows_per_warp;
                 im.rpw_chosen = true;
+                im.invalidate_graph();
+            }
+            if (im.tile_mode != 0) {   // the queue's items are strips
+                im.tile_mode = 0;
                 im.invalidate_graph();
             }
             im.prologue();
@@ -2657,6 +2762,7 @@ hp2d_status hp2d_set_layout(hp2d_ctx* ctx, int32_t cells_per_lane) {
     if (cells_per_lane != 1 && cells_per_lane != 2) return HP2D_INVALID_ARG;
     return with_impl(ctx, [&](auto& m) {
         m.cells_per_lane = cells_per_lane;
+        m.tile_mode = 0;
         m.invalidate_graph();
         return HP2D_OK;
     });
@@ -2667,6 +2773,7 @@ hp2d_status hp2d_set_tuning(hp2d_ctx* ctx, int32_t rows_per_warp) {
     return with_impl(ctx, [&](auto& m) {
         m.rows_per_warp = rows_per_warp;
         m.rpw_chosen = true;
+        m.tile_mode = 0;
         m.invalidate_graph();
         return HP2D_OK;
     });

@@ -106,6 +106,17 @@ template <typename R> __device__ __forceinline__ R pow53(R x) {
     return x * (c * c);
 }
 
+// The IEEE quotient a / b by a number whose reciprocal y = 1 / b is at hand (correctly rounded):
+// a y, then twice the exact residual's correction.  After the first correction the quotient is
+// within one ulp, and by Markstein's theorem the second one rounds it correctly.  Five dependent
+// FP64 operations instead of the division's sequence, whose latency (about 35 cycles an
+// operation) a step's clock would wait for.
+__device__ __host__ __forceinline__ double div_by(double a, double b, double y) {
+    double q = a * y;
+    q = fma(fma(-b, q, a), y, q);
+    return fma(fma(-b, q, a), y, q);
+}
+
 // ---------------- per-step constants (computed in FP64, rounded once) ------------------
 template <typename R> struct StepConsts {
     R dt, gdt, dt_over_dx, dx_over_dt, inv_dt, inv_dx, g, tol, thr;
@@ -184,6 +195,19 @@ struct StepScalars {
     // slabs redoes the refresh with the maxima of all slabs (hp2d_apply_refresh)
     unsigned long long last_vbits, last_cbits;
     int last_refreshed, last_unstable;
+    // a step whose launch has run and whose end (verdict, refresh, clock) the next launch computes
+    // from its accumulators (StepAcc), and the uniform rain depth that step applied [m]
+    int pending, pad3;
+    double rain_cell;
+};
+// The sums and maxima of one step's CTAs.  Four of them rotate: launch n reads the pending step's
+// from slot n % 4, adds its own to slot (n + 1) % 4 and clears slot (n + 2) % 4.
+struct StepAcc {
+    unsigned long long vmax, cmax;   // ordered bits of max speed^2; celerity code (0 none, bits + 1)
+    double rain, inf, out, stage;    // [m] (times cell area later)
+    unsigned long long bad;          // cells ending non-finite or too negative
+    unsigned long long skipw, skipr; // records not rewritten, of those not read
+    unsigned timeout, negn;          // a row copy timed out; an outlet cell asks for the clamp skip
 };
 // StepScalars::status bits
 constexpr unsigned kStatusNumerical = 1u;   // a step was rejected (non-finite / negative depth)
@@ -313,6 +337,18 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  : "memory");
 }
 
+// asynchronous copy of a record from global into shared memory (16 bytes at a time), waited for by
+// the thread that issued it
+template <typename V> __device__ __forceinline__ void copy_async(V* dst, const V* src) {
+    static_assert(sizeof(V) % 16 == 0, "whole 16-byte pieces");
+#pragma unroll
+    for (int b = 0; b < int(sizeof(V)); b += 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst) + unsigned(b)),
+                     "l"(reinterpret_cast<const char*>(src) + b)
+                     : "memory");
+}
+__device__ __forceinline__ void copy_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ---------------- Green-Ampt soil class table -----------------------------------------
 template <typename R> struct SoilClass {
     R ks, psi, dth, lu, kout, tr, minsm, pad;
@@ -348,6 +384,35 @@ __device__ __host__ inline double uniform_integral(const RainDesc& rd, double a,
     }
     return acc;
 }
+
+// uniform_integral by one warp, an entry of the table per lane; the terms are summed in the
+// table's order (all lanes return the same)
+__device__ __forceinline__ double uniform_integral_warp(const RainDesc& rd, double a, double b, int lane) {
+    double acc = 0.0;
+    if (!(b > a)) return acc;
+    for (int q0 = 0; q0 < rd.n_uniform; q0 += 32) {
+        const int q = q0 + lane;
+        double term = 0.0;
+        bool on = false;
+        if (q < rd.n_uniform) {
+            const double lo = rd.t_start[q], rate = rd.rate[q];
+            const double hi = q + 1 < rd.n_uniform ? rd.t_start[q + 1] : b;
+            const double ov = fmax(0.0, fmin(b, hi) - fmax(a, lo));
+            on = ov > 0.0 && isfinite(rate);
+            term = rate * ov;
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, on); m; m &= m - 1u)
+            acc += __shfl_sync(0xffffffffu, term, __ffs(m) - 1);
+    }
+    return acc;
+}
+// Programmatic dependent launch: `dependents_may_launch` lets the next launch's CTAs take free
+// slots and run their heads; `wait_for_launches_before` returns when every launch before this one has
+// completed and its writes are visible.
+__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_launches_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 template <typename R>
 __device__ __forceinline__ R map_rate(const RainDesc& rd, const float* f, int i, int j, int ny, int nx);
@@ -512,6 +577,20 @@ template <typename R> struct RainStep {
             }
         }
     }
+    // make() by one warp (the maps' part by its first lane); `out` in shared memory
+    static __device__ void make_warp(RainStep& out, const RainDesc& rd, double a, double b, int lane) {
+        if (rd.n_maps) {
+            if (lane == 0) out.make(rd, a, b);
+            return;
+        }
+        const double v = rd.n_uniform ? uniform_integral_warp(rd, a, b, lane) : 0.0;
+        if (lane == 0) {
+            out.depth = R(div_by(v, 60000.0, 1.0 / 60000.0));
+            out.nm = 0;
+            out.m[0] = out.m[1] = 0;
+            out.w[0] = out.w[1] = R(0);
+        }
+    }
     // depth [m] the step adds at cell (i, j)
     __device__ R at(const RainDesc& rd, int i, int j, int ny, int nx) const {
         if (!rd.n_maps) return depth;
@@ -525,21 +604,50 @@ template <typename R> struct RainStep {
 };
 
 
+// A step's rain, kept in device memory by the step before: that of the interval [key_a, key_b]
+// (the host voids the keys when it changes the forcing); and the save clock of the step that
+// starts at key_b.
+template <typename R> struct StepPrep {
+    double key_a, key_b;
+    double time_save;
+    RainStep<R> rs;
+};
+
+// Bilinear sample of a coarse map at the cell centres, in two halves: map_row places a row of
+// cells between two rows of the map, map_column interpolates those two rows at a column.
+template <typename R> struct MapRow {
+    int iy0, iy1;
+    R wy;
+};
+template <typename R> __device__ __forceinline__ MapRow<R> map_row(int i, int my, R scale_y) {
+    const R half = R(0.5);
+    R fy = (R(i) + half) * scale_y - half;
+    fy = fmin(fmax(fy, R(0)), R(my - 1));
+    MapRow<R> m;
+    m.iy0 = (int)floor(fy);
+    m.iy1 = min(m.iy0 + 1, my - 1);
+    m.wy = fy - R(m.iy0);
+    return m;
+}
+template <typename R>
+__device__ __forceinline__ void map_column(const float* f, const MapRow<R>& m, int j, int mx, R scale_x, R& top, R& bot) {
+    const R half = R(0.5);
+    R fx = (R(j) + half) * scale_x - half;
+    fx = fmin(fmax(fx, R(0)), R(mx - 1));
+    const int ix0 = (int)floor(fx);
+    const int ix1 = min(ix0 + 1, mx - 1);
+    const R wx = fx - R(ix0);
+    const R f00 = R(f[m.iy0 * mx + ix0]), f01 = R(f[m.iy0 * mx + ix1]);
+    const R f10 = R(f[m.iy1 * mx + ix0]), f11 = R(f[m.iy1 * mx + ix1]);
+    top = (R(1) - wx) * f00 + wx * f01;
+    bot = (R(1) - wx) * f10 + wx * f11;
+}
 template <typename R>
 __device__ __forceinline__ R map_rate(const RainDesc& rd, const float* f, int i, int j, int ny, int nx) {
-    const R half = R(0.5);
-    R fy = (R(i) + half) * R(double(rd.my) / ny) - half;
-    R fx = (R(j) + half) * R(double(rd.mx) / nx) - half;
-    fy = fmin(fmax(fy, R(0)), R(rd.my - 1));
-    fx = fmin(fmax(fx, R(0)), R(rd.mx - 1));
-    int iy0 = (int)floor(fy), ix0 = (int)floor(fx);
-    int iy1 = min(iy0 + 1, rd.my - 1), ix1 = min(ix0 + 1, rd.mx - 1);
-    R wy = fy - R(iy0), wx = fx - R(ix0);
-    R f00 = R(f[iy0 * rd.mx + ix0]), f01 = R(f[iy0 * rd.mx + ix1]);
-    R f10 = R(f[iy1 * rd.mx + ix0]), f11 = R(f[iy1 * rd.mx + ix1]);
-    R top = (R(1) - wx) * f00 + wx * f01;
-    R bot = (R(1) - wx) * f10 + wx * f11;
-    return (R(1) - wy) * top + wy * bot;
+    const MapRow<R> m = map_row<R>(i, rd.my, R(double(rd.my) / ny));
+    R top, bot;
+    map_column<R>(f, m, j, rd.mx, R(double(rd.mx) / nx), top, bot);
+    return (R(1) - m.wy) * top + m.wy * bot;
 }
 
 // ---------------- Green-Ampt (one cell) -----------------------------------------------
@@ -737,6 +845,81 @@ __device__ __forceinline__ R face_momentum(bool wet, R Hf, R S, R qp, R n2c, con
     const R thr = H * R(10);
     qq = fmin(fmax(qq, -thr), thr);
     return wet ? qq : R(0);
+}
+
+// ---------------- the fused steps' form of the same arithmetic -------------------------------
+// The wet path is bound by instruction issue, so these leave out what cannot change a result of the
+// fused kernels: the depths that enter are >= 0 (or NaN, next to closed faces only); a face's value
+// is selected once, at the end; closed faces and depths below the smallest normal number, rare, are
+// left to branches that whole warps skip.  Every face and cell gets the bits of face_flux,
+// donor_scale, limit_face and cfl_cell (up to the sign of a zero).
+//
+// face_open: the face depth and slope of an open face; returns whether it is open (a closed one's
+// depth comes from face_closed).
+template <typename R, bool IS_X>
+__device__ __forceinline__ bool face_open(R ha, R hb, R dz, R& Hf, R& S, const StepConsts<R>& K) {
+    const R up = fmax(dz, R(0)), dn = fmin(dz, R(0));
+    if (IS_X) {
+        Hf = fmax(fmax(ha - up, hb + dn), R(0));
+        S = (dz + (hb - ha)) * K.inv_dx;
+    } else {
+        Hf = fmax(fmax(ha + dn, hb - up), R(0));
+        S = (dz + (ha - hb)) * K.inv_dx;
+    }
+    return fabs(dz) <= R(3.0e38);
+}
+template <typename R> __device__ __forceinline__ R face_closed(R ha, R hb, R dz) {
+    return isnan(dz) ? fmax(fmax(ha, hb), R(0)) : R(0);
+}
+// x^(7/3) of a normal positive number
+template <typename R> __device__ __forceinline__ R pow73_normal(R x) {
+    R r = bits_seed(x);
+    const R third = R(1.0 / 3.0);
+#pragma unroll
+    for (int it = 0; it < RcbrtTraits<R>::iters; ++it) {
+        const R t = (x * r) * r;
+        const R e = fma(-t, r, R(1));
+        r = fma(r * e, third, r);
+    }
+    const R c = x * (r * r);
+    return (x * x) * c;
+}
+template <typename R> __device__ __noinline__ R pow73_any(R x) { return pow73_pos(x); }
+__device__ __forceinline__ bool finite_abs(float x) { return fabsf(x) <= 3.402823466e+38f; }
+__device__ __forceinline__ bool finite_abs(double x) { return fabs(x) <= 1.7976931348623157e+308; }
+// the momentum update of a face; what is not wet gets 0 (its operands may be anything)
+template <typename R, int SCH = 0>
+__device__ __forceinline__ R face_update(bool wet, R H, R h73, R S, R qp, R n2c, const StepConsts<R>& K,
+                                         int flag_critical, int scheme = 1, R q_lo = R(0), R q_hi = R(0)) {
+    R qn = qp;
+    if (SCH) qn = diffused_momentum(qp, q_lo, q_hi, H, K, scheme);
+    const R num = fma(-(K.gdt * H), S, qn);
+    const R den = fma(K.gdt * n2c, fabs(qp), h73);
+    R qq = qdiv(num * h73, den);
+    const bool ok = wet && finite_abs(qq);
+    if (flag_critical == 1) {
+        const R crit = H * sqrt(K.g * H);
+        qq = fmin(fmax(qq, -crit), crit);
+    }
+    const R thr = H * R(10);
+    qq = fmin(fmax(qq, -thr), thr);
+    return ok ? qq : R(0);
+}
+// what leaves a cell and what it holds, as rates: its faces are limited when the first exceeds the
+// second (donor_scale)
+template <typename R> __device__ __forceinline__ R donor_out(R qR, R qL, R qU, R qD) {
+    R out = fmax(qR, R(0));
+    out = out + fmax(-qL, R(0));
+    out = out + fmax(qU, R(0));
+    return out + fmax(-qD, R(0));
+}
+template <typename R> __device__ __forceinline__ R limit_by(R q, R s_pos, R s_neg) { return q * (q > R(0) ? s_pos : s_neg); }
+// velocity of a face (FP32's quotient gives 0 for q = 0 whatever the depth; FP64's needs the test)
+__device__ __forceinline__ float face_velocity(float q, float hf, const StepConsts<float>& K) {
+    return qdiv(q, hf < K.tol ? 1e9f : hf);
+}
+__device__ __forceinline__ double face_velocity(double q, double hf, const StepConsts<double>& K) {
+    return q == 0.0 ? 0.0 : q / (hf < K.tol ? 1e9 : hf);
 }
 
 // outgoing rate of a cell over its four faces and its donor scale factor

@@ -50,13 +50,9 @@ constexpr int kStages = HP2D_STAGES;   // shared-memory ring depth of the row pi
 #define HP2D_ROW_UNROLL 1
 #endif
 constexpr int kRowUnroll = HP2D_ROW_UNROLL;   // row-loop unroll (register renaming of the window)
-#ifndef HP2D_FACE_ILP
-#define HP2D_FACE_ILP 1   // 1: interleaved faces in every instantiation, 0: infiltration / rain maps only, -1: none
-#endif
-// The faces of a row as interleaved, branch-free momentum updates (face_geom + face_momentum)
+// The faces of a row are interleaved, branch-free momentum updates (face_open + face_update)
 // rather than one face_flux after the other: measured faster on every workload (wet 2048^2 40.2
 // vs 39.1 GCUPS, 60-minute dam-break 98.3 vs 96.3, Green-Ampt + rain maps 21.4 vs 21.0).
-template <int INF, bool MAP> constexpr bool kFaceIlp = HP2D_FACE_ILP > 0 || (HP2D_FACE_ILP == 0 && (INF != 0 || MAP));
 // Phase (F) without a per-lane branch around each cell's body (stores and reductions masked
 // instead), so that the CPL cells interleave: wet 2048^2 41.6 vs 40.8 GCUPS, 60-minute dam-break
 // 115.5 vs 111.8, 128-member ensemble 44.6 vs 43.0; the Green-Ampt + rain-map instantiation ran
@@ -77,6 +73,9 @@ template <typename R> struct FusedArgs {
     double tol_mm, thr_mm;
     double t_end;                // routing_time + min_time_step/60 [min]
     double min_dt, max_dt, inc, tsc, alfa_min, alfa_max;
+    double inv_inc, inv_tsc, inv_res;   // correctly rounded reciprocals (div_by)
+    R k_const[4];                // StepConsts' inv_dx, g, tol, thr
+    R map_sy, map_sx;            // rain map cells per grid cell
     int flag_timestep, adaptive, flag_critical, outlet_type, ga;   // ga: infiltration on (either model)
     int scheme;                  // flag_numerical_scheme: 1 Bates, 2 s-upwind, 3 s-centred
     unsigned int wait_polls;     // polls of a row-copy wait before it gives up (HP2D_TIMEOUT)
@@ -104,25 +103,41 @@ template <typename R> struct FusedArgs {
     // multiple of 4, so that a warp reads its rows' flags as one word per lane)
     unsigned char* dryflag;
     int dry_rows;
+    int tile_nx;                 // tiles per row of tiles (hp2d_tile.cuh); 0: strips
+    int tile_rpt;                // rows per thread of the tile step
+    unsigned tile_grid;          // CTAs of the tile step's launch at most
     StepScalars* sc;
+    StepPrep<R>* prep;           // [2] the step's rain, prepared by the step before
+    StepAcc* acc;                // [4] accumulators (see StepAcc); sc is [2] in the same rotation
 };
 
-__device__ __host__ inline double finalize_dt(double vmax, double cmax, double res, double alfa_min,
-                                              double alfa_max, double min_dt, double max_dt, double inc,
-                                              int flag_timestep) {
+// refreshing_timestep.m:94-134, :315-359 in three parts, so that the quotients q_adv = res / max(vmax,
+// 1e-10), q_wave = alfa_min res / cmax and the last one by the increment can be formed elsewhere
+__device__ __host__ inline double finalize_new(double vmax, double cmax, double q_adv, double q_wave, double alfa_min,
+                                               double alfa_max, double max_dt, int flag_timestep) {
     double dt_adv;
     if (vmax > 0) {
-        dt_adv = 1.0 * res / fmax(vmax, 1e-10);
+        dt_adv = q_adv;
         double tsf = fmax(alfa_max - 2.0 * fmax(vmax - 5.0, 0.0), alfa_min);
         dt_adv = fmin(dt_adv * tsf, max_dt);
     } else {
         dt_adv = max_dt;
     }
-    double dt_wave = cmax > 0 ? (alfa_min * res) / cmax : max_dt;
+    double dt_wave = cmax > 0 ? q_wave : max_dt;
     double nw = flag_timestep == 1 ? fmin(dt_adv, dt_wave) : dt_wave;
     if (isnan(nw) || isinf(nw)) nw = max_dt;
-    double tcr = fmax(inc * floor(nw / inc), min_dt);
+    return nw;
+}
+__device__ __host__ inline double finalize_snap(double q_inc, double min_dt, double max_dt, double inc) {
+    double tcr = fmax(inc * floor(q_inc), min_dt);
     return fmin(tcr, max_dt);
+}
+__device__ __host__ inline double finalize_dt(double vmax, double cmax, double res, double alfa_min,
+                                              double alfa_max, double min_dt, double max_dt, double inc,
+                                              int flag_timestep) {
+    const double nw = finalize_new(vmax, cmax, 1.0 * res / fmax(vmax, 1e-10), (alfa_min * res) / cmax, alfa_min,
+                                   alfa_max, max_dt, flag_timestep);
+    return finalize_snap(nw / inc, min_dt, max_dt, inc);
 }
 
 // compensated (Kahan) running sum: s + c tracks the exact sum of the added terms to about one
@@ -137,6 +152,7 @@ template <typename R> struct Kahan {
         s = t;
     }
     __device__ __forceinline__ double value() const { return double(s) - double(c); }
+    __device__ __forceinline__ bool any() const { return s != R(0) || c != R(0); }
 };
 
 template <typename R> __device__ __forceinline__ R warp_max(R v) {
@@ -237,62 +253,485 @@ __device__ __noinline__ void structure_prepare(const FusedArgs<R>& a, const Rain
     if (tid == 0) structure_transfers(a.strct, time_step, a.res * a.res);
 }
 
-template <typename R, int NT, int INF, bool MAP, int CPL = 1, bool INFL = false, int SCH = 0>
-__device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned blk) {
+// The clock of a step, as its launch finds it once the step before has ended.
+struct StepNow {
+    double t_min, time_step, dts;        // [min], [min], [s]
+    double rain_a, rain_b, t_prev;
+    double tcr, vm, time_save;           // of the step that ended: refreshed step [s], max speed, save clock
+    long long rec_count;
+    int cur, skip, done, halted;
+    int rec;                             // slot that receives this step's input depth (-1: none)
+    int rec_last, rec_pending;
+    int ended, accepted, refresh;        // a pending step ended, it was accepted, it refreshed the time step
+};
+
+// What every thread of a step's CTA shares: the step's scalars, constants and rain, and the
+// CTA's reductions.
+template <typename R, int NT> struct StepShared {
+    StepScalars sc;      // as found (step_books brings them up to date)
+    StepAcc acc;         // the pending step's sums
+    StepPrep<R> p;       // this step's rain
+    StepNow now;
+    StepConsts<R> K;
+    RainStep<R> rsn;     // the next step's rain
+    double save_next;    // save clock of this step (the next launch ends it)
+    int negn;            // an outlet cell would go below -1e-11 m after the next rain
+    int last;            // ensemble item: this CTA finished its member and the step was accepted
+    double stage;        // depth the stage overwrites of this CTA added [m]
+    unsigned skipw;      // cells whose unchanged record this CTA did not rewrite
+    unsigned skipr;      // of those, cells of skipped blocks (not read either)
+    R red_s2[NT / 32];
+    unsigned long long red_c[NT / 32];
+    double red_d[3][NT / 32];
+    int red_to[NT / 32];
+    unsigned red_bad[NT / 32];
+};
+
+// words of a struct in global memory (written by other SMs in an earlier launch) into shared memory
+template <int NT, typename T> __device__ __forceinline__ void copy_words(T& dst, const T* src, int tid) {
+    static_assert(sizeof(T) % 4 == 0, "whole words");
+    unsigned* d = reinterpret_cast<unsigned*>(&dst);
+    const unsigned* s = reinterpret_cast<const unsigned*>(src);
+#pragma unroll
+    for (int w = 0; w < int(sizeof(T) / 4); w += NT)
+        if (w + tid < int(sizeof(T) / 4)) d[w + tid] = __ldcg(s + w + tid);
+}
+template <typename T> __device__ __forceinline__ void store_words(T* dst, const T& src, int lane) {
+    unsigned* d = reinterpret_cast<unsigned*>(dst);
+    const unsigned* s = reinterpret_cast<const unsigned*>(&src);
+#pragma unroll
+    for (int w = 0; w < int(sizeof(T) / 4); w += 32)
+        if (w + lane < int(sizeof(T) / 4)) d[w + lane] = s[w + lane];
+}
+
+// The verdict on a step: rejected when a row copy timed out, when more cells ended it non-finite
+// or too negative than the run started with, or when the host's test hook names it.
+__device__ __forceinline__ bool step_rejected(const StepScalars& sc, const StepAcc& acc) {
+    return acc.timeout != 0u || acc.bad > sc.n_bad0 || (sc.fault_n > 0 && sc.k == sc.fault_k);
+}
+
+// The clock by one warp: ends the step `pending` (refreshing_timestep and the clock,
+// HydroPol2D_Main_While.m:691-705, :779) from its scalars and sums, and forms the constants of the
+// step that follows.  Only what that step's cells wait for is done here (the books are
+// step_books'), in registers, with the independent FP64 divisions of a stage side by side in
+// different lanes: one thread doing it all through memory took 8000 cycles, one warp with the
+// books 3600.
+// A rejected step commits nothing: the state stays in buffer cur and the clock and counters stay,
+// and the launches halt until the host has prepared the retry (HydroPol2D_Main_While.m:926-993).
+template <typename R>
+__device__ __forceinline__ double save_clock(const FusedArgs<R>& a, double t) {
+    return div_by((ceil(div_by(t * 60.0, a.tsc, a.inv_tsc)) - 1.0) * a.tsc, 60.0, 1.0 / 60.0);
+}
+template <typename R>
+__device__ __forceinline__ void step_clock(const FusedArgs<R>& a, const StepScalars& sc, const StepAcc& acc,
+                                           const StepPrep<R>& p, bool pending, StepNow& now, StepConsts<R>& K) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool accepted = pending && !step_rejected(sc, acc);
+    const double t = sc.t_min, tp = sc.t_prev;
+    const long long k = sc.k;
+    double ts1 = sc.time_step, t1 = t;
+    double tcr = 0.0, time_save = 0.0, vm = 0.0;
+    bool refresh = false;
+    int halted = sc.halted | ((pending && !accepted) ? 1 : 0);
+    if (accepted) {
+        // lane 0: max speed and the advective bound, lane 1: max celerity and the wave bound
+        const unsigned long long cb = acc.cmax;
+        const R arg = lane == 0 || !cb ? bits_to<R>(acc.vmax) : bits_to<R>(cb - 1ull);
+        double m = double(sqrt(arg));
+        if (lane != 0) m = !cb ? 0.0 : (a.adaptive == 1 ? fmax(m, double(R(1e-10))) : double(arg));
+        const double q = (lane == 0 ? 1.0 * a.res : a.alfa_min * a.res) / (lane == 0 ? fmax(m, 1e-10) : m);
+        time_save = p.key_b == t ? p.time_save : save_clock(a, t);
+        refresh = (time_save - sc.tsp > 0 || k == 1) &&
+                  (sc.refresh_every <= 1 || k == 1 || (k - 1) % sc.refresh_every == 0);
+        vm = __shfl_sync(FULL, m, 0);
+        const double nw = finalize_new(vm, __shfl_sync(FULL, m, 1), __shfl_sync(FULL, q, 0), __shfl_sync(FULL, q, 1),
+                                       a.alfa_min, a.alfa_max, sc.max_dt, a.flag_timestep);
+        tcr = refresh ? finalize_snap(div_by(nw, a.inc, a.inv_inc), a.min_dt, sc.max_dt, a.inc)
+                      : ts1 * 60.0;   // refreshing_timestep.m:361-365
+        ts1 = div_by(tcr, 60.0, 1.0 / 60.0);
+        t1 = ts1 + t;
+        if (refresh && tcr == a.min_dt && sc.dt_floor_stop) halted = 1;   // this step is kept; the next launches wait
+    }
+    // StepConsts::make, a constant per lane
+    const double dts = ts1 * 60.0;
+    const double q2 = (lane == 3 ? a.res : 1.0) / dts;
+    const double v = lane == 0 ? dts : lane == 1 ? kG * dts : lane == 2 ? div_by(dts, a.res, a.inv_res) : q2;
+    static_assert(sizeof(StepConsts<R>) == 9 * sizeof(R), "nine constants");
+    if (lane < 9) reinterpret_cast<R*>(&K)[lane] = lane < 5 ? R(v) : a.k_const[lane < 5 ? 0 : lane - 5];
+    if (lane == 0) {
+        now.t_min = t1;
+        now.time_step = ts1;
+        now.dts = dts;
+        // the next step's rain: update_spatial_BC over [t_previous, t]
+        // (HydroPol2D_Main_While.m:721), then t_previous <- the clock increment on the first
+        // step and t after it (:734-738), and the clock advances by the new step (:779)
+        now.rain_a = accepted ? tp : sc.rain_a;
+        now.rain_b = accepted ? t : sc.rain_b;
+        now.t_prev = accepted ? (k == 1 ? ts1 : t) : tp;
+        now.tcr = tcr;
+        now.vm = vm;
+        now.time_save = time_save;
+        now.cur = sc.cur ^ (accepted ? 1 : 0);
+        now.skip = accepted ? (acc.negn ? 1 : 0) : sc.skip_clamp;   // gathered by every CTA's outlets
+        now.halted = halted;
+        now.done = !(t1 <= a.t_end) || halted;
+        now.ended = pending;
+        now.accepted = accepted;
+        now.refresh = refresh;
+        now.rec = -1;
+        if (a.rec.n_times > 0) {   // save_output_maps.m:25-27 with t_save = t + new dt (:740)
+            long long count = sc.rec_count;
+            int rp = sc.rec_pending, rl = sc.rec_last;
+            if (accepted) {
+                if (rp) { count += 1; rp = 0; }   // recorded by the step that ended
+                const int idx = last_record_below(a.rec.times, a.rec.n_times, t + ts1);
+                if (idx > rl && a.rec.n_slots > 0) rp = 1;
+                if (idx > rl) rl = idx;
+            }
+            now.rec_count = count;
+            now.rec_last = rl;
+            now.rec_pending = rp;
+            if (rp && a.rec.n_slots > 0) now.rec = int(count % a.rec.n_slots);
+        }
+    }
+    __syncwarp();
+}
+
+// The books of the step that step_clock ended (one warp): sc, as found, becomes what the next
+// launch or the host reads.
+template <typename R, bool INFL>
+__device__ __noinline__ void step_books(const FusedArgs<R>& a, StepScalars& __restrict__ sc, const StepAcc& __restrict__ acc,
+                                         const StepNow& __restrict__ now) {
+    if ((threadIdx.x & 31) == 0) {
+        sc.pending = 0;
+        if (now.ended) {
+            if (acc.timeout) sc.status |= kStatusTimeout;
+            if (acc.bad > sc.n_bad0) sc.status |= kStatusNumerical;
+            if (sc.fault_n > 0 && sc.k == sc.fault_k) {   // the host's test hook
+                sc.fault_n -= 1;
+                sc.status |= kStatusNumerical;
+            }
+            sc.skipped_cells += acc.skipw;
+            sc.skipped_read_cells += acc.skipr;
+            sc.halted = now.halted;
+        }
+        if (now.accepted) {
+            if (sc.skip_clamp) sc.neg_warn += 1;
+            double rain_s = acc.rain;
+            // uniform rain: the same depth on every cell with a finite depth
+            if (a.rain.n_uniform) rain_s += sc.rain_cell * double(sc.n_finite);
+            sc.tsp = now.time_save;
+            sc.last_vbits = acc.vmax;
+            sc.last_cbits = acc.cmax;
+            sc.last_refreshed = now.refresh;
+            sc.last_unstable = 0;
+            if (now.refresh) {
+                sc.vmax_last = now.vm;
+                sc.last_unstable = now.tcr == a.min_dt;
+                if (now.tcr == a.min_dt) {   // refreshing_timestep.m:357-359 (unstable)
+                    sc.unstable += 1;
+                    if (sc.dt_floor_stop) sc.status |= kStatusDtFloor;
+                }
+            }
+            const double area = a.res * a.res;
+            sc.rain_vol += rain_s * area;
+            sc.inf_vol += acc.inf * area;
+            sc.out_vol += acc.out * area;
+            if constexpr (INFL) {
+                if (a.inflow.n_gauges) {   // every cell of a gauge with a finite elevation got its depth
+                    double v = 0.0;
+                    for (int g = 0; g < a.inflow.n_gauges; ++g) v += double(a.inflow.depth[g]) * a.inflow.gauge_cells[g];
+                    sc.inflow_vol += v * area;
+                }
+                if (a.inflow.n_stage) sc.stage_vol += acc.stage * area;
+                if (a.strct.n) {   // the structures' extras this step applied
+                    double v = 0.0;
+                    for (int q = 0; q < a.strct.n_slots; ++q) v += double(a.strct.extra[q]) * area;
+                    sc.struct_vol += v;
+                }
+            }
+            if (a.rec.n_times > 0) {
+                sc.rec_count = now.rec_count;
+                sc.rec_pending = now.rec_pending;
+                sc.rec_last = now.rec_last;
+                if (now.rec >= 0) a.rec.snap_t[now.rec] = sc.t_min;
+            }
+            sc.rain_a = now.rain_a;
+            sc.rain_b = now.rain_b;
+            sc.t_prev = now.t_prev;
+            sc.time_step = now.time_step;
+            sc.t_min = now.t_min;
+            sc.k += 1;
+            sc.cur = now.cur;
+            sc.skip_clamp = now.skip;
+        }
+    }
+    __syncwarp();
+}
+
+// the next step's gauge depths and stages (one warp)
+template <typename R> __device__ __forceinline__ void gauges_prepare(const FusedArgs<R>& a, const StepScalars& sc, int lane) {
+    for (int g = lane; g < a.inflow.n_gauges; g += 32)
+        a.inflow.depth[g] = R(inflow_integral(a.inflow, g, sc.rain_a, sc.rain_b) / 60000.0);
+    for (int g = lane; g < a.inflow.n_stage; g += 32) a.inflow.stage_now[g] = R(stage_at(a.inflow, g, sc.t_min));
+}
+
+// The head of a step's CTA, by all its threads.  A solo grid's launch (SOLO) finds the step before
+// pending and ends it here, in every CTA alike, from its scalars and sums: one round trip to L2,
+// then warp 0's arithmetic while the other warps fetch their records (`early`, given the buffer that
+// holds the state, which only needs the verdict).  This replaces a ticket and a tail in the last
+// CTA, which the whole GPU waited for (release, ticket, reload and one thread's FP64 chain: 9000 of
+// a small grid's 18000 cycles per step).  CTA 0 keeps the books for the next launch (step_publish).
+// Items of an ensemble (not SOLO) find their member's scalars finished by step_finish's last CTA.
+// The rain comes prepared from the step before (its table walk is off the critical path); thread 0
+// makes what is missing on a call's first step.  ASYNC: the next step's rain is computed by warp 1
+// after the last barrier here and is visible after the caller's next CTA barrier.
+template <typename R, int NT>
+__device__ __forceinline__ void step_next(const FusedArgs<R>& a, StepShared<R, NT>& sh, int lane) {
+    RainStep<R>::make_warp(sh.rsn, a.rain, sh.now.t_prev, sh.now.t_min, lane);
+    if (lane == 0) sh.save_next = save_clock(a, sh.now.t_min);
+    __syncwarp();
+}
+template <typename R, int NT, bool ASYNC, bool SOLO, typename Early>
+__device__ __forceinline__ void step_begin(const FusedArgs<R>& a, StepShared<R, NT>& sh, int phase, Early early) {
+    const int tid = threadIdx.x, warp = tid >> 5;
+    if (SOLO) {
+        dependents_may_launch();
+        wait_for_launches_before();
+    }
+    copy_words<NT>(sh.sc, a.sc + (SOLO ? (phase & 1) : 0), tid);
+    copy_words<NT>(sh.p, a.prep + (SOLO ? (phase & 1) : 0), tid);
+    if (SOLO) copy_words<NT>(sh.acc, a.acc + phase, tid);
+    if (tid == 0) {
+        sh.negn = 0;
+        sh.stage = 0.0;
+        sh.skipw = 0u;
+        sh.skipr = 0u;
+    }
+    __syncthreads();
+    const bool pending = SOLO && sh.sc.pending;
+    early(sh.sc.cur ^ ((pending && !step_rejected(sh.sc, sh.acc)) ? 1 : 0));
+    const int lane = tid & 31;
+    if (warp == 0) {
+        step_clock(a, sh.sc, sh.acc, sh.p, pending, sh.now, sh.K);
+        if (!(sh.p.key_a == sh.now.rain_a && sh.p.key_b == sh.now.rain_b))
+            RainStep<R>::make_warp(sh.p.rs, a.rain, sh.now.rain_a, sh.now.rain_b, lane);
+        // the next step applies the rain of [t_previous, t] (HydroPol2D_Main_While.m:721)
+        if (!ASYNC) step_next(a, sh, lane);
+    }
+    __syncthreads();
+}
+
+// step_begin and step_publish of the strip kernels, out of line: inlined, their registers would
+// count against the row loop's
+template <typename R, int NT, bool SOLO, bool INFL>
+__device__ __noinline__ void step_begin_strips(const FusedArgs<R>& a, StepShared<R, NT>& sh, unsigned blk, int phase);
+
+// CTA 0's warp 0, any time after step_begin (and step_next): the scalars, the
+// next step's rain and a clear accumulator for the launches that follow.
+template <typename R, int NT, bool INFL>
+__device__ __forceinline__ void step_publish(const FusedArgs<R>& a, StepShared<R, NT>& sh, int phase) {
+    const int lane = threadIdx.x & 31;
+    step_books<R, INFL>(a, sh.sc, sh.acc, sh.now);
+    if (lane == 0) {
+        sh.sc.rain_cell = double(sh.p.rs.depth);
+        sh.sc.pending = !sh.now.done;
+        StepPrep<R>& np = a.prep[(phase + 1) & 1];
+        np.key_a = sh.now.t_prev;
+        np.key_b = sh.now.t_min;
+        np.time_save = sh.save_next;
+        np.rs = sh.rsn;
+    }
+    __syncwarp();
+    store_words(a.sc + ((phase + 1) & 1), sh.sc, lane);
+    unsigned* z = reinterpret_cast<unsigned*>(a.acc + ((phase + 2) & 3));
+    for (int w = lane; w < int(sizeof(StepAcc) / 4); w += 32) z[w] = 0u;
+}
+
+template <typename R, int NT, bool SOLO, bool INFL>
+__device__ __noinline__ void step_begin_strips(const FusedArgs<R>& a, StepShared<R, NT>& sh, unsigned blk, int phase) {
+    step_begin<R, NT, false, SOLO>(a, sh, phase, [](int) {});
+    if (SOLO && blk == 0 && threadIdx.x < 32) step_publish<R, NT, INFL>(a, sh, phase);
+}
+
+// warp maximum of ordered bits of non-negative numbers (or of the celerity code): one redux in FP32
+template <typename R> __device__ __forceinline__ unsigned long long warp_max_code(unsigned long long v) {
+    if constexpr (sizeof(R) == 4) return __reduce_max_sync(0xffffffffu, unsigned(v));
+    else return warp_max_u(v);
+}
+
+// The end of a CTA's part of a step, called by all its threads: one warp reduction each of the
+// sums the kernel can have, then the step's accumulators.  A solo grid is done with that: the next
+// launch ends the step.  An ensemble item takes a ticket of its member, and the CTA that finishes
+// the member last ends its step.  Returns false when one of the CTA's row copies timed out.
+template <typename R, int NT, int INF, bool MAP, bool INFL, bool SOLO>
+__device__ __forceinline__ bool step_finish(const FusedArgs<R>& a, StepShared<R, NT>& sh, double rain_acc,
+                                            double inf_acc, double out_acc, R s2max, R cmaxv, unsigned nbad,
+                                            bool timed_out, int phase, const typename Vec<R>::V4* sout,
+                                            const typename Vec<R>::V2* gout) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NWARP = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long scode = warp_max_code<R>(ord_bits(s2max));
+    // 0: no non-stagnant cell; else the bits of the (non-negative, +0 for -0) maximum + 1
+    unsigned long long cenc = warp_max_code<R>(cmaxv >= R(0) ? ord_bits(cmaxv + R(0)) + 1ull : 0ull);
+    if (MAP) rain_acc = warp_sum(rain_acc);
+    if (INF) inf_acc = warp_sum(inf_acc);
+    if (__any_sync(FULL, out_acc != 0.0)) out_acc = warp_sum(out_acc);   // strips and tiles with outlets
+    const int to_any = __any_sync(FULL, timed_out);
+    nbad = __reduce_add_sync(FULL, nbad);
+    if (lane == 0) {
+        sh.red_bad[warp] = nbad;
+        sh.red_s2[warp] = bits_to<R>(scode);
+        sh.red_c[warp] = cenc;
+        sh.red_d[0][warp] = rain_acc;
+        sh.red_d[1][warp] = inf_acc;
+        sh.red_d[2][warp] = out_acc;
+        sh.red_to[warp] = to_any;
+    }
+    __syncthreads();
+    bool cta_ok = true;
+#pragma unroll
+    for (int w = 0; w < NWARP; ++w) cta_ok = cta_ok && sh.red_to[w] == 0;
+    if (warp == 0) {
+        const int w = lane < NWARP ? lane : 0;
+        scode = warp_max_code<R>(ord_bits(sh.red_s2[w]));
+        cenc = warp_max_code<R>(sh.red_c[w]);
+        const unsigned bad = __reduce_add_sync(FULL, lane < NWARP ? sh.red_bad[w] : 0u);
+        double sum[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            if ((q == 0 && !MAP) || (q == 1 && !INF)) continue;
+            const double v = lane < NWARP ? sh.red_d[q][w] : 0.0;
+            if (__any_sync(FULL, v != 0.0)) sum[q] = warp_sum(v);
+        }
+        StepAcc* const acc = a.acc + (SOLO ? ((phase + 1) & 3) : 0);
+        unsigned ticket = 0u;
+        if (lane == 0) {
+            if (!cta_ok) atomicOr(&acc->timeout, 1u);   // a row copy did not arrive in time
+            if (bad) atomicAdd(&acc->bad, (unsigned long long)bad);
+            if (scode) atomicMax(&acc->vmax, scode);
+            if (cenc) atomicMax(&acc->cmax, cenc);
+            if (sum[0] != 0.0) atomicAdd(&acc->rain, sum[0]);
+            if (sum[1] != 0.0) atomicAdd(&acc->inf, sum[1]);
+            if (sum[2] != 0.0) atomicAdd(&acc->out, sum[2]);
+            if (sh.negn) atomicOr(&acc->negn, 1u);
+            if (INFL && sh.stage != 0.0) atomicAdd(&acc->stage, sh.stage);
+            if (sh.skipw) atomicAdd(&acc->skipw, (unsigned long long)sh.skipw);
+            if (sh.skipr) atomicAdd(&acc->skipr, (unsigned long long)sh.skipr);
+            // the accumulators above are released before the ticket, and acquired by the last CTA
+            if (!SOLO)
+                asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(&a.sc->counter) : "memory");
+        }
+        if (!SOLO) {
+            const bool last = __shfl_sync(FULL, ticket, 0) == a.n_ctas - 1;
+            if (lane == 0) sh.last = 0;
+            if (last) {
+                copy_words<32>(sh.acc, a.acc, lane);
+                __syncwarp();
+                step_clock(a, sh.sc, sh.acc, sh.p, true, sh.now, sh.K);
+                const bool accepted = sh.now.accepted;
+                if (lane == 0) {
+                    sh.sc.rain_cell = double(sh.p.rs.depth);   // of the step that ends
+                    sh.sc.counter = 0u;
+                    sh.last = accepted;
+                    sh.p.key_a = sh.now.rain_a;
+                    sh.p.key_b = sh.now.rain_b;
+                    sh.p.rs = sh.rsn;
+                }
+                __syncwarp();
+                step_books<R, INFL>(a, sh.sc, sh.acc, sh.now);
+                store_words(a.sc, sh.sc, lane);
+                if (accepted) store_words(a.prep, sh.p, lane);
+                unsigned* z = reinterpret_cast<unsigned*>(a.acc);
+                for (int q = lane; q < int(sizeof(StepAcc) / 4); q += 32) z[q] = 0u;
+                if (INFL && accepted) gauges_prepare(a, sh.sc, lane);
+            }
+        }
+    }
+    if constexpr (INFL && !SOLO) {
+        if (a.strct.n) {   // the next step's structure transfers, from its d_tot
+            __syncthreads();
+            if (sh.last) {
+                __threadfence();   // records of other CTAs
+                structure_prepare<R, INF, MAP, INFL>(a, sh.rsn, sh.sc.skip_clamp != 0, sh.K, sout, gout, tid, NT,
+                                                     sh.sc.time_step);
+            }
+        }
+    }
+    return cta_ok;
+}
+
+// Ends the step that launch phase - 1 left pending (one CTA): after the last launch of a batch, for
+// the host, and after every launch of a grid with gauges, stages or control structures, whose next
+// step's depths, stages and transfers it prepares too.  Leaves the scalars in slot 0, nothing
+// pending and every accumulator clear.
+template <typename R, int INF, bool MAP>
+__global__ void __launch_bounds__(128) k_step_flush(const __grid_constant__ FusedArgs<R> a, int phase) {
+    __shared__ StepShared<R, 128> sh;
+    const int tid = threadIdx.x, lane = tid & 31;
+    copy_words<128>(sh.sc, a.sc + (phase & 1), tid);
+    copy_words<128>(sh.acc, a.acc + phase, tid);
+    copy_words<128>(sh.p, a.prep + (phase & 1), tid);
+    __syncthreads();
+    const bool pending = sh.sc.pending != 0;
+    if (tid < 32) {
+        step_clock(a, sh.sc, sh.acc, sh.p, pending, sh.now, sh.K);
+        step_books<R, true>(a, sh.sc, sh.acc, sh.now);
+        store_words(a.sc, sh.sc, lane);
+        store_words(a.prep, sh.p, lane);
+        if (sh.now.accepted) gauges_prepare(a, sh.sc, lane);
+    }
+    unsigned* z = reinterpret_cast<unsigned*>(a.acc);
+    for (int w = tid; w < int(4 * sizeof(StepAcc) / 4); w += 128) z[w] = 0u;
+    __syncthreads();
+    if (a.strct.n && sh.now.accepted) {
+        if (tid == 0) sh.rsn.make(a.rain, sh.sc.rain_a, sh.sc.rain_b);
+        __syncthreads();
+        structure_prepare<R, INF, MAP, true>(a, sh.rsn, sh.sc.skip_clamp != 0, sh.K, sh.sc.cur ? a.st1 : a.st0,
+                                             sh.sc.cur ? a.gs1 : a.gs0, tid, 128, sh.sc.time_step);
+    }
+}
+
+// the rain of a step at one cell, out of line (the few outlet cells of a grid with rain maps)
+template <typename R> __device__ __noinline__ R rain_at_cell(const FusedArgs<R>& a, const RainStep<R>& rs, int i, int j) {
+    return rs.at(a.rain, i, j, a.ny, a.nx);
+}
+
+template <typename R, int NT, int INF, bool MAP, int CPL, bool INFL, int SCH, bool SOLO>
+__device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned blk, const int phase) {
     using V4 = typename Vec<R>::V4;
     using V2 = typename Vec<R>::V2;
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ StepConsts<R> s_K;
-    __shared__ double s_tmin, s_dts;
-    __shared__ int s_cur, s_skip, s_done, s_last;
-    __shared__ int s_negn;   // an outlet cell would go below -1e-11 m after the next rain
-    __shared__ int s_rec;    // slot that receives this step's input depth (-1: none)
-    __shared__ double s_stage;   // depth the stage overwrites of this CTA added [m]
-    __shared__ unsigned s_skipw;  // cells whose unchanged record this CTA did not rewrite
-    __shared__ unsigned s_skipr;  // of those, cells of skipped blocks (not read either)
-    __shared__ RainStep<R> s_rs, s_rsn;   // this step's rain and the next one's
-    __shared__ R red_s2[NT / 32];
-    __shared__ unsigned long long red_c[NT / 32];
-    __shared__ double red_d[3][NT / 32];
-    __shared__ int red_to[NT / 32];
-    __shared__ unsigned red_bad[NT / 32];
+    __shared__ StepShared<R, NT> sh;
+    const int& s_rec = sh.now.rec;
+    int& s_negn = sh.negn;
+    double& s_stage = sh.stage;
+    unsigned& s_skipw = sh.skipw;
+    unsigned& s_skipr = sh.skipr;
+    const RainStep<R>& s_rs = sh.p.rs;
+    const RainStep<R>& s_rsn = sh.rsn;
+    __shared__ R s_map[2][2][MAP ? NT * CPL : 1];   // rain maps in force: rows above / below, per cell of a lane
     __shared__ __align__(8) unsigned long long s_bar[NT / 32][kStages];
     extern __shared__ __align__(128) unsigned char smem_dyn[];
     bool timed_out = false;
 
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        StepScalars* sc = a.sc;
-        s_tmin = sc->t_min;
-        s_dts = sc->time_step * 60.0;
-        s_cur = sc->cur;
-        s_skip = sc->skip_clamp;
-        s_negn = 0;
-        s_stage = 0.0;
-        s_skipw = 0u;
-        s_skipr = 0u;
-        s_rec = (sc->rec_pending && a.rec.n_slots > 0) ? int(sc->rec_count % a.rec.n_slots) : -1;
-        s_done = !(s_tmin <= a.t_end) || sc->halted;
-        s_K.make(s_dts, a.res, a.tol_mm, a.thr_mm);
-        s_rs.make(a.rain, sc->rain_a, sc->rain_b);
-        // the next step applies the rain of [t_previous, t] (HydroPol2D_Main_While.m:721)
-        s_rsn.make(a.rain, sc->t_prev, s_tmin);
-        if (!s_done && s_skip && blk == 0) sc->neg_warn += 1;
-    }
-    __syncthreads();
-    if (s_done) return true;
+    step_begin_strips<R, NT, SOLO, INFL>(a, sh, blk, phase);
+    if (sh.now.done) return true;
 
-    const StepConsts<R> K = s_K;
+    const StepConsts<R> K = sh.K;
     const int ny = a.ny, nx = a.nx;
-    const int cur = s_cur;
-    const bool skip = s_skip != 0;
+    const int cur = sh.now.cur;
+    const R clamp0 = sh.now.skip ? R(0) : R(1e-9);   // depths below are zero (Hydrological_Model.m:45-52)
     const RainStep<R> RS = s_rs;
     const V4* __restrict__ sin = cur ? a.st1 : a.st0;
     V4* __restrict__ sout = cur ? a.st0 : a.st1;
     const V2* __restrict__ gin = cur ? a.gs1 : a.gs0;
     V2* __restrict__ gout = cur ? a.gs0 : a.gs1;
     const V4* __restrict__ stat = a.stat;
-    const R t_arr = R(s_tmin * 60.0 + s_dts);
+    const R t_arr = R(sh.now.t_min * 60.0 + sh.now.dts);
     const R NaNR = R(__int_as_float(0x7fc00000));
 
     const int lane = tid & 31, warp = tid >> 5;
@@ -381,6 +820,8 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
         // the last row's (F) computed it
         R vcar[CPL];
         bool vcar_ok = false;
+        bool lim2 = false;   // lim1 of the row before
+        int map_iy = -1;   // row of the rain map whose interpolation s_map holds
         unsigned mt1[CPL], mt2[CPL];
 #pragma unroll
         for (int h = 0; h < CPL; ++h) {
@@ -432,12 +873,6 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
             fence_proxy_async_smem();   // reads of the ring by an earlier item come first
             for (int k = 0; k < kStages && k <= last_k; ++k) issue(k);
         }
-        V2 nG[CPL];
-#pragma unroll
-        for (int h = 0; h < CPL; ++h) {
-            nG[h] = V2{R(0), R(0)};
-            if (INF && col_ok[h] && r0 - 2 >= 0) nG[h] = gin[size_t(r0 - 2) * nx + j[h]];
-        }
 #pragma unroll kRowUnroll
         for (int k = 0; k <= last_k; ++k) {
             const int r = r0 - 2 + k;
@@ -472,10 +907,35 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
             R hT0[CPL];
             unsigned meta[CPL];
             bool all_dry = true;
+            // rain maps: the rows of the map around this row, and per lane their interpolation at its
+            // columns, made anew only when those rows change (every ny / my rows) and kept in shared
+            // memory (urban 2048^2 with 64 x 64 maps: four gathers and 30 instructions less per cell)
+            R map_wy = R(0);
+            if (MAP && rok) {
+                const MapRow<R> mr = map_row<R>(r, a.rain.my, a.map_sy);
+                map_wy = mr.wy;
+                if (mr.iy0 != map_iy) {
+                    map_iy = mr.iy0;
+#pragma unroll 1
+                    for (int q = 0; q < s_rs.nm; ++q)
+#pragma unroll
+                        for (int h = 0; h < CPL; ++h)
+                            if (col_ok[h])
+                                map_column<R>(a.rain.maps + size_t(s_rs.m[q]) * a.rain.my * a.rain.mx, mr, j[h],
+                                              a.rain.mx, a.map_sx, s_map[q][0][h * NT + tid], s_map[q][1][h * NT + tid]);
+                }
+            }
+            auto rain_row = [&](int h) -> R {   // RainStep::at of this row
+                if (s_rs.nm == 0) return R(0);
+                const R w1 = R(1) - map_wy;
+                R v = s_rs.w[0] * (w1 * s_map[0][0][h * NT + tid] + map_wy * s_map[0][1][h * NT + tid]);
+                if (s_rs.nm > 1) v = v + s_rs.w[1] * (w1 * s_map[1][0][h * NT + tid] + map_wy * s_map[1][1][h * NT + tid]);
+                return v;
+            };
 #pragma unroll
             for (int h = 0; h < CPL; ++h) {
-                const V2 Gs = nG[h];
-                if (INF && col_ok[h] && r + 1 >= 0 && r + 1 < ny) nG[h] = gin[size_t(r + 1) * nx + j[h]];
+                // soil records: the row after next is brought to L1 (a register prefetch spilled)
+                if (INF && col_ok[h] && r + 2 >= 0 && r + 2 < ny) prefetch_l1(gin + (size_t(r + 2) * nx + j[h]));
                 meta[h] = meta_bits(S[h].w);
                 // (A) hydrology of (r, j)
                 hT0[h] = R(0);
@@ -484,14 +944,14 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                     R hh = X[h].x;
                     // a pending map record keeps the depth this step starts from
                     if (s_rec >= 0 && own_lane[h] && own_row) a.rec.snap[size_t(s_rec) * (size_t(ny) * nx) + c] = hh;
-                    // map weights are read from shared memory where they are used
-                    const R rr = MAP ? s_rs.at(a.rain, r, j[h], ny, nx) : RS.depth;
+                    const R rr = MAP ? rain_row(h) : RS.depth;
                     hh = hh + rr;
                     const bool own = own_lane[h] && own_row && r >= a.own_r0 && r < a.own_r1;
                     // uniform rain volume comes from the count of finite cells at the end
                     if (MAP && own && isfinite(hh)) rain_acc_r.add(rr);
                     if (INF) {
                         const unsigned sc = meta[h] & 255u;
+                        const V2 Gs = gin[c];
                         V2 go = Gs;
                         if (sc != 255u) {
                             R Ic = Gs.x, Tc = Gs.y;
@@ -506,9 +966,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                     }
                     // inflow hydrographs after the infiltration (Hydrological_Model.m:27-28)
                     if (INFL) add_inflow(a.inflow, meta[h], hh);
-                    if (!skip && hh < R(1e-9)) hh = R(0);
-                    if (hh < R(0)) hh = R(0);
-                    hT0[h] = hh;
+                    hT0[h] = hh < clamp0 ? R(0) : hh;
                 }
                 all_dry = all_dry && hT0[h] == R(0);
             }
@@ -559,6 +1017,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                         if (SCH) qyp1[h] = X[h].z;
                     }
                     vcar_ok = false;
+                    lim2 = false;
                     continue;
                 }
             }
@@ -568,6 +1027,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                 qxu0[h] = hfx0[h] = qyu0[h] = hfy0[h] = qxl1[h] = qyl1[h] = R(0);
                 sc1[h] = R(1);
             }
+            bool lim1 = false;   // some cell of row r-1 has its faces limited (sc1 != 1)
             if ((dry & 7u) != 7u) {
                 // (B) x face (r, j) between (r, j) and (r, j+1)
                 R hR[CPL];
@@ -586,22 +1046,34 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                     for (int h = 0; h < CPL; ++h)
                         if (!(j[h] >= 1 && j[h] + 1 < nx)) qxa[h] = qxb[h] = R(0);
                 }
-                if constexpr (kFaceIlp<INF, MAP>) {
                 // (B) and (C) interleaved: the geometry of the 2 x CPL faces, then -- unless no
                 // lane of the warp has a wet one -- their momentum updates without branches
                 R Sx[CPL], Sy[CPL], ya[CPL], yb[CPL];
                 bool wx[CPL], wy[CPL];
-                bool any_wet = false;
+                bool any_wet = false, any_rare = false, any_out = false;
 #pragma unroll
                 for (int h = 0; h < CPL; ++h) {
-                    const bool inx = col_ok[h] && rok;
-                    const bool iny = inx && r >= r0 - 1;
-                    R H;
-                    wx[h] = face_geom<R, true>(hT0[h], hR[h], S[h].x, H, Sx[h], K) && inx;
-                    hfx0[h] = inx ? H : R(0);
-                    wy[h] = face_geom<R, false>(hT1[h], hT0[h], S[h].y, H, Sy[h], K) && iny;
-                    hfy0[h] = iny ? H : R(0);
+                    wx[h] = face_open<R, true>(hT0[h], hR[h], S[h].x, hfx0[h], Sx[h], K);
+                    wy[h] = face_open<R, false>(hT1[h], hT0[h], S[h].y, hfy0[h], Sy[h], K);
+                    any_out = any_out || !(wx[h] && wy[h] && col_ok[h]);
+                }
+                if (__any_sync(FULL, any_out) || !rok || r < r0 - 1) {   // the grid's edges and idx_nan cells
+#pragma unroll
+                    for (int h = 0; h < CPL; ++h) {
+                        const bool inx = col_ok[h] && rok;
+                        const bool iny = inx && r >= r0 - 1;
+                        hfx0[h] = !inx ? R(0) : wx[h] ? hfx0[h] : face_closed(hT0[h], hR[h], S[h].x);
+                        hfy0[h] = !iny ? R(0) : wy[h] ? hfy0[h] : face_closed(hT1[h], hT0[h], S[h].y);
+                        wx[h] = wx[h] && inx;
+                        wy[h] = wy[h] && iny;
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < CPL; ++h) {
+                    wx[h] = wx[h] && hfx0[h] > R(0);
+                    wy[h] = wy[h] && hfy0[h] > R(0);
                     any_wet = any_wet || wx[h] || wy[h];
+                    any_rare = any_rare || (wx[h] && below_normal(hfx0[h])) || (wy[h] && below_normal(hfy0[h]));
                     ya[h] = yb[h] = R(0);
                     // schemes 2/3: the previous q_y of rows r-1 (kept from the row before) and r+1
                     if (SCH && wy[h] && r >= 1 && r + 1 < ny) {
@@ -610,48 +1082,60 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                     }
                 }
                 if (__any_sync(FULL, any_wet)) {
+                    R px[CPL], py[CPL];   // H^(7/3)
 #pragma unroll
                     for (int h = 0; h < CPL; ++h) {
-                        qxu0[h] = face_momentum<R, SCH>(wx[h], hfx0[h], Sx[h], X[h].y, S[h].z, K, a.flag_critical,
-                                                         a.scheme, SCH ? qxa[h] : R(0), SCH ? qxb[h] : R(0));
-                        qyu0[h] = face_momentum<R, SCH>(wy[h], hfy0[h], Sy[h], X[h].z, S[h].z, K, a.flag_critical,
-                                                         a.scheme, ya[h], yb[h]);
+                        px[h] = pow73_normal(hfx0[h]);
+                        py[h] = pow73_normal(hfy0[h]);
                     }
-                }
-                } else {
+                    if (__any_sync(FULL, any_rare)) {
 #pragma unroll
-                for (int h = 0; h < CPL; ++h)
-                    if (col_ok[h] && rok)
-                        face_flux<R, true, SCH>(hT0[h], hR[h], S[h].x, X[h].y, S[h].z, K, a.flag_critical, hfx0[h],
-                                                qxu0[h], a.scheme, SCH ? qxa[h] : R(0), SCH ? qxb[h] : R(0));
-                // (C) y face (r, j) between (r-1, j) and (r, j); schemes 2/3 read the previous
-                // q_y of rows r-1 (kept from the row before) and r+1 (from memory)
-#pragma unroll
-                for (int h = 0; h < CPL; ++h)
-                    if (col_ok[h] && rok && r >= r0 - 1) {
-                        R ya = R(0), yb = R(0);
-                        if (SCH && r >= 1 && r + 1 < ny) {
-                            ya = qyp1[h];
-                            yb = sin[size_t(r + 1) * nx + j[h]].z;
+                        for (int h = 0; h < CPL; ++h) {
+                            if (wx[h] && below_normal(hfx0[h])) px[h] = pow73_any(hfx0[h]);
+                            if (wy[h] && below_normal(hfy0[h])) py[h] = pow73_any(hfy0[h]);
                         }
-                        face_flux<R, false, SCH>(hT1[h], hT0[h], S[h].y, X[h].z, S[h].z, K, a.flag_critical, hfy0[h],
-                                                 qyu0[h], a.scheme, ya, yb);
+                    }
+#pragma unroll
+                    for (int h = 0; h < CPL; ++h) {
+                        qxu0[h] = face_update<R, SCH>(wx[h], hfx0[h], px[h], Sx[h], X[h].y, S[h].z, K, a.flag_critical,
+                                                       a.scheme, SCH ? qxa[h] : R(0), SCH ? qxb[h] : R(0));
+                        qyu0[h] = face_update<R, SCH>(wy[h], hfy0[h], py[h], Sy[h], X[h].z, S[h].z, K, a.flag_critical,
+                                                       a.scheme, ya[h], yb[h]);
                     }
                 }
-                // (D) donor scale of (r-1, j)
-                R qxu1_left[CPL];
+                // (D) which cells of row r-1 have their faces limited
+                R qxu1_left[CPL], out[CPL];
                 left_of<R, CPL>(qxu1, qxu1_left, lane);
                 const bool drow = r >= r0 && r - 1 >= 0 && r - 1 < ny;
-#pragma unroll
-                for (int h = 0; h < CPL; ++h)
-                    if (col_ok[h] && drow) sc1[h] = donor_scale_finite(qxu1[h], qxu1_left[h], qyu1[h], qyu0[h], hT1[h], K);
-                // (E) limited faces of row r-1
-                R sc1_right[CPL];
-                right_of<R, CPL>(sc1, sc1_right, lane);
+                bool lim = false;
 #pragma unroll
                 for (int h = 0; h < CPL; ++h) {
-                    qxl1[h] = limit_face_finite(qxu1[h], sc1[h], sc1_right[h]);
-                    qyl1[h] = limit_face_finite(qyu1[h], sc1[h], sc2[h]);
+                    out[h] = donor_out(qxu1[h], qxu1_left[h], qyu1[h], qyu0[h]);
+                    lim = lim || (col_ok[h] && out[h] > hT1[h] * K.dx_over_dt);
+                }
+                lim1 = drow && __any_sync(FULL, lim);
+                if (lim1) {
+#pragma unroll
+                    for (int h = 0; h < CPL; ++h) {
+                        const R avail = hT1[h] * K.dx_over_dt;
+                        if (col_ok[h] && out[h] > avail) sc1[h] = avail / out[h];
+                    }
+                }
+                // (E) limited faces of row r-1
+                if (lim1 || lim2) {
+                    R sc1_right[CPL];
+                    right_of<R, CPL>(sc1, sc1_right, lane);
+#pragma unroll
+                    for (int h = 0; h < CPL; ++h) {
+                        qxl1[h] = limit_by(qxu1[h], sc1[h], sc1_right[h]);
+                        qyl1[h] = limit_by(qyu1[h], sc1[h], sc2[h]);
+                    }
+                } else {
+#pragma unroll
+                    for (int h = 0; h < CPL; ++h) {
+                        qxl1[h] = qxu1[h];
+                        qyl1[h] = qyu1[h];
+                    }
                 }
             }
             // (F) continuity, outlet, maxima and CFL of row r-2.  When rows r-3..r-1 are dry
@@ -688,7 +1172,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                         R hn = quiet ? h_in + R(0) : continuity(h_in, qxl2_left[h], qxl2[h], qyl2[h], qyl1[h], K);
                         const R negtol = -K.tol;
                         R hf3 = R(0);
-                        const unsigned ord = outlet_ord(mt2[h]);
+                        const unsigned ord = INFL ? outlet_ord(mt2[h]) : mt2[h] >> 8;
                         if (act && ord) {
                             const int o = int(ord) - 1;
                             R ho;
@@ -701,7 +1185,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                             // infiltrating soils) stays negative after the next rain
                             // (Hydrological_Model.m:45-50); only outlet cells can end negative
                             if (mine && !(a.ga && (mt2[h] & 255u) != 255u) &&
-                                hn + (MAP ? s_rsn.at(a.rain, rm2, j[h], ny, nx) : s_rsn.depth) < R(-1e-11))
+                                hn + (MAP ? rain_at_cell(a, s_rsn, rm2, j[h]) : s_rsn.depth) < R(-1e-11))
                                 s_negn = 1;   // rare: kept in shared memory, not a register
                         }
                         // stage hydrograph: the cell's depth becomes the gauge's stage
@@ -726,30 +1210,28 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
     #pragma unroll
                     for (int h = 0; h < CPL; ++h) vras[h] = R(0);
                     if (!quiet && mine) {
-                        const R big = R(1e9);
     #pragma unroll
                         for (int h = 0; h < CPL; ++h) {
                             const bool act = own_lane[h];
-                            const R vr = qxl2[h] == R(0) ? qxl2[h] : qdiv(qxl2[h], hfx2[h] < K.tol ? big : hfx2[h]);
+                            const R vr = face_velocity(qxl2[h], hfx2[h], K);
                             R vu;
                             if (vcar_ok) vu = vcar[h];
-                            else vu = qyl2[h] == R(0) ? qyl2[h] : qdiv(qyl2[h], hfy2[h] < K.tol ? big : hfy2[h]);
-                            const R vb = qyl1[h] == R(0) ? qyl1[h] : qdiv(qyl1[h], hfy1[h] < K.tol ? big : hfy1[h]);
+                            else vu = face_velocity(qyl2[h], hfy2[h], K);
+                            const R vb = face_velocity(qyl1[h], hfy1[h], K);
                             vcar[h] = vb;
                             if (INFL) vras[h] = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb));
-                            const R rc = j[h] == 0 ? R(0.5) * vr : vr;
+                            const R rc = vr * (j[h] == 0 ? R(0.5) : R(1));
                             const R uc = R(0.5) * (vu + vb);
                             const R s2 = rc * rc + uc * uc;
                             if (act) s2max = fmax(s2max, s2);
-                            const R dts = fmax(fmax(hfx2[h], hfy2[h]), hf3_[h]);
-                            R cval;
-                            if (a.adaptive == 1) {
-                                cval = K.g * fmax(dts, R(0));
-                            } else {
+                            // the largest depth of a moving cell; its celerity is taken at the end (the
+                            // product by g is monotone)
+                            R dts = fmax(fmax(hfx2[h], hfy2[h]), hf3_[h]);
+                            if (a.adaptive != 1) {
                                 const R wc = fmax(sqrt(K.g * fmax(dts, R(0))), R(1e-10));
-                                cval = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb)) + wc;
+                                dts = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb)) + wc;
                             }
-                            if (act && s2 >= a.stag_s2) cmaxv = fmax(cmaxv, cval);
+                            if (act && s2 >= a.stag_s2) cmaxv = fmax(cmaxv, dts);
                         }
                     }
     #pragma unroll
@@ -794,7 +1276,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                         R hn = quiet ? h_in + R(0) : continuity(h_in, qxl2_left[h], qxl2[h], qyl2[h], qyl1[h], K);
                         const R negtol = -K.tol;
                         R hf3 = R(0);
-                        const unsigned ord = outlet_ord(mt2[h]);
+                        const unsigned ord = INFL ? outlet_ord(mt2[h]) : mt2[h] >> 8;
                         if (ord) {
                             const int o = int(ord) - 1;
                             R ho;
@@ -807,7 +1289,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                             // infiltrating soils) stays negative after the next rain
                             // (Hydrological_Model.m:45-50); only outlet cells can end negative
                             if (mine && !(a.ga && (mt2[h] & 255u) != 255u) &&
-                                hn + (MAP ? s_rsn.at(a.rain, rm2, j[h], ny, nx) : s_rsn.depth) < R(-1e-11))
+                                hn + (MAP ? rain_at_cell(a, s_rsn, rm2, j[h]) : s_rsn.depth) < R(-1e-11))
                                 s_negn = 1;   // rare: kept in shared memory, not a register
                         }
                         // stage hydrograph: the cell's depth becomes the gauge's stage
@@ -828,28 +1310,24 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                         // refreshing_timestep.m:61-89, :139-150, :181-238 for this cell
                         R vras = R(0);   // velocity raster: largest |face velocity| (refreshing_timestep.m:109-111)
                         if (!quiet && mine) {
-                            const R big = R(1e9);
-                            const R vr = qxl2[h] == R(0) ? qxl2[h] : qdiv(qxl2[h], hfx2[h] < K.tol ? big : hfx2[h]);
+                            const R vr = face_velocity(qxl2[h], hfx2[h], K);
                             R vu;
                             if (vcar_ok) vu = vcar[h];
-                            else vu = qyl2[h] == R(0) ? qyl2[h] : qdiv(qyl2[h], hfy2[h] < K.tol ? big : hfy2[h]);
-                            const R vb = qyl1[h] == R(0) ? qyl1[h] : qdiv(qyl1[h], hfy1[h] < K.tol ? big : hfy1[h]);
+                            else vu = face_velocity(qyl2[h], hfy2[h], K);
+                            const R vb = face_velocity(qyl1[h], hfy1[h], K);
                             vcar[h] = vb;
                             if (INFL) vras = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb));
-                            const R rc = j[h] == 0 ? R(0.5) * vr : vr;
+                            const R rc = vr * (j[h] == 0 ? R(0.5) : R(1));
                             const R uc = R(0.5) * (vu + vb);
                             const R s2 = rc * rc + uc * uc;
                             s2max = fmax(s2max, s2);
                             if (s2 >= a.stag_s2) {
-                                const R dts = fmax(fmax(hfx2[h], hfy2[h]), hf3);
-                                R cval;
-                                if (a.adaptive == 1) {
-                                    cval = K.g * fmax(dts, R(0));
-                                } else {
+                                R dts = fmax(fmax(hfx2[h], hfy2[h]), hf3);
+                                if (a.adaptive != 1) {
                                     const R wc = fmax(sqrt(K.g * fmax(dts, R(0))), R(1e-10));
-                                    cval = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb)) + wc;
+                                    dts = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb)) + wc;
                                 }
-                                cmaxv = fmax(cmaxv, cval);
+                                cmaxv = fmax(cmaxv, dts);
                             }
                         }
                         V4 o4;
@@ -873,6 +1351,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                 }
             }
             vcar_ok = !quiet && mine && frow;
+            lim2 = lim1;
             if (flg && lane == 0) dfl[r - 2] = 0;   // rewritten: no longer known dry
             // (G) shift the window down one row
 #pragma unroll
@@ -896,211 +1375,12 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
         }  // !blk_skip
     }
 
-    // ---- CTA reductions ---------------------------------------------------------------
-    // (the last CTA reads only the step accumulators, which thread 0 publishes before its
-    // ticket; the state records reach the next launch through the kernel boundary)
-    rain_acc += rain_acc_r.value();
-    inf_acc += inf_acc_r.value();
-    out_acc += out_acc_r.value();
-    const int lane_ = tid & 31, warp_ = tid >> 5;
-    s2max = warp_max(s2max);
-    // 0: no non-stagnant cell; else the bits of the (non-negative, +0 for -0) maximum + 1
-    unsigned long long cenc = cmaxv >= R(0) ? ord_bits(cmaxv + R(0)) + 1ull : 0ull;
-    cenc = warp_max_u(cenc);
-    rain_acc = warp_sum(rain_acc);
-    inf_acc = warp_sum(inf_acc);
-    out_acc = warp_sum(out_acc);
-    const int to_any = __any_sync(0xffffffffu, timed_out);
-    nbad = __reduce_add_sync(0xffffffffu, nbad);
-    if (lane_ == 0) {
-        red_bad[warp_] = nbad;
-        red_s2[warp_] = s2max;
-        red_c[warp_] = cenc;
-        red_d[0][warp_] = rain_acc;
-        red_d[1][warp_] = inf_acc;
-        red_d[2][warp_] = out_acc;
-        red_to[warp_] = to_any;
-    }
-    __syncthreads();
-    const int negn = s_negn;
-    if (tid == 0) {
-        int to = 0;
-        for (int w = 0; w < NT / 32; ++w) to |= red_to[w];
-        if (to) atomicOr(&a.sc->status, kStatusTimeout);   // a row copy did not arrive in time
-        unsigned bad = 0u;
-        for (int w = 0; w < NT / 32; ++w) bad += red_bad[w];
-        if (bad) atomicAdd(&a.sc->acc_bad, (unsigned long long)bad);
-        for (int w = 1; w < NT / 32; ++w) {
-            s2max = fmax(s2max, red_s2[w]);
-            cenc = red_c[w] > cenc ? red_c[w] : cenc;
-            rain_acc += red_d[0][w];
-            inf_acc += red_d[1][w];
-            out_acc += red_d[2][w];
-        }
-        StepScalars* sc = a.sc;
-        if (s2max > R(0)) atomicMax(&sc->acc_vmax, ord_bits(s2max));
-        if (cenc) atomicMax(&sc->acc_cmax, cenc);
-        if (rain_acc != 0.0) atomicAdd(&sc->acc_rain, rain_acc);
-        if (inf_acc != 0.0) atomicAdd(&sc->acc_inf, inf_acc);
-        if (out_acc != 0.0) atomicAdd(&sc->acc_out, out_acc);
-        if (negn) atomicOr(&sc->skip_next, 1);
-        if (INFL && s_stage != 0.0) atomicAdd(&sc->acc_stage, s_stage);
-        if (s_skipw) atomicAdd(&sc->skipped_cells, (unsigned long long)s_skipw);
-        if (s_skipr) atomicAdd(&sc->skipped_read_cells, (unsigned long long)s_skipr);
-        __threadfence();
-        const unsigned int ticket = atomicAdd(&sc->counter, 1u);
-        s_last = (ticket == a.n_ctas - 1);
-    }
-    __syncthreads();
-    bool cta_ok = true;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) cta_ok = cta_ok && red_to[w] == 0;
-    if (!s_last) return cta_ok;
-
-    // ---- last CTA: refreshing_timestep + clock (HydroPol2D_Main_While.m:691-705, :779)
-    __threadfence();
-    // a rejected step commits nothing: the state stays in buffer cur, the clock, counters and
-    // volumes stay, and the launches halt until the host has prepared the retry
-    // (HydroPol2D_Main_While.m:926-993); s_last doubles as the verdict for the CTA below
-    if (tid == 0) {
-        StepScalars* sc = a.sc;
-        bool reject = (atomicAdd(&sc->status, 0u) & kStatusTimeout) != 0u;
-        if (atomicAdd(&sc->acc_bad, 0ull) > sc->n_bad0) {
-            reject = true;
-            sc->status |= kStatusNumerical;
-        }
-        if (sc->fault_n > 0 && sc->k == sc->fault_k) {   // the host's test hook
-            sc->fault_n -= 1;
-            reject = true;
-            sc->status |= kStatusNumerical;
-        }
-        if (reject) {
-            sc->halted = 1;
-            if (s_skip) sc->neg_warn -= 1;   // the attempt's clamp warning is withdrawn
-            sc->acc_vmax = 0ull;
-            sc->acc_cmax = 0ull;
-            sc->acc_rain = 0.0;
-            sc->acc_inf = 0.0;
-            sc->acc_out = 0.0;
-            sc->acc_stage = 0.0;
-            sc->acc_bad = 0ull;
-            sc->counter = 0u;
-            atomicExch(&sc->skip_next, 0);
-            s_last = 0;
-        }
-    }
-    __syncthreads();
-    if (!s_last) return cta_ok;
-    if (tid == 0) {
-        StepScalars* sc = a.sc;
-        const unsigned long long vbits = atomicAdd(&sc->acc_vmax, 0ull);
-        const unsigned long long cbits = atomicAdd(&sc->acc_cmax, 0ull);
-        const R vR = sqrt(bits_to<R>(vbits));
-        double vm = double(vR);
-        double cm = 0.0;
-        if (cbits) {
-            const R v = bits_to<R>(cbits - 1ull);
-            cm = a.adaptive == 1 ? double(fmax(sqrt(v), R(1e-10))) : double(v);
-        }
-        double rain_s = atomicAdd(&sc->acc_rain, 0.0);
-        // uniform rain: the same depth on every cell with a finite depth
-        if (a.rain.n_uniform) rain_s += double(s_rs.depth) * double(sc->n_finite);
-        const double inf_s = atomicAdd(&sc->acc_inf, 0.0);
-        const double out_s = atomicAdd(&sc->acc_out, 0.0);
-        const double t = s_tmin;
-        const double pos_save = ceil((t * 60.0) / a.tsc);
-        const double time_save = (pos_save - 1.0) * a.tsc / 60.0;
-        const double delta = time_save - sc->tsp;
-        sc->tsp = time_save;
-        double tcr = sc->time_step * 60.0;   // refreshing_timestep.m:361-365
-        sc->last_vbits = vbits;
-        sc->last_cbits = cbits;
-        sc->last_refreshed = 0;
-        sc->last_unstable = 0;
-        if ((delta > 0 || sc->k == 1) &&
-            (sc->refresh_every <= 1 || sc->k == 1 || (sc->k - 1) % sc->refresh_every == 0)) {
-            tcr = finalize_dt(vm, cm, a.res, a.alfa_min, a.alfa_max, a.min_dt, sc->max_dt, a.inc,
-                              a.flag_timestep);
-            sc->vmax_last = vm;
-            sc->last_refreshed = 1;
-            sc->last_unstable = tcr == a.min_dt;
-            if (tcr == a.min_dt) {   // refreshing_timestep.m:357-359 (unstable)
-                sc->unstable += 1;
-                if (sc->dt_floor_stop) {
-                    sc->status |= kStatusDtFloor;
-                    sc->halted = 1;   // this step is kept; the next launches wait for the host
-                }
-            }
-        }
-        const double area = a.res * a.res;
-        sc->rain_vol += rain_s * area;
-        sc->inf_vol += inf_s * area;
-        sc->out_vol += out_s * area;
-        if (a.inflow.n_gauges) {   // every cell of a gauge with a finite elevation got its depth
-            double v = 0.0;
-            for (int g = 0; g < a.inflow.n_gauges; ++g) v += double(a.inflow.depth[g]) * a.inflow.gauge_cells[g];
-            sc->inflow_vol += v * area;
-        }
-        if (a.inflow.n_stage) {
-            sc->stage_vol += __ldcg(&sc->acc_stage) * area;
-            sc->acc_stage = 0.0;
-        }
-        if (INFL && a.strct.n) {   // the structures' extras this step applied
-            double v = 0.0;
-            for (int q = 0; q < a.strct.n_slots; ++q) v += double(a.strct.extra[q]) * area;
-            sc->struct_vol += v;
-        }
-        // the next step's rain: update_spatial_BC over [t_previous, t]
-        // (HydroPol2D_Main_While.m:721), then t_previous <- the clock increment on the first
-        // step and t after it (:734-738), and the clock advances by the new step (:779)
-        sc->rain_a = sc->t_prev;
-        sc->rain_b = t;
-        sc->t_prev = sc->k == 1 ? tcr / 60.0 : t;
-        if (a.rec.n_times > 0) {   // save_output_maps.m:25-27 with t_save = t + new dt (:740)
-            if (sc->rec_pending) { sc->rec_count += 1; sc->rec_pending = 0; }   // recorded by this step
-            const int idx = last_record_below(a.rec.times, a.rec.n_times, t + tcr / 60.0);
-            if (idx > sc->rec_last && a.rec.n_slots > 0) {
-                sc->rec_pending = 1;
-                a.rec.snap_t[sc->rec_count % a.rec.n_slots] = t;
-            }
-            if (idx > sc->rec_last) sc->rec_last = idx;
-        }
-        sc->time_step = tcr / 60.0;
-        sc->t_min = tcr / 60.0 + t;
-        sc->k += 1;
-        sc->cur = cur ^ 1;
-        sc->acc_vmax = 0ull;
-        sc->acc_cmax = 0ull;
-        sc->acc_rain = 0.0;
-        sc->acc_inf = 0.0;
-        sc->acc_out = 0.0;
-        sc->acc_bad = 0ull;
-        sc->counter = 0u;
-        sc->skip_clamp = atomicExch(&sc->skip_next, 0);   // gathered by every CTA's outlets
-    }
-    if (a.inflow.n_gauges || a.inflow.n_stage) {   // the next step's gauge depths and stages
-        __syncthreads();
-        const double ra = a.sc->rain_a, rb = a.sc->rain_b, tn = a.sc->t_min;
-        for (int g = tid; g < a.inflow.n_gauges; g += NT)
-            a.inflow.depth[g] = R(inflow_integral(a.inflow, g, ra, rb) / 60000.0);
-        for (int g = tid; g < a.inflow.n_stage; g += NT) a.inflow.stage_now[g] = R(stage_at(a.inflow, g, tn));
-    }
-    if constexpr (INFL) {
-        if (a.strct.n) {   // the next step's structure transfers, from its d_tot
-            __syncthreads();
-            __shared__ StepConsts<R> s_Kn;
-            __shared__ int s_skn;
-            __shared__ double s_tsn;
-            if (tid == 0) {
-                s_tsn = a.sc->time_step;
-                s_Kn.make(s_tsn * 60.0, a.res, a.tol_mm, a.thr_mm);
-                s_skn = a.sc->skip_clamp;
-            }
-            __syncthreads();
-            structure_prepare<R, INF, MAP, INFL>(a, s_rsn, s_skn != 0, s_Kn, sout, gout, tid, NT, s_tsn);
-        }
-    }
-    return cta_ok;
+    if (a.adaptive == 1 && cmaxv >= R(0)) cmaxv = K.g * cmaxv;
+    if (MAP) rain_acc += rain_acc_r.value();
+    if (INF) inf_acc += inf_acc_r.value();
+    if (out_acc_r.any()) out_acc += out_acc_r.value();
+    return step_finish<R, NT, INF, MAP, INFL, SOLO>(a, sh, rain_acc, inf_acc, out_acc, s2max, cmaxv, nbad, timed_out,
+                                                    phase, sout, gout);
 }
 
 // Rain maps from gauges by inverse-distance weighting, one full-resolution map per record
@@ -1320,8 +1600,24 @@ __global__ void k_struct_prime(const FusedArgs<R> a) {
 }
 
 template <typename R, int NT, int INF, bool MAP, int CPL = 1, bool INFL = false, int SCH = 0>
-__global__ void __launch_bounds__(NT, FusedOcc<R, CPL>::minb) k_fused_step(const FusedArgs<R> a) {
-    fused_item<R, NT, INF, MAP, CPL, INFL, SCH>(a, blockIdx.x);
+__global__ void __launch_bounds__(NT, FusedOcc<R, CPL>::minb) k_fused_step(const __grid_constant__ FusedArgs<R> a, int phase) {
+    fused_item<R, NT, INF, MAP, CPL, INFL, SCH, true>(a, blockIdx.x, phase);
+}
+
+// a step's launch, allowed to begin before the launch before it has ended (step_begin waits)
+template <typename K, typename... A>
+inline void launch_step(K kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // ---- batched ensemble ----------------------------------------------------------------
@@ -1414,7 +1710,7 @@ k_ens_step(const FusedArgs<R>* __restrict__ members, int n_members, const unsign
             for (int w = tid; w < int(sizeof(FusedArgs<R>) / 4); w += NT) dst[w] = src[w];
         }
         __syncthreads();
-        if (!fused_item<R, NT, INF, MAP, CPL, INFL, SCH>(s_a, s_local)) return;   // ring unusable after a timeout
+        if (!fused_item<R, NT, INF, MAP, CPL, INFL, SCH, false>(s_a, s_local, 0)) return;   // ring unusable after a timeout
     }
 }
 

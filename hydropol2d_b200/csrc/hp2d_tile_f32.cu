@@ -1,0 +1,7 @@
+// Instantiations of the tile step (hp2d_tile.cuh) for float.
+#define HP2D_TILE_INSTANTIATE
+#include "hp2d_tile.cuh"
+
+namespace hp2d {
+template void launch_tile_step<float>(const FusedArgs<float>&, int, bool, bool, bool, int, cudaStream_t);
+}
