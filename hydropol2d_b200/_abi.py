@@ -59,7 +59,7 @@ NN_EXPORTS = [
     "hp2d_nn_gemm", "hp2d_nn_conv3x3", "hp2d_nn_check", "hp2d_nn_error", "hp2d_nn_im2col3x3", "hp2d_nn_transpose",
     "hp2d_nn_maxpool2", "hp2d_nn_maxpool2_bwd", "hp2d_nn_upsample2", "hp2d_nn_upsample2_bwd",
     "hp2d_nn_copy_channels", "hp2d_nn_relu_bwd", "hp2d_nn_colsum", "hp2d_nn_mse", "hp2d_nn_adam",
-    "hp2d_nn_flip3x3", "hp2d_nn_f32_to_bf16",
+    "hp2d_nn_flip3x3", "hp2d_nn_f32_to_bf16", "hp2d_nn_conv3x3_any", "hp2d_nn_conv3x3_wgrad", "hp2d_nn_relu_colsum",
 ]
 
 NN_EPI = {"f32": 0, "f32_atomic": 1, "bf16_bias_relu": 2, "bf16_bias": 3, "f32_bias": 4}
@@ -198,6 +198,9 @@ def lib() -> C.CDLL:
     sig.update({
         "hp2d_nn_gemm": ([i32, i32, i32, vp, i32, vp, i32, vp, i32, vp, i32, i32, vp], C.c_int),
         "hp2d_nn_conv3x3": ([vp, i32, i32, i32, i32, vp, i32, i32, vp, vp, i32, i32, vp], C.c_int),
+        "hp2d_nn_conv3x3_any": ([vp, i32, i32, i32, i32, vp, i32, i32, vp, vp, i32, i32, vp], C.c_int),
+        "hp2d_nn_conv3x3_wgrad": ([vp, i32, i32, i32, i32, vp, i32, vp, i32, vp], C.c_int),
+        "hp2d_nn_relu_colsum": ([vp, vp, i64, i32, vp, vp], C.c_int),
         "hp2d_nn_check": ([], C.c_int),
         "hp2d_nn_error": ([], C.c_char_p),
         "hp2d_nn_im2col3x3": ([vp, i32, i32, i32, i32, vp, i32, i32, vp], C.c_int),

@@ -8,11 +8,12 @@
 
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "hp2d.h"
 #include "hp2d_nn.h"
-#include "hp2d_nn_gemm.cuh"
+#include "hp2d_nn_conv.cuh"
 
 using namespace hp2d;
 using namespace hp2d::nn;
@@ -55,20 +56,23 @@ bool make_map(CUtensorMap* m, const void* base, int rows, int K, int ld, int box
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// NHWC BF16 activations [B, H, W, C] as a 4-D map (C innermost); box kb channels x
-// min(W, 128) pixels x 128/min(W,128) rows x 1 image = the 128 pixels of one GEMM tile.
-// Coordinates outside the image read as zeros (the convolution's padding).
-bool make_map_nhwc(CUtensorMap* m, const void* base, int B, int H, int W, int C, int kb) {
+// NHWC BF16 activations [B, H, W, C] as a 4-D map (C innermost), boxes of kb channels x bw x bh
+// pixels of one image; 128-byte swizzle for 64 channels, 64-byte for 32.  Coordinates outside the
+// image read as zeros (the convolution's padding).
+bool make_map_nhwc(CUtensorMap* m, const void* base, int B, int H, int W, int C, int kb, int bw = kTX, int bh = kTY) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
-    const int bw = W < kBM ? W : kBM;
     cuuint64_t dims[4] = {cuuint64_t(C), cuuint64_t(W), cuuint64_t(H), cuuint64_t(B)};
     cuuint64_t strides[3] = {cuuint64_t(C) * 2, cuuint64_t(W) * C * 2, cuuint64_t(H) * W * C * 2};
-    cuuint32_t box[4] = {cuuint32_t(kb), cuuint32_t(bw), cuuint32_t(kBM / bw), 1};
+    cuuint32_t box[4] = {cuuint32_t(kb), cuuint32_t(bw), cuuint32_t(bh), 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, kb == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+TileGeom tile_geom(int B, int H, int W) {
+    const int tx = (W + kTX - 1) / kTX, ty = (H + kTY - 1) / kTY;
+    return TileGeom{H, W, tx, ty, B * tx * ty};
 }
 
 hp2d_status fail(const std::string& msg, hp2d_status st = HP2D_INVALID_ARG) {
@@ -168,7 +172,7 @@ hp2d_status gemm_bn(int M, int N, int K, const void* A, int lda, const void* B, 
     int* err = err_ptr();
     if (!err) return fail("cannot resolve the error flag", HP2D_CUDA_ERROR);
     return launch_tiles<BN, kBK, false>(ma, mb, M, N, kt, per, (M + kBM - 1) / kBM, (N + BN - 1) / BN, splits, C,
-                                        ldc, bias, epi, err, ConvGeom{0, 0, 0}, st);
+                                        ldc, bias, epi, err, ConvGeom{}, st);
 }
 
 template <int BN, int KB>
@@ -181,8 +185,9 @@ hp2d_status conv_bn(const void* x, int B, int H, int W, int Cin, const void* w, 
     if (!err) return fail("cannot resolve the error flag", HP2D_CUDA_ERROR);
     const int M = B * H * W;
     const int kt = 9 * Cin / KB;
-    return launch_tiles<BN, KB, true>(ma, mb, M, Co, kt, kt, M / kBM, (Co + BN - 1) / BN, 1, y, ldy, bias, epi, err,
-                                      ConvGeom{H, W, Cin / KB}, st);
+    const TileGeom g = tile_geom(B, H, W);
+    return launch_tiles<BN, KB, true>(ma, mb, M, Co, kt, kt, g.total, (Co + BN - 1) / BN, 1, y, ldy, bias, epi, err,
+                                      ConvGeom{g, Cin / KB}, st);
 }
 
 template <int KB>
@@ -192,6 +197,94 @@ hp2d_status conv_kb(const void* x, int B, int H, int W, int Cin, const void* w, 
     if (Co <= 64) return conv_bn<64, KB>(x, B, H, W, Cin, w, ldw, Co, bias, y, ldy, epi, st);
     if (Co <= 128) return conv_bn<128, KB>(x, B, H, W, Cin, w, ldw, Co, bias, y, ldy, epi, st);
     return conv_bn<256, KB>(x, B, H, W, Cin, w, ldw, Co, bias, y, ldy, epi, st);
+}
+
+// first use of a kernel on a device: its dynamic shared memory; returns the SM count
+template <typename K> int kernel_setup(K kernel, size_t smem, int (&sms)[64]) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lock(g_launch_init_mutex);
+    if (!sms[dev]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        sms[dev] = sm_count(dev);
+    }
+    return sms[dev];
+}
+
+template <int CB, int BN>
+hp2d_status conv_halo(const void* x, int B, int H, int W, const void* w, int ldw, int Co, const float* bias, void* y,
+                      int ldy, int epi, int* err, cudaStream_t st) {
+    CUtensorMap mx, mw;
+    if (!make_map_nhwc(&mx, x, B, H, W, CB, CB, kHX, kHY) || !make_map(&mw, w, Co, 9 * CB, ldw, BN, CB))
+        return fail("cuTensorMapEncodeTiled rejected an operand (alignment or pitch)");
+    static int sms[64] = {};
+    constexpr size_t smem = conv_smem<CB, BN>();
+    const int n = kernel_setup(k_conv_halo<CB, BN>, smem, sms);
+    if (!n) return launched("cudaFuncSetAttribute");
+    const TileGeom g = tile_geom(B, H, W);
+    const int ctas = std::min(g.total, n * int(std::min<size_t>(227 * 1024 / (smem + 1024), 4)));
+    k_conv_halo<CB, BN><<<ctas, kPtThreads, smem, st>>>(mx, mw, Co, y, ldy, bias, epi, err, g);
+    return launched("k_conv_halo");
+}
+template <int C, int BN>
+hp2d_status conv_small(const uint16_t* x, int B, int H, int W, const void* w, int ldw, int Co, const float* bias, void* y,
+                       int ldy, int epi, int* err, cudaStream_t st) {
+    CUtensorMap mw;
+    if (!make_map(&mw, w, Co, 64, ldw, BN)) return fail("cuTensorMapEncodeTiled rejected the weights (alignment or pitch)");
+    static int sms[64] = {};
+    constexpr size_t smem = kBM * 128 + BN * 128 + 1024;
+    const int n = kernel_setup(k_conv_small<C, BN>, smem, sms);
+    if (!n) return launched("cudaFuncSetAttribute");
+    const TileGeom g = tile_geom(B, H, W);
+    const int per_sm = std::min(8, 512 / BN);
+    k_conv_small<C, BN><<<std::min(g.total, n * per_sm), 128, smem, st>>>(x, mw, Co, y, ldy, bias, epi, err, g);
+    return launched("k_conv_small");
+}
+template <int C>
+hp2d_status conv_small_n(const uint16_t* x, int B, int H, int W, const void* w, int ldw, int Co, const float* bias, void* y,
+                         int ldy, int epi, int* err, cudaStream_t st) {
+    if (Co <= 32) return conv_small<C, 32>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (Co <= 64) return conv_small<C, 64>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    return conv_small<C, 128>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+}
+
+template <int CB, int BN, int SMALL, bool BSMALL>
+hp2d_status wgrad(const uint16_t* x, int B, int H, int W, int Ci, const uint16_t* dy, int Co, float* gW, int ldw, int* err,
+                  cudaStream_t st) {
+    CUtensorMap mx{}, md{};
+    if ((!SMALL && !make_map_nhwc(&mx, x, B, H, W, Ci, CB, kHX, kHY)) || (!BSMALL && !make_map_nhwc(&md, dy, B, H, W, Co, BN)))
+        return fail("cuTensorMapEncodeTiled rejected an operand (alignment or pitch)");
+    static int sms[64] = {};
+    constexpr size_t smem = wgrad_smem<CB, BN, SMALL>();
+    const int n = kernel_setup(k_wgrad<CB, BN, SMALL, BSMALL>, smem, sms);
+    if (!n) return launched("cudaFuncSetAttribute");
+    const TileGeom g = tile_geom(B, H, W);
+    const int ci_blocks = SMALL ? 1 : Ci / CB, units = ci_blocks * ((Co + BN - 1) / BN);
+    // A unit's tiles are split over the SMs, each part adds its sums into gW once.  The tensor core
+    // truncates its sums, so an accumulator's error grows with its chain (2^-24 of it a step): long
+    // chains (beyond 128 steps of 16 pixels) keep the length that the split-K GEMM over pixels has,
+    // 296 parts over its 128 x 256 output tiles.
+    const int kp = (9 * Ci + 63) / 64 * 64;
+    const int gemm_tiles = ((Co + 127) / 128) * (kp > 128 ? (kp + 255) / 256 : 1);
+    int splits = std::max(1, n / units);
+    if (int64_t(B) * H * W > int64_t(splits) * 128 * 16) splits = std::max(1, 2 * n / gemm_tiles);
+    splits = std::min(g.total, splits);
+    k_wgrad<CB, BN, SMALL, BSMALL><<<dim3(splits, units), kPtThreads, smem, st>>>(mx, md, x, dy, Ci, Co, gW, ldw, err, g,
+                                                                                 ci_blocks);
+    return launched("k_wgrad");
+}
+template <int CB, int SMALL>
+hp2d_status wgrad_n(const uint16_t* x, int B, int H, int W, int Ci, const uint16_t* dy, int Co, float* gW, int ldw, int* err,
+                    cudaStream_t st) {
+    // 64 -> 32 channels as two units of 32: their 2 x 98 parts at full resolution fill the GPU two to an
+    // SM, where 98 parts of 64 channels left a third of it idle
+    if constexpr (CB == 64 && SMALL == 0)
+        if (Ci == 64 && Co == 32) return wgrad<32, 32, 0, false>(x, B, H, W, Ci, dy, Co, gW, ldw, err, st);
+    if (Co % 64 == 0) return wgrad<CB, 64, SMALL, false>(x, B, H, W, Ci, dy, Co, gW, ldw, err, st);
+    if (Co % 32 == 0) return wgrad<CB, 32, SMALL, false>(x, B, H, W, Ci, dy, Co, gW, ldw, err, st);
+    return wgrad<CB, 32, SMALL, true>(x, B, H, W, Ci, dy, Co, gW, ldw, err, st);
 }
 
 inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
@@ -382,23 +475,42 @@ __global__ void k_colsum(const uint16_t* __restrict__ dz, int64_t P, int C, int 
     }
 }
 
-__global__ void k_mse(const float* __restrict__ pred, int ldp, const float* __restrict__ t, const float* __restrict__ w,
-                      int64_t P, int nch, float scale, float* loss, uint16_t* __restrict__ dpred, int ldd) {
-    float acc = 0.0f;
+// The loss is summed in FP64 up to a cluster of 8 blocks, then one FP32 atomic each (16 in all): one
+// atomic per warp rounded 38000 times into the running sum, an error of up to 6e-6.
+constexpr int kMseCluster = 8, kMseBlocks = 128;
+__global__ void __cluster_dims__(kMseCluster, 1, 1) __launch_bounds__(512)
+k_mse(const float* __restrict__ pred, int ldp, const float* __restrict__ t, const float* __restrict__ w, int64_t P, int nch,
+      float scale, float* loss, uint16_t* __restrict__ dpred, int ldd) {
+    __shared__ double part[16];
+    __shared__ double block_sum[kMseCluster];
+    double acc = 0.0;
     for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < P; p += int64_t(gridDim.x) * blockDim.x) {
         for (int c = 0; c < ldd; ++c) {
             uint16_t g = 0;
             if (c < nch) {
                 const float d = pred[p * ldp + c] - t[p * nch + c];
                 const float wc = w ? w[p * nch + c] : 1.0f;
-                acc += wc * d * d;
+                acc += double(wc * d * d);
                 g = f2bf(2.0f * wc * d * scale);
             }
             dpred[p * ldd + c] = g;
         }
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && acc != 0.0f) atomicAdd(loss, acc * scale);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    auto cluster = cooperative_groups::this_cluster();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int i = 0; i < 16; ++i) s += part[i];
+        cluster.map_shared_rank(block_sum, 0)[cluster.block_rank()] = s;
+    }
+    cluster.sync();
+    if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+        double s = 0.0;
+        for (int i = 0; i < kMseCluster; ++i) s += block_sum[i];
+        if (s != 0.0) atomicAdd(loss, float(s * double(scale)));
+    }
 }
 
 __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -435,6 +547,142 @@ __global__ void k_flip3x3(const float* __restrict__ w, int Co, int Ci, int Kp, u
 __global__ void k_f32_to_bf16(const float* __restrict__ in, uint16_t* __restrict__ out, int64_t n) {
     for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n; e += int64_t(gridDim.x) * blockDim.x)
         out[e] = f2bf(in[e]);
+}
+
+// ---- the same layers on 16-byte pieces (8 channels): channel counts that are multiples of 8 and
+// aligned bases.  One element per thread and a 64-bit division per element made the layers between
+// the convolutions as expensive as the convolutions (upsampling 16 x 256^2 x 64: 259 us, 0.65 TB/s).
+struct Vec8 {
+    uint32_t w[4];
+    __device__ __forceinline__ float get(int i) const { return __uint_as_float((i & 1) ? (w[i >> 1] & 0xffff0000u) : (w[i >> 1] << 16)); }
+    __device__ __forceinline__ uint32_t bits(int i) const { return (i & 1) ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu; }
+    __device__ __forceinline__ void set(int i, uint32_t b) {
+        w[i >> 1] = (i & 1) ? (w[i >> 1] & 0xffffu) | (b << 16) : (w[i >> 1] & 0xffff0000u) | b;
+    }
+};
+__device__ __forceinline__ Vec8 load8(const uint4* p) {
+    const uint4 u = *p;
+    return Vec8{{u.x, u.y, u.z, u.w}};
+}
+__device__ __forceinline__ void store8(uint4* p, const Vec8& v) { *p = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]); }
+
+// a row of the smaller image per block row (grid-stride), pixels x channel groups across threads
+__global__ void k_maxpool2_v8(const uint4* __restrict__ x, int rows, int W, int C8, uint4* __restrict__ y) {
+    const int Wo = W / 2;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= Wo * C8) return;
+    const int xo = e / C8, c = e - xo * C8;
+    for (int q = blockIdx.y; q < rows; q += gridDim.y) {
+        const uint4* p = x + (size_t(2 * q) * W + 2 * xo) * C8 + c;
+        Vec8 m = load8(p);
+        const size_t offs[3] = {size_t(C8), size_t(W) * C8, size_t(W) * C8 + C8};
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const Vec8 u = load8(p + offs[t]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (u.get(i) > m.get(i)) m.set(i, u.bits(i));
+        }
+        store8(y + size_t(q) * Wo * C8 + e, m);
+    }
+}
+__global__ void k_maxpool2_bwd_v8(const uint4* __restrict__ x, const uint4* __restrict__ y, const uint4* __restrict__ dy,
+                                  int rows, int W, int C8, uint4* __restrict__ dx, int acc) {
+    const int Wo = W / 2;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= Wo * C8) return;
+    const int xo = e / C8, c = e - xo * C8;
+    const size_t offs[4] = {0, size_t(C8), size_t(W) * C8, size_t(W) * C8 + C8};
+    for (int q = blockIdx.y; q < rows; q += gridDim.y) {
+        const size_t i00 = (size_t(2 * q) * W + 2 * xo) * C8 + c;
+        const Vec8 m = load8(y + size_t(q) * Wo * C8 + e), d = load8(dy + size_t(q) * Wo * C8 + e);
+        unsigned routed = 0u;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const Vec8 u = load8(x + i00 + offs[t]);
+            Vec8 o = acc ? load8(dx + i00 + offs[t]) : Vec8{{0u, 0u, 0u, 0u}};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const bool hit = !((routed >> i) & 1u) && u.get(i) == m.get(i);
+                if (hit) {
+                    o.set(i, acc ? uint32_t(f2bf(o.get(i) + d.get(i))) : d.bits(i));
+                    routed |= 1u << i;
+                }
+            }
+            store8(dx + i00 + offs[t], o);
+        }
+    }
+}
+// W, rows: of the smaller image
+__global__ void k_upsample2_v8(const uint4* __restrict__ x, int rows, int W, int C8, uint4* __restrict__ y) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= W * C8) return;
+    const int xi = e / C8, c = e - xi * C8;
+    for (int q = blockIdx.y; q < rows; q += gridDim.y) {
+        const uint4 v = x[size_t(q) * W * C8 + e];
+        uint4* o = y + (size_t(2 * q) * (2 * W) + 2 * xi) * C8 + c;
+        o[0] = v;
+        o[C8] = v;
+        o[size_t(2 * W) * C8] = v;
+        o[size_t(2 * W) * C8 + C8] = v;
+    }
+}
+__global__ void k_upsample2_bwd_v8(const uint4* __restrict__ dy, int rows, int W, int C8, uint4* __restrict__ dx) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= W * C8) return;
+    const int xi = e / C8, c = e - xi * C8;
+    for (int q = blockIdx.y; q < rows; q += gridDim.y) {
+        const uint4* p = dy + (size_t(2 * q) * (2 * W) + 2 * xi) * C8 + c;
+        const Vec8 a = load8(p), b = load8(p + C8), d = load8(p + size_t(2 * W) * C8), f = load8(p + size_t(2 * W) * C8 + C8);
+        Vec8 o;
+#pragma unroll
+        for (int i = 0; i < 8; i += 2)
+            o.w[i / 2] = uint32_t(f2bf((a.get(i) + b.get(i)) + (d.get(i) + f.get(i)))) |
+                         (uint32_t(f2bf((a.get(i + 1) + b.get(i + 1)) + (d.get(i + 1) + f.get(i + 1)))) << 16);
+        store8(dx + size_t(q) * W * C8 + e, o);
+    }
+}
+// n8 channel groups of each pixel; the group of a thread is fixed, pixels grid-stride
+__global__ void k_copy_channels_v8(const uint4* __restrict__ in, int cin8, int c08, int n8, int64_t P, uint4* __restrict__ out,
+                                   int cout8, int o08) {
+    const int c = threadIdx.x % n8, pl = threadIdx.x / n8, per = blockDim.x / n8;
+    if (pl >= per) return;
+    for (int64_t p = int64_t(blockIdx.x) * per + pl; p < P; p += int64_t(gridDim.x) * per)
+        out[p * cout8 + o08 + c] = in[p * cin8 + c08 + c];
+}
+// The ReLU's mask on dy (in place, y null: none) and dy's column sums into out, in one pass: a thread
+// keeps the sums of its 8 channels over its pixels, the block adds its threads' up in shared memory.
+__global__ void __launch_bounds__(256) k_relu_colsum_v8(const uint4* __restrict__ y, uint4* __restrict__ dy, int64_t P, int C8,
+                                                        float* __restrict__ out) {
+    extern __shared__ float s_part[];   // [256 / C8][C8 * 8]
+    const int c = threadIdx.x % C8, pl = threadIdx.x / C8, per = 256 / C8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (pl < per) {
+        for (int64_t p = int64_t(blockIdx.x) * per + pl; p < P; p += int64_t(gridDim.x) * per) {
+            Vec8 d = load8(dy + p * C8 + c);
+            if (y) {
+                const Vec8 v = load8(y + p * C8 + c);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (!(v.get(i) > 0.0f)) d.set(i, 0u);
+                store8(dy + p * C8 + c, d);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] += d.get(i);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s_part[pl * (C8 * 8) + c * 8 + i] = acc[i];
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < C8 * 8; k += 256) {
+        float s = 0.0f;
+        for (int q = 0; q < per; ++q) s += s_part[q * (C8 * 8) + k];
+        atomicAdd(out + k, s);
+    }
+}
+// launch shape of the row kernels: threads over a row's pixels x channel groups
+dim3 row_grid(int64_t rows, int64_t groups) {
+    return dim3(unsigned((groups + 255) / 256), unsigned(std::min<int64_t>(rows, 65535)));
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -521,34 +769,55 @@ hp2d_status hp2d_nn_transpose(const uint16_t* in, int32_t rows, int32_t cols, in
 
 hp2d_status hp2d_nn_maxpool2(const uint16_t* x, int32_t B, int32_t H, int32_t W, int32_t C, uint16_t* y, void* stream) {
     if (!x || !y || H % 2 || W % 2 || B <= 0 || C <= 0) return fail("maxpool2: bad shape");
-    k_maxpool2<<<blocks(int64_t(B) * H * W * C / 4), 256, 0, S(stream)>>>(x, B, H, W, C, y);
+    if (C % 8 == 0 && aligned16(x) && aligned16(y))
+        k_maxpool2_v8<<<row_grid(int64_t(B) * (H / 2), int64_t(W / 2) * (C / 8)), 256, 0, S(stream)>>>(
+            reinterpret_cast<const uint4*>(x), B * (H / 2), W, C / 8, reinterpret_cast<uint4*>(y));
+    else
+        k_maxpool2<<<blocks(int64_t(B) * H * W * C / 4), 256, 0, S(stream)>>>(x, B, H, W, C, y);
     return launched("maxpool2");
 }
 
 hp2d_status hp2d_nn_maxpool2_bwd(const uint16_t* x, const uint16_t* y, const uint16_t* dy, int32_t B, int32_t H,
                                  int32_t W, int32_t C, uint16_t* dx, int32_t accumulate, void* stream) {
     if (!x || !y || !dy || !dx || H % 2 || W % 2) return fail("maxpool2_bwd: bad shape");
-    k_maxpool2_bwd<<<blocks(int64_t(B) * H * W * C / 4), 256, 0, S(stream)>>>(x, y, dy, B, H, W, C, dx, accumulate);
+    if (C % 8 == 0 && B > 0 && aligned16(x) && aligned16(y) && aligned16(dy) && aligned16(dx))
+        k_maxpool2_bwd_v8<<<row_grid(int64_t(B) * (H / 2), int64_t(W / 2) * (C / 8)), 256, 0, S(stream)>>>(
+            reinterpret_cast<const uint4*>(x), reinterpret_cast<const uint4*>(y), reinterpret_cast<const uint4*>(dy),
+            B * (H / 2), W, C / 8, reinterpret_cast<uint4*>(dx), accumulate);
+    else
+        k_maxpool2_bwd<<<blocks(int64_t(B) * H * W * C / 4), 256, 0, S(stream)>>>(x, y, dy, B, H, W, C, dx, accumulate);
     return launched("maxpool2_bwd");
 }
 
 hp2d_status hp2d_nn_upsample2(const uint16_t* x, int32_t B, int32_t H, int32_t W, int32_t C, uint16_t* y, void* stream) {
     if (!x || !y) return fail("upsample2: null");
-    k_upsample2<<<blocks(int64_t(B) * H * W * C * 4), 256, 0, S(stream)>>>(x, B, H, W, C, y);
+    if (C % 8 == 0 && B > 0 && H > 0 && W > 0 && aligned16(x) && aligned16(y))
+        k_upsample2_v8<<<row_grid(int64_t(B) * H, int64_t(W) * (C / 8)), 256, 0, S(stream)>>>(
+            reinterpret_cast<const uint4*>(x), B * H, W, C / 8, reinterpret_cast<uint4*>(y));
+    else
+        k_upsample2<<<blocks(int64_t(B) * H * W * C * 4), 256, 0, S(stream)>>>(x, B, H, W, C, y);
     return launched("upsample2");
 }
 
 hp2d_status hp2d_nn_upsample2_bwd(const uint16_t* dy, int32_t B, int32_t H, int32_t W, int32_t C, uint16_t* dx,
                                   void* stream) {
     if (!dy || !dx) return fail("upsample2_bwd: null");
-    k_upsample2_bwd<<<blocks(int64_t(B) * H * W * C), 256, 0, S(stream)>>>(dy, B, H, W, C, dx);
+    if (C % 8 == 0 && B > 0 && H > 0 && W > 0 && aligned16(dx) && aligned16(dy))
+        k_upsample2_bwd_v8<<<row_grid(int64_t(B) * H, int64_t(W) * (C / 8)), 256, 0, S(stream)>>>(
+            reinterpret_cast<const uint4*>(dy), B * H, W, C / 8, reinterpret_cast<uint4*>(dx));
+    else
+        k_upsample2_bwd<<<blocks(int64_t(B) * H * W * C), 256, 0, S(stream)>>>(dy, B, H, W, C, dx);
     return launched("upsample2_bwd");
 }
 
 hp2d_status hp2d_nn_copy_channels(const uint16_t* in, int32_t cin, int32_t c0, int32_t n, int64_t P, uint16_t* out,
                                   int32_t cout, int32_t o0, void* stream) {
     if (!in || !out || c0 + n > cin || o0 + n > cout || n <= 0) return fail("copy_channels: bad range");
-    k_copy_channels<<<blocks(P * n), 256, 0, S(stream)>>>(in, cin, c0, n, P, out, cout, o0);
+    if (((cin | c0 | n | cout | o0) & 7) == 0 && n <= 2048 && aligned16(in) && aligned16(out))
+        k_copy_channels_v8<<<blocks(P * (n / 8)), 256, 0, S(stream)>>>(reinterpret_cast<const uint4*>(in), cin / 8, c0 / 8,
+                                                                       n / 8, P, reinterpret_cast<uint4*>(out), cout / 8, o0 / 8);
+    else
+        k_copy_channels<<<blocks(P * n), 256, 0, S(stream)>>>(in, cin, c0, n, P, out, cout, o0);
     return launched("copy_channels");
 }
 
@@ -565,10 +834,70 @@ hp2d_status hp2d_nn_colsum(const uint16_t* dz, int64_t P, int32_t C, int32_t ld,
     return launched("colsum");
 }
 
+hp2d_status hp2d_nn_relu_colsum(const uint16_t* y, uint16_t* dy, int64_t P, int32_t C, float* out, void* stream) {
+    if (!dy || !out || P <= 0 || C <= 0) return fail("relu_colsum: bad shape");
+    if (C % 8 == 0 && C <= 2048 && aligned16(dy) && (!y || aligned16(y))) {
+        const int per = 256 / std::min(C / 8, 256);
+        const unsigned grid = unsigned(std::min<int64_t>((P + per - 1) / per, 148 * 4));
+        k_relu_colsum_v8<<<grid, 256, size_t(per) * C * sizeof(float), S(stream)>>>(
+            reinterpret_cast<const uint4*>(y), reinterpret_cast<uint4*>(dy), P, C / 8, out);
+        return launched("relu_colsum");
+    }
+    if (y) {
+        const hp2d_status r = hp2d_nn_relu_bwd(y, dy, P * C, stream);
+        if (r != HP2D_OK) return r;
+    }
+    return hp2d_nn_colsum(dy, P, C, C, out, stream);
+}
+
+hp2d_status hp2d_nn_conv3x3_any(const uint16_t* x, int32_t B, int32_t H, int32_t W, int32_t C, const uint16_t* w,
+                                int32_t ldw, int32_t Co, const float* bias, void* y, int32_t ldy, int32_t epi,
+                                void* stream) {
+    if (!x || !w || !y || B <= 0 || H <= 0 || W <= 0 || Co <= 0 || C <= 0) return fail("conv3x3_any: bad shape");
+    const bool small = C == 1 || C == 2 || C == 4;
+    if ((!small && C % 32) || (small && Co > 128)) return fail("conv3x3_any: unsupported channel counts", HP2D_UNSUPPORTED_FLAG);
+    if (ldw < (small ? 64 : 9 * C) || ldw % 8 || !aligned16(x) || !aligned16(w)) return fail("conv3x3_any: weight pitch or alignment");
+    if (ldy < Co) return fail("conv3x3_any: ldy < Co");
+    if (epi != HP2D_NN_EPI_F32 && epi != HP2D_NN_EPI_BF16_BIAS_RELU && epi != HP2D_NN_EPI_BF16_BIAS &&
+        epi != HP2D_NN_EPI_F32_BIAS)
+        return fail("conv3x3_any: unsupported epilogue");
+    if (epi != HP2D_NN_EPI_F32 && !bias) return fail("conv3x3_any: bias epilogue without bias");
+    int* err = err_ptr();
+    if (!err) return fail("cannot resolve the error flag", HP2D_CUDA_ERROR);
+    cudaStream_t st = S(stream);
+    if (C == 4) return conv_small_n<4>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (C == 2) return conv_small_n<2>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (C == 1) return conv_small_n<1>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    // the weights of up to 64 input and 128 output channels stay in shared memory beside the halo tiles
+    if (C == 32 && Co <= 32) return conv_halo<32, 32>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (C == 32 && Co <= 64) return conv_halo<32, 64>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (C == 64 && Co <= 32) return conv_halo<64, 32>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (C == 64 && Co <= 64) return conv_halo<64, 64>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (C == 64 && Co <= 128) return conv_halo<64, 128>(x, B, H, W, w, ldw, Co, bias, y, ldy, epi, err, st);
+    if (C % 64 == 0) return conv_kb<64>(x, B, H, W, C, w, ldw, Co, bias, y, ldy, epi, st);
+    return conv_kb<32>(x, B, H, W, C, w, ldw, Co, bias, y, ldy, epi, st);
+}
+
+hp2d_status hp2d_nn_conv3x3_wgrad(const uint16_t* x, int32_t B, int32_t H, int32_t W, int32_t C, const uint16_t* dy,
+                                  int32_t Co, float* gw, int32_t ldw, void* stream) {
+    if (!x || !dy || !gw || B <= 0 || H <= 0 || W <= 0 || C <= 0 || Co <= 0 || ldw < 9 * C) return fail("conv3x3_wgrad: bad shape");
+    const bool small = C == 1 || C == 2 || C == 4;
+    if ((!small && C % 32) || (Co % 32 && Co > 4)) return fail("conv3x3_wgrad: unsupported channel counts", HP2D_UNSUPPORTED_FLAG);
+    if (!aligned16(x) || !aligned16(dy)) return fail("conv3x3_wgrad: alignment");
+    int* err = err_ptr();
+    if (!err) return fail("cannot resolve the error flag", HP2D_CUDA_ERROR);
+    cudaStream_t st = S(stream);
+    if (C == 4) return wgrad_n<64, 4>(x, B, H, W, C, dy, Co, gw, ldw, err, st);
+    if (C == 2) return wgrad_n<64, 2>(x, B, H, W, C, dy, Co, gw, ldw, err, st);
+    if (C == 1) return wgrad_n<64, 1>(x, B, H, W, C, dy, Co, gw, ldw, err, st);
+    if (C % 64 == 0) return wgrad_n<64, 0>(x, B, H, W, C, dy, Co, gw, ldw, err, st);
+    return wgrad_n<32, 0>(x, B, H, W, C, dy, Co, gw, ldw, err, st);
+}
+
 hp2d_status hp2d_nn_mse(const float* pred, int32_t ldp, const float* target, const float* w, int64_t P, int32_t nch,
                         float scale, float* loss, uint16_t* dpred, int32_t ldd, void* stream) {
     if (!pred || !target || !loss || !dpred || ldp < nch || ldd < nch) return fail("mse: bad shape");
-    k_mse<<<blocks(P), 256, 0, S(stream)>>>(pred, ldp, target, w, P, nch, scale, loss, dpred, ldd);
+    k_mse<<<kMseBlocks, 512, 0, S(stream)>>>(pred, ldp, target, w, P, nch, scale, loss, dpred, ldd);
     return launched("mse");
 }
 

@@ -42,11 +42,31 @@ template <int BN, int KB = kBK> constexpr size_t gemm_smem_bytes() {
     return size_t(kGemmStages) * (kBM * KB * 2 + BN * KB * 2) + 1024;   // + alignment slack
 }
 
-// Geometry of an implicit-GEMM 3x3 convolution (A is read straight from the NHWC input):
-// the 128 output pixels of a tile are 128 consecutive pixels of one image (W >= 128) or
-// 128/W whole rows (W < 128); k tile kt is tap kt / cblocks, channel block kt % cblocks.
+// Output tiles of a convolution: kTX x kTY = 128 pixels of one image.
+constexpr int kTX = 8, kTY = 16;
+static_assert(kTX * kTY == kBM, "a tile is one tcgen05 M");
+struct TileGeom {
+    int H, W, tiles_x, tiles_y, total;   // total: over the batch
+    __device__ __forceinline__ void at(int t, int& b, int& y0, int& x0) const {
+        const int per = tiles_x * tiles_y;
+        b = t / per;
+        const int r = t - b * per;
+        const int ty = r / tiles_x;
+        y0 = ty * kTY;
+        x0 = (r - ty * tiles_x) * kTX;
+    }
+    // the output row of pixel m of the tile at (b, y0, x0), -1 outside the image
+    __device__ __forceinline__ int row(int b, int y0, int x0, int m) const {
+        const int y = y0 + m / kTX, x = x0 + m % kTX;
+        return (y < H && x < W) ? (b * H + y) * W + x : -1;
+    }
+};
+// Geometry of an implicit-GEMM 3x3 convolution (A is read straight from the NHWC input, a box of
+// KB channels x the tile's pixels shifted by the tap): k tile kt is tap kt / cblocks, channel block
+// kt % cblocks.
 struct ConvGeom {
-    int H, W, cblocks;
+    TileGeom t;
+    int cblocks;
 };
 
 // ---- PTX wrappers ----------------------------------------------------------------------
@@ -224,13 +244,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     if (tid == 0 && nk > 0) {
         // producer: TMA tiles of A (rows m0..) and B (rows n0..), k tile kt0 + i
         int img = 0, y0 = 0, x0 = 0;
-        if (IM2COL) {
-            const int hw = g.H * g.W;
-            img = m0 / hw;
-            const int rem = m0 - img * hw;
-            y0 = rem / g.W;
-            x0 = rem - y0 * g.W;
-        }
+        if (IM2COL) g.t.at(int(blockIdx.x), img, y0, x0);
         for (int i = 0; i < nk; ++i) {
             const int s = i % kGemmStages;
             const uint32_t fb = smem_addr(&bar_full[s]);
@@ -275,13 +289,18 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const bool landed = nk > 0 ? bar_wait(smem_addr(&bar_done), 0u) : true;
     if (!landed) atomicExch(&s_fail, 1);
     tc_fence_after();
-    const int row = m0 + warp * 32 + lane;
+    int row = m0 + warp * 32 + lane;
+    if (IM2COL) {
+        int img, y0, x0;
+        g.t.at(int(blockIdx.x), img, y0, x0);
+        row = g.t.row(img, y0, x0, warp * 32 + lane);
+    }
     if (landed && nk > 0) {
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 32) {
             float v[32];
             tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0), v);
-            store_row32(v, row, n0 + c0, M, N, C, ldc, bias, epi);
+            if (row >= 0) store_row32(v, row, n0 + c0, M, N, C, ldc, bias, epi);
         }
     }
     tc_fence_before();
@@ -370,13 +389,7 @@ k_gemm_bf16_pt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 int m0, n0, kt0, nk;
                 tile(t, m0, n0, kt0, nk);
                 int img = 0, y0 = 0, x0 = 0;
-                if (IM2COL) {
-                    const int hw = g.H * g.W;
-                    img = m0 / hw;
-                    const int rem = m0 - img * hw;
-                    y0 = rem / g.W;
-                    x0 = rem - y0 * g.W;
-                }
+                if (IM2COL) g.t.at(m0 / kBM, img, y0, x0);
                 for (int i = 0; i < nk; ++i) {
                     const uint32_t it = issued;
                     const int s = int(it % kGemmStages);
@@ -456,12 +469,17 @@ k_gemm_bf16_pt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 break;
             }
             tc_fence_after();
-            const int row = m0 + q * 32 + lane;
+            int row = m0 + q * 32 + lane;
+            if (IM2COL) {
+                int img, y0, x0;
+                g.t.at(m0 / kBM, img, y0, x0);
+                row = g.t.row(img, y0, x0, q * 32 + lane);
+            }
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 float v[32];
                 tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(b * BN + c0), v);
-                store_row32(v, row, n0 + c0, M, N, C, ldc, bias, epi);
+                if (row >= 0) store_row32(v, row, n0 + c0, M, N, C, ldc, bias, epi);
             }
             tc_fence_before();
             mbar_arrive(smem_addr(&acc_empty[b]));

@@ -67,6 +67,33 @@ def conv3x3(x: torch.Tensor, w16: torch.Tensor, Co: int, out: torch.Tensor, epil
                              EPI[epilogue], _stream()))
 
 
+def conv_any_ok(ci: int, co: int, ldw: int) -> bool:
+    """Whether ``conv3x3_any`` takes these channel counts (weights of row pitch ``ldw``)."""
+    return (ci in (1, 2, 4) and co <= 128 and ldw >= 64) or ci % 32 == 0
+
+
+def conv3x3_any(x: torch.Tensor, w16: torch.Tensor, Co: int, out: torch.Tensor, epilogue: str,
+                bias: torch.Tensor | None = None):
+    """``conv3x3`` for any image size (``conv_any_ok`` channel counts)."""
+    Bn, H, W, Cc = x.shape
+    assert x.is_contiguous() and w16.stride(1) == 1 and out.stride(1) == 1
+    _ok(_L().hp2d_nn_conv3x3_any(_p(x), Bn, H, W, Cc, _p(w16), w16.stride(0), Co, _p(bias), _p(out), out.stride(0),
+                                 EPI[epilogue], _stream()))
+
+
+def wgrad_ok(ci: int, co: int) -> bool:
+    """Whether ``conv3x3_wgrad`` takes these channel counts."""
+    return (ci in (1, 2, 4) or ci % 32 == 0) and (co <= 4 or co % 32 == 0)
+
+
+def conv3x3_wgrad(x: torch.Tensor, dy: torch.Tensor, gW: torch.Tensor):
+    """gW[co, tap*C + c] += the weight gradient of a 3x3 convolution of x [B, H, W, C] whose output
+    gradient is dy [B, H, W, Co]."""
+    Bn, H, W, Cc = x.shape
+    assert x.is_contiguous() and dy.is_contiguous() and gW.stride(1) == 1
+    _ok(_L().hp2d_nn_conv3x3_wgrad(_p(x), Bn, H, W, Cc, _p(dy), dy.shape[-1], _p(gW), gW.stride(0), _stream()))
+
+
 def im2col3x3(x: torch.Tensor, Kp: int, transpose: bool = False, out: torch.Tensor | None = None):
     Bn, H, W, Cc = x.shape
     P = Bn * H * W
@@ -127,6 +154,13 @@ def relu_bwd(y, dy):
 def colsum(dz2d, out):
     P, Cc = dz2d.shape
     _ok(_L().hp2d_nn_colsum(_p(dz2d), P, Cc, dz2d.stride(0), _p(out), _stream()))
+
+
+def relu_colsum(y, dy2d, out):
+    """``relu_bwd`` of dy2d [P, C] by y (None: no ReLU) and ``colsum`` of the result, in one pass."""
+    P, Cc = dy2d.shape
+    assert dy2d.is_contiguous() and (y is None or y.is_contiguous())
+    _ok(_L().hp2d_nn_relu_colsum(_p(y), _p(dy2d), P, Cc, _p(out), _stream()))
 
 
 def mse(pred, target, weight, scale, loss, dpred):

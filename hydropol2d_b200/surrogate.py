@@ -9,10 +9,10 @@ member's peak-depth map, and members on which the networks disagree by more than
 threshold go back to the solver (``screening``).
 
 Layout: activations NHWC BF16; a 3x3 convolution is ``y[P, Co] = cols[P, Kp] . W[Co, Kp]^T``
-with K index (ky*3 + kx)*Ci + ci, computed as an implicit GEMM that reads tap-shifted boxes of
-the input through TMA (``nn.conv3x3``) where the shape allows, else as im2col + GEMM; backward
-gives ``dx`` as the convolution of dy with the flipped kernel (same two forms) and
-``dW = dy^T . cols`` (split-K GEMM over pixels).
+with K index (ky*3 + kx)*Ci + ci, computed straight from the NHWC input through TMA tiles
+(``nn.conv3x3_any``) for the channel counts it takes, else as im2col + GEMM; backward gives ``dx`` as
+the convolution of dy with the flipped kernel (same two forms) and ``dW = dy^T . cols`` from the
+activations themselves (``nn.conv3x3_wgrad``), else as a split-K GEMM over pixels.
 """
 from __future__ import annotations
 
@@ -91,8 +91,8 @@ class Conv3x3:
         head = self.name == "head"
         y = torch.empty(P, self.co, dtype=torch.float32 if head else torch.bfloat16, device=x.device)
         epi = "f32_bias" if head else ("bf16_bias_relu" if self.relu else "bf16_bias")
-        if nn.conv_ok(x.shape):
-            nn.conv3x3(x.contiguous(), self.W16, self.co, y, epi, bias=self.b)   # implicit GEMM
+        if nn.conv_any_ok(self.ci, self.co, self.kp):
+            nn.conv3x3_any(x.contiguous(), self.W16, self.co, y, epi, bias=self.b)
         else:
             nn.gemm(nn.im2col3x3(x, self.kp), self.W16, y, epi, bias=self.b)
         if keep:
@@ -105,21 +105,22 @@ class Conv3x3:
         B, H, W, _ = x.shape
         P = B * H * W
         dy2 = dy.reshape(P, self.co)
-        if self.relu:
-            nn.relu_bwd(self.y, dy2)
-        nn.colsum(dy2, self.gb)
-        dyT = nn.transpose(dy2)
-        colsT = nn.im2col3x3(x, self.kp, transpose=True)
-        tiles = -(-self.co // 128) * -(-self.kp // (256 if self.kp > 128 else self.kp))
-        split = max(1, min(P // 64, (2 * 148) // max(tiles, 1)))
-        nn.gemm(dyT, colsT, self.gW, "f32_atomic", split_k=split)
+        nn.relu_colsum(self.y if self.relu else None, dy2, self.gb)
+        if nn.wgrad_ok(self.ci, self.co):
+            nn.conv3x3_wgrad(x.contiguous(), dy2.view(B, H, W, self.co), self.gW)
+        else:
+            dyT = nn.transpose(dy2)
+            colsT = nn.im2col3x3(x, self.kp, transpose=True)
+            tiles = -(-self.co // 128) * -(-self.kp // (256 if self.kp > 128 else self.kp))
+            split = max(1, min(P // 64, (2 * 148) // max(tiles, 1)))
+            nn.gemm(dyT, colsT, self.gW, "f32_atomic", split_k=split)
         if not need_dx:
             return None
         wt = nn.flip3x3(self.W, self.co, self.ci, self.kp, self.kp2)
         dx = torch.empty(P, self.ci, dtype=torch.bfloat16, device=x.device)
         dyv = dy2.view(B, H, W, self.co)
-        if nn.conv_ok(dyv.shape):
-            nn.conv3x3(dyv, wt, self.ci, dx, "bf16_bias", bias=self.zero_ci)
+        if nn.conv_any_ok(self.co, self.ci, self.kp2):
+            nn.conv3x3_any(dyv, wt, self.ci, dx, "bf16_bias", bias=self.zero_ci)
         else:
             nn.gemm(nn.im2col3x3(dyv, self.kp2), wt, dx, "bf16_bias", bias=self.zero_ci)
         return dx.view(B, H, W, self.ci)

@@ -45,6 +45,17 @@ hp2d_status hp2d_nn_gemm(int32_t M, int32_t N, int32_t K, const void* A, int32_t
 hp2d_status hp2d_nn_conv3x3(const uint16_t* x, int32_t B, int32_t H, int32_t W, int32_t C, const uint16_t* w,
                             int32_t ldw, int32_t Co, const float* bias, void* y, int32_t ldy, int32_t epilogue,
                             void* stream);
+/* hp2d_nn_conv3x3 for any H and W and for C = 1, 2 or 4 (w then has rows of at least 64 columns, zero
+ * beyond 9C, and Co <= 128) or a multiple of 32; HP2D_UNSUPPORTED_FLAG for other channel counts.  The
+ * same results bit for bit as im2col followed by the GEMM. */
+hp2d_status hp2d_nn_conv3x3_any(const uint16_t* x, int32_t B, int32_t H, int32_t W, int32_t C, const uint16_t* w,
+                                int32_t ldw, int32_t Co, const float* bias, void* y, int32_t ldy, int32_t epilogue,
+                                void* stream);
+/* Weight gradient of that convolution: gw[co, (ky*3+kx)*C + c] += sum over pixels of dy[p, co] times the
+ * tap's x, fp32 (pitch ldw), dy [B,H,W,Co] NHWC BF16; C = 1, 2, 4 or a multiple of 32, Co <= 4 or a
+ * multiple of 32 (HP2D_UNSUPPORTED_FLAG otherwise). */
+hp2d_status hp2d_nn_conv3x3_wgrad(const uint16_t* x, int32_t B, int32_t H, int32_t W, int32_t C, const uint16_t* dy,
+                                  int32_t Co, float* gw, int32_t ldw, void* stream);
 /* sticky error of the kernels (1 = a wait ran out); reading clears it; synchronises */
 hp2d_status hp2d_nn_check(void);
 const char* hp2d_nn_error(void);
@@ -74,6 +85,8 @@ hp2d_status hp2d_nn_copy_channels(const uint16_t* in, int32_t cin, int32_t c0, i
 hp2d_status hp2d_nn_relu_bwd(const uint16_t* y, uint16_t* dy, int64_t n, void* stream);
 /* out[c] += sum_p dz[p, c]  (dz [P, C] pitch ld) */
 hp2d_status hp2d_nn_colsum(const uint16_t* dz, int64_t P, int32_t C, int32_t ld, float* out, void* stream);
+/* hp2d_nn_relu_bwd (y null: none) and hp2d_nn_colsum of the result in one pass over dy [P, C] */
+hp2d_status hp2d_nn_relu_colsum(const uint16_t* y, uint16_t* dy, int64_t P, int32_t C, float* out, void* stream);
 /* masked squared error over channels 0..nch-1 of pred [P, ldp] (fp32) against target
  * [P, nch] with weights w [P, nch] (fp32): loss += sum w (pred - t)^2 * scale and
  * dpred [P, ldd] (bf16, other channels zero) = 2 w (pred - t) * scale */
