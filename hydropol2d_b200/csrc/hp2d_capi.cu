@@ -10,8 +10,7 @@
 //   gs2[2]    n x {I, T}                             Green-Ampt record, double-buffered
 //   arrival   n x R
 //   per outlet: coefficient, Hf(:,:,3) and sink rate
-// plus, for the unfused entry points only, structure-of-arrays copies (dz_x, dz_y, n^2,
-// soil class, outlet bitmask) and scratch (h, q, dmax, I, T, Hf, unlimited q, scale).
+// plus, for the unfused entry points only, the face depths of the last routing step.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -306,13 +305,10 @@ template <typename R> struct Impl : Base {
     Dev<int32_t> outlet_cells;
     Dev<R> outlet_coef, hf3, qo;
     int n_out = 0;
-    // unfused path: structure-of-arrays copies and scratch
-    Dev<R> dzx, dzy, n2;
-    Dev<uint8_t> soil;
+    // unfused path: outlet cells as bits, face depths of the last routing step
     Dev<uint32_t> outlet_bits;
     int bit_words = 0;
-    Dev<R> h, qx, qy, dmax, I, T;
-    Dev<R> hfx, hfy, qxu, qyu, scale;
+    Dev<R> hfx, hfy;
     // forcing, clock
     Dev<double> rain_t, rain_r;
     // inflow hydrographs
@@ -404,11 +400,12 @@ template <typename R> struct Impl : Base {
         // and maps 291 / 259, wet 189 / 160.
         const size_t most = sizeof(R) == 8 ? 4000000 : (inf_mode() || rain.n_maps) ? 4300000 : 2500000;
         if (n > most) return 0;
-        // one row per thread while the grid gives the GPU little more than one wave of tiles (256^2 wet
-        // FP32 6.5 / 7.4 us with one / two rows, 400^2 9.7 / 9.5; FP64 Green-Ampt 600^2 43 / 46,
-        // 1000^2 103 / 103)
-        return n > (sizeof(R) == 8 ? 1000000u : 200000u) ? 2 : 1;
+        return default_tile_rpt();
     }
+    // one row per thread while the grid gives the GPU little more than one wave of tiles (256^2 wet
+    // FP32 6.5 / 7.4 us with one / two rows, 400^2 9.7 / 9.5; FP64 Green-Ampt 600^2 43 / 46,
+    // 1000^2 103 / 103)
+    int default_tile_rpt() const { return n > (sizeof(R) == 8 ? 1000000u : 200000u) ? 2 : 1; }
     bool tile_on() const { return tile_rpt() != 0; }
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
@@ -463,8 +460,21 @@ template <typename R> struct Impl : Base {
     void h2d(void* dev, const void* host, size_t bytes) {
         stage.copy(dev, const_cast<void*>(host), bytes, true, st(), ctx->device);
     }
-    void push_sc() { HP_CK(cudaMemcpyAsync(sc.p, &hs, sizeof(hs), cudaMemcpyHostToDevice, st())); HP_CK(cudaStreamSynchronize(st())); }
-    void pull_sc() { HP_CK(cudaMemcpyAsync(&hs, sc.p, sizeof(hs), cudaMemcpyDeviceToHost, st())); HP_CK(cudaStreamSynchronize(st())); }
+    // The scalars between host and device.  pull_sc reads them back unless the mirror hs is known to
+    // hold them: every launch or copy that changes them on the device calls sc_changed first.
+    bool hs_current = false;
+    void sc_changed() { hs_current = false; }
+    void push_sc() {
+        HP_CK(cudaMemcpyAsync(sc.p, &hs, sizeof(hs), cudaMemcpyHostToDevice, st()));
+        HP_CK(cudaStreamSynchronize(st()));
+        hs_current = true;
+    }
+    void pull_sc() {
+        if (hs_current) return;
+        HP_CK(cudaMemcpyAsync(&hs, sc.p, sizeof(hs), cudaMemcpyDeviceToHost, st()));
+        HP_CK(cudaStreamSynchronize(st()));
+        hs_current = true;
+    }
 
     // the library's own host vectors: one copy (the driver stages pageable memory itself; the
     // context's staging chunks are for the caller's large arrays, whose page-locked allocation
@@ -487,13 +497,6 @@ template <typename R> struct Impl : Base {
         k_fill<T><<<blocks_for(count), kThreads, 0, st()>>>(count, p, v);
         HP_CK(cudaGetLastError());
         HP_CK(cudaStreamSynchronize(st()));
-    }
-    GridView<R> view() const {
-        GridView<R> gv;
-        gv.ny = ny; gv.nx = nx; gv.res = res;
-        gv.tol_mm = ctx->p.depth_tolerance;
-        gv.thr_mm = ctx->p.arrival_threshold;
-        return gv;
     }
     int blocks_for(size_t count) const {
         size_t b = (count + kThreads - 1) / kThreads;
@@ -564,8 +567,7 @@ template <typename R> struct Impl : Base {
             int i = cells[o] / nx, j = cells[o] % nx;
             bits[size_t(i) * bit_words + (j >> 5)] |= 1u << (j & 31);
         }
-        // the records (and the unfused entry points' structure-of-arrays copies) are built
-        // on the device from the caller's FP64 arrays
+        // the records are built on the device from the caller's FP64 arrays
         {
             Dev<double> dr_;
             Dev<uint32_t> dm_;
@@ -584,10 +586,7 @@ template <typename R> struct Impl : Base {
             } else {
                 upload(dm_.p, host_meta);
             }
-            // the unfused entry points' copies are extracted from the records on first use
-            dzx.free(); dzy.free(); n2.free();
-            k_build_static<R><<<blocks_for(n), kThreads, 0, st()>>>(ny, nx, z_keep.p, dr_.p, dm_.p, stat.p, nullptr,
-                                                                     nullptr, nullptr);
+            k_build_static<R><<<blocks_for(n), kThreads, 0, st()>>>(ny, nx, z_keep.p, dr_.p, dm_.p, stat.p);
             HP_CK(cudaGetLastError());
             HP_CK(cudaStreamSynchronize(st()));
         }
@@ -635,8 +634,6 @@ template <typename R> struct Impl : Base {
             for (size_t k = a; k < b; ++k) host_meta[k] = (host_meta[k] & ~255u) | cls[k];
         });
         write_meta();
-        soil.alloc(n);
-        upload(soil.p, host_soil);
         // soil records: keep I if present, recovery timer restarts at Tr
         std::vector<V2> g(n);
         if (gs2[0].p) g = fetch(gs2[hs.cur].p, n);
@@ -694,8 +691,6 @@ template <typename R> struct Impl : Base {
             for (size_t k = a; k < b; ++k) host_meta[k] = (host_meta[k] & ~255u) | cls[k];
         });
         write_meta();
-        soil.alloc(n);
-        upload(soil.p, host_soil);
         std::vector<V2> g(n);
         if (gs2[0].p) g = fetch(gs2[hs.cur].p, n);
         else for (size_t k = 0; k < n; ++k) g[k] = V2{R(0), R(0)};
@@ -1184,143 +1179,118 @@ template <typename R> struct Impl : Base {
         return HP2D_OK;
     }
 
-    void fold_accumulators() {
-        pull_sc();
-        double area = res * res;
-        hs.rain_vol += hs.acc_rain * area;
-        hs.inf_vol += hs.acc_inf * area;
-        hs.out_vol += hs.acc_out * area;
-        hs.acc_rain = hs.acc_inf = hs.acc_out = 0;
-        hs.acc_vmax = hs.acc_cmax = 0;
-        hs.acc_neg = 0;
-        push_sc();
-    }
-
     // ---------------- unfused entry points ----------------
-    // each call unpacks the records of the current buffer into the SoA scratch, runs
-    // the stage kernels and packs the result back
-    void ensure_scratch() {
-        if (!h.p) {
-            h.alloc(n); qx.alloc(n); qy.alloc(n); dmax.alloc(n); I.alloc(n); T.alloc(n);
-            hfx.alloc(n); hfy.alloc(n); qxu.alloc(n); qyu.alloc(n); scale.alloc(n);
+    // (hp2d_unfused.cuh): one pass over the records each; the scalars are read back once, at the end
+    void ensure_face_depths() {
+        if (!hfx.p) {
+            hfx.alloc(n); hfy.alloc(n);
             fill(hfx.p, n, R(0));
             fill(hfy.p, n, R(0));
         }
     }
-    void unpack() {
-        ensure_scratch();
-        const int cur = hs.cur;
-        k_unpack<R><<<blocks_for(n), kThreads, 0, st()>>>(n, st4[cur].p, gs2[cur].p, h.p, qx.p, qy.p, dmax.p, I.p, T.p);
+    StepConsts<R> consts(double dt_s) const {
+        StepConsts<R> K;
+        K.make(dt_s, res, ctx->p.depth_tolerance, ctx->p.arrival_threshold);
+        return K;
+    }
+    // the call's sums into the volumes, the buffers' roles exchanged; soil records that the call did
+    // not write stay with the state
+    void unfused_end(const FusedArgs<R>& a, int call, bool soil_written) {
+        sc_changed();
+        k_unfused_end<R><<<1, 32, 0, st()>>>(a, call, hs.max_dt);
+        HP_CK(cudaGetLastError());
+        if (call != CALL_TIME_STEP) {
+            if (gs2[0].p && !soil_written) {
+                std::swap(gs2[0].p, gs2[1].p);
+                invalidate_graph();
+            }
+            dirty = true;
+        }
+        pull_sc();
+    }
+    template <int INF> void launch_hydrology(const FusedArgs<R>& a, const StepConsts<R>& K, int pass) {
+        const dim3 g = rows_grid(ny, nx);
+        if (rain.n_maps > 0) k_hydrology<R, INF, true><<<g, 128, 0, st()>>>(a, hs.cur, hs.rain_a, hs.rain_b, K, pass);
+        else k_hydrology<R, INF, false><<<g, 128, 0, st()>>>(a, hs.cur, hs.rain_a, hs.rain_b, K, pass);
         HP_CK(cudaGetLastError());
     }
-    void pack() {
-        const int cur = hs.cur;
-        k_pack<R><<<blocks_for(n), kThreads, 0, st()>>>(n, st4[cur].p, gs2[cur].p, h.p, qx.p, qy.p, dmax.p, I.p, T.p);
-        HP_CK(cudaGetLastError());
-    }
-
     hp2d_status hydrology_step(double time_step) {
         pull_sc();
-        hs.acc_neg = 0;
-        push_sc();
-        unpack();
-        double dts = time_step * 60.0;
+        ensure_face_depths();
+        sc_changed();
+        const FusedArgs<R> a = fused_args();
+        const StepConsts<R> K = consts(time_step * 60.0);
         if (inflow.n_gauges) {   // gauge depths of the current rain interval
             k_inflow_depth<R><<<1, kThreads, 0, st()>>>(inflow, sc.p);
             HP_CK(cudaGetLastError());
         }
-        k_hydro_rain_ga<R><<<blocks_for(n), kThreads, 0, st()>>>(view(), hs.rain_a, hs.rain_b, dts, rain, h.p, I.p, T.p, soil.p,
-                                                               classes.p, classes_vg.p, vgg, inf_mode(), inflow,
-                                                               stat.p, sc.p);
-        HP_CK(cudaGetLastError());
-        k_hydro_clamp<R><<<blocks_for(n), kThreads, 0, st()>>>(n, h.p, sc.p);
-        HP_CK(cudaGetLastError());
-        pack();
-        std::vector<R> gd;
-        if (inflow.n_gauges) gd = fetch(inf_depth.p, size_t(inflow.n_gauges));
-        pull_sc();
-        if (hs.acc_neg) hs.neg_warn += 1;
-        for (size_t g = 0; g < gd.size(); ++g) hs.inflow_vol += double(gd[g]) * host_gcells[g] * res * res;
-        push_sc();
-        fold_accumulators();
-        dirty = true;
+        const int inf = inf_mode();
+        for (int pass = 0; pass < 2; ++pass) {
+            if (inf == 1) launch_hydrology<1>(a, K, pass);
+            else if (inf == 2) launch_hydrology<2>(a, K, pass);
+            else launch_hydrology<0>(a, K, pass);
+        }
+        unfused_end(a, CALL_HYDROLOGY, inf != 0);
         return HP2D_OK;
     }
 
     hp2d_status li_step(double time_step) {
         pull_sc();
-        unpack();
-        double dts = time_step * 60.0;
-        auto gv = view();
-        int nb = blocks_for(n);
-        if (!dzx.p) {   // structure-of-arrays copies of the static record, made once
-            dzx.alloc(n); dzy.alloc(n); n2.alloc(n);
-            k_static_soa<R><<<nb, kThreads, 0, st()>>>(n, stat.p, dzx.p, dzy.p, n2.p);
-            HP_CK(cudaGetLastError());
-        }
-        k_faces<R><<<nb, kThreads, 0, st()>>>(gv, dts, h.p, dzx.p, dzy.p, n2.p, qx.p, qy.p, hfx.p, hfy.p, qxu.p,
-                                            qyu.p, ctx->p.flag_critical, ctx->p.flag_numerical_scheme);
-        HP_CK(cudaGetLastError());
-        k_scale<R><<<nb, kThreads, 0, st()>>>(gv, dts, h.p, qxu.p, qyu.p, scale.p);
-        HP_CK(cudaGetLastError());
-        k_limit<R><<<nb, kThreads, 0, st()>>>(gv, qxu.p, qyu.p, scale.p, qx.p, qy.p);
-        HP_CK(cudaGetLastError());
+        ensure_face_depths();
+        sc_changed();
+        const double dts = time_step * 60.0;
+        FusedArgs<R> a = fused_args();
+        a.own_r0 = 0;
+        a.own_r1 = ny;
+        tile_shape(a, default_tile_rpt());
+        LiArgs<R> li{consts(dts), hfx.p, hfy.p};
         if (strct.n) {
-            k_struct_unfused<R><<<1, 32, 0, st()>>>(strct, h.p, time_step, res * res, sc.p);
+            k_struct_unfused<R><<<1, 32, 0, st()>>>(strct, st4[hs.cur].p, time_step, res * res, sc.p);
             HP_CK(cudaGetLastError());
         }
-        k_continuity<R><<<nb, kThreads, 0, st()>>>(gv, dts, h.p, qx.p, qy.p);
+        launch_tile_li<R>(a, li, strct.n > 0, ctx->p.flag_numerical_scheme != 1, hs.cur, st());
         HP_CK(cudaGetLastError());
-        if (n_out) {
-            k_outlet<R><<<(n_out + kThreads - 1) / kThreads, kThreads, 0, st()>>>(
-                gv, dts, h.p, outlet_cells.p, outlet_coef.p, n_out, ctx->p.outlet_type, hf3.p, qo.p, sc.p);
-            HP_CK(cudaGetLastError());
-        }
-        pack();
         last_dt_s = dts;
-        fold_accumulators();
-        dirty = true;
+        unfused_end(a, CALL_ROUTING, false);
         return HP2D_OK;
     }
 
     hp2d_status cfl_dt(double* ts_out, double* vmax_out) {
         if (!(last_dt_s > 0)) { ctx->err = "hp2d_cfl_dt needs a preceding hp2d_li_step"; return HP2D_NOT_READY; }
         pull_sc();
-        hs.acc_vmax = hs.acc_cmax = 0;
-        push_sc();
-        unpack();
-        k_cfl<R><<<blocks_for(n), kThreads, 0, st()>>>(view(), last_dt_s, qx.p, qy.p, hfx.p, hfy.p, outlet_bits.p,
-                                                     bit_words, outlet_cells.p, hf3.p, n_out,
-                                                     ctx->p.flag_adaptive_timestepping, sc.p);
+        sc_changed();
+        const FusedArgs<R> a = fused_args();
+        k_cfl<R><<<rows_grid(ny, nx), 128, 0, st()>>>(a, hs.cur, consts(last_dt_s), hfx.p, hfy.p, outlet_bits.p, bit_words);
         HP_CK(cudaGetLastError());
-        pull_sc();
-        const bool is_d = sizeof(R) == 8;
-        double vm = from_ord(hs.acc_vmax, is_d), cm = from_ord(hs.acc_cmax, is_d);
-        const hp2d_params& p = ctx->p;
-        double tcr = finalize_dt(vm, cm, res, p.alfa_min, p.alfa_max, p.min_time_step, hs.max_dt,
-                                 p.time_step_increments, p.flag_timestep);
-        hs.acc_vmax = hs.acc_cmax = 0;
-        hs.vmax_last = vm;
-        if (tcr == p.min_time_step) hs.unstable += 1;
-        push_sc();
-        *ts_out = tcr / 60.0;
-        if (vmax_out) *vmax_out = vm;
+        unfused_end(a, CALL_TIME_STEP, false);
+        *ts_out = hs.refreshed_s / 60.0;
+        if (vmax_out) *vmax_out = hs.vmax_last;
         return HP2D_OK;
     }
 
     hp2d_status track_maxima(double t_end) {
         pull_sc();
-        unpack();
-        R thr = R(ctx->p.arrival_threshold / 1000.0);
-        k_track<R><<<blocks_for(n), kThreads, 0, st()>>>(n, h.p, dmax.p, arrival.p, thr, R(t_end * 60.0));
+        ensure_face_depths();
+        const R thr = R(ctx->p.arrival_threshold / 1000.0);
+        k_track<R><<<blocks_for(n), kThreads, 0, st()>>>(n, st4[hs.cur].p, arrival.p, thr, R(t_end * 60.0));
         HP_CK(cudaGetLastError());
-        pack();
         HP_CK(cudaStreamSynchronize(st()));
         dirty = true;   // the records were rewritten from outside a fused step
         return HP2D_OK;
     }
 
     // ---------------- fused path ----------------
+    // the launch of the tile kernels with `rpt` rows per thread
+    void tile_shape(FusedArgs<R>& a, int rpt) {
+        if (!n_sms) HP_CK(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, ctx->device));
+        using T1 = TileShape<R, 1>;
+        using T2 = TileShape<R, 2>;
+        const int rows = rpt == 2 ? T2::OR : T1::OR;
+        a.tile_rpt = rpt;
+        a.tile_nx = (nx + T1::OC - 1) / T1::OC;
+        a.tile_grid = unsigned(n_sms * (rpt == 2 ? T2::MINB : T1::MINB));
+        a.n_ctas = unsigned(a.tile_nx * ((ny + rows - 1) / rows));
+    }
     FusedArgs<R> fused_args(int cpl = 0) {
         if (cpl <= 0) cpl = cells_per_lane;
         FusedArgs<R> a{};
@@ -1365,14 +1335,7 @@ template <typename R> struct Impl : Base {
         a.dryflag = dry_usable(rpw) && tb_chosen <= 1 && !slab() ? dryf.p : nullptr;
         a.tile_nx = 0;
         if (tile_on()) {
-            if (!n_sms) HP_CK(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, ctx->device));
-            using T1 = TileShape<R, 1>;
-            using T2 = TileShape<R, 2>;
-            a.tile_rpt = tile_rpt();
-            const int rows = a.tile_rpt == 2 ? T2::OR : T1::OR;
-            a.tile_nx = (nx + T1::OC - 1) / T1::OC;
-            a.tile_grid = unsigned(n_sms * (a.tile_rpt == 2 ? T2::MINB : T1::MINB));
-            a.n_ctas = unsigned(a.tile_nx * ((ny + rows - 1) / rows));
+            tile_shape(a, tile_rpt());
             a.dryflag = dry_enabled && tb_chosen <= 1 && !slab() ? dryf.p : nullptr;
         }
         a.vmax = hz_on ? vmaxm.p : nullptr;
@@ -1460,6 +1423,7 @@ template <typename R> struct Impl : Base {
     // `count` steps in a row, the last one ended for the host.  Gauges, stages and control structures
     // need the step's end before the next step's launch (its depths, stages and transfers).
     void launch_row(const FusedArgs<R>& a, int64_t count) {
+        sc_changed();
         const bool each = a.inflow.n_gauges > 0 || a.inflow.n_stage > 0 || a.strct.n > 0;
         for (int64_t s = 0; s < count; ++s) {
             launch_fused(a, each ? 0 : int(s & 3));
@@ -1549,6 +1513,7 @@ template <typename R> struct Impl : Base {
         hs.acc_bad = 0;
         hs.bad_domain = 0;
         push_sc();
+        sc_changed();
         k_skip_flag<R><<<blocks_for(n), kThreads, 0, st()>>>(st4[hs.cur].p, stat.p, ny, nx, rain, ga() ? 1 : 0, res,
                                                            ctx->p.depth_tolerance, ctx->p.arrival_threshold, sc.p,
                                                            own_r0, own_r1 < 0 ? ny : own_r1);
@@ -1588,6 +1553,7 @@ template <typename R> struct Impl : Base {
 
     void launch_steps(int64_t count) {
         FusedArgs<R> a = fused_args();
+        sc_changed();
         int64_t remaining = count;
         if (remaining >= kGraphChunk) {
             ensure_graph(a);
@@ -1759,6 +1725,7 @@ template <typename R> struct Impl : Base {
         }
     }
     void tb_launch(const FusedArgs<R>& a, int k) {
+        sc_changed();
         if (k == 2) tb_launch_k<2>(a);
         else if (k == 3) tb_launch_k<3>(a);
         else tb_launch_k<4>(a);
@@ -1844,6 +1811,7 @@ template <typename R> struct Impl : Base {
             const R lo = R(t * 60.0 + dts);
             for (int q = 1; q < std::max(tb_chosen, 1); ++q) t = dts / 60.0 + t;
             const R hi = R(t * 60.0 + dts);
+            sc_changed();
             k_retry_scan<R><<<blocks_for(n), kThreads, 0, st()>>>(a, inf_mode(), lo, hi);
             HP_CK(cudaGetLastError());
         }
@@ -1975,6 +1943,7 @@ template <typename R> struct Impl : Base {
         }
         copy_dev(arrival.p, s.arr.p, n);
         if (n_out) { copy_dev(hf3.p, s.hf3s.p, n_out); copy_dev(qo.p, s.qos.p, n_out); }
+        sc_changed();
         copy_dev(sc.p, s.scs.p, 1);   // after a flush: nothing pending
         reset_dry();
         HP_CK(cudaStreamSynchronize(st()));
@@ -2438,6 +2407,7 @@ struct hp2d_ensemble {
         HP_CK(cudaMemcpyAsync(&q, queue.p, sizeof(q), cudaMemcpyDeviceToHost, stream));
         HP_CK(cudaStreamSynchronize(stream));
         for (int m = 0; m < nm; ++m) {
+            impl(m).sc_changed();
             impl(m).pull_sc();
             impl(m).flush_records();
         }
@@ -2508,6 +2478,7 @@ struct hp2d_ensemble {
             HP_CK(cudaEventElapsedTime(&ms, e0, e1));
             if (ms < best_ms) { best_ms = ms; best = c; best_cpl = cpl; }
             for (int m = 0; m < nm; ++m) {
+                impl(m).sc_changed();
                 impl(m).pull_sc();
                 stalled = stalled || (impl(m).hs.status & kStatusTimeout) != 0;
                 impl(m).put_back(*snaps[m]);

@@ -199,6 +199,7 @@ struct StepScalars {
     // from its accumulators (StepAcc), and the uniform rain depth that step applied [m]
     int pending, pad3;
     double rain_cell;
+    double refreshed_s;   // unfused time-step call: its result [s]
 };
 // The sums and maxima of one step's CTAs.  Four of them rotate: launch n reads the pending step's
 // from slot n % 4, adds its own to slot (n + 1) % 4 and clears slot (n + 2) % 4.

@@ -1413,13 +1413,12 @@ static __global__ void k_idw_maps(int ny, int nx, double res, double x_ul, doubl
 }
 
 // ---------------- host boundary on the device: records built from the caller's arrays ----
-// static record {dz_x, dz_y, n^2, meta} and the unfused path's copies, from the elevation and
-// roughness in FP64 (dz formed in FP64 and rounded once; the closed domain edges +inf).  A cell
+// static record {dz_x, dz_y, n^2, meta} from the elevation and roughness in FP64 (dz formed in FP64 and rounded once; the closed domain edges +inf).  A cell
 // of NaN elevation (idx_nan) gets n^2 = NaN: its own faces are closed by their NaN dz before
 // n^2 is read, so the NaN only marks the cell as outside the domain (k_skip_flag reads it).
 template <typename R>
 __global__ void k_build_static(int ny, int nx, const double* z, const double* rough, const uint32_t* meta,
-                               typename Vec<R>::V4* stat, R* dzx, R* dzy, R* n2) {
+                               typename Vec<R>::V4* stat) {
     const size_t n = size_t(ny) * nx;
     const double edge = __longlong_as_double(0x7ff0000000000000ll);   // +inf
     for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x) {
@@ -1428,21 +1427,6 @@ __global__ void k_build_static(int ny, int nx, const double* z, const double* ro
         const R b = R((i >= 1) ? z[k - nx] - z[k] : edge);
         const R c = isnan(z[k]) ? R(__longlong_as_double(0x7ff8000000000000ll)) : R(rough[k] * rough[k]);
         stat[k] = typename Vec<R>::V4{a, b, c, make_meta<R>(meta[k])};
-        if (dzx) {
-            dzx[k] = a;
-            dzy[k] = b;
-            n2[k] = c;
-        }
-    }
-}
-// the unfused entry points' structure-of-arrays copies of the static record
-template <typename R>
-__global__ void k_static_soa(size_t n, const typename Vec<R>::V4* stat, R* dzx, R* dzy, R* n2) {
-    for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < n; k += size_t(gridDim.x) * blockDim.x) {
-        const auto v = stat[k];
-        dzx[k] = v.x;
-        dzy[k] = v.y;
-        n2[k] = v.z;
     }
 }
 // state record {h, q_x, q_y, dmax = -inf} from depths.d_t [mm] and outflow_bates pages 1-2
@@ -1744,42 +1728,6 @@ __global__ void k_skip_flag(const typename Vec<R>::V4* st, const typename Vec<R>
     for (int o = 16; o > 0; o >>= 1) fin += __shfl_xor_sync(0xffffffffu, fin, o);
     if ((threadIdx.x & 31) == 0 && fin) atomicAdd(&sc->n_finite, fin);
     if (__syncthreads_or(neg) && threadIdx.x == 0) atomicOr(&sc->skip_clamp, 1);
-}
-
-// SoA <-> record conversion for the unfused entry points
-template <typename R>
-__global__ void k_unpack(size_t n, const typename Vec<R>::V4* st, const typename Vec<R>::V2* gs, R* h, R* qx, R* qy,
-                         R* dmax, R* I, R* T) {
-    for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < n; c += size_t(gridDim.x) * blockDim.x) {
-        const auto v = st[c];
-        h[c] = v.x;
-        qx[c] = v.y;
-        qy[c] = v.z;
-        dmax[c] = v.w;
-        if (gs) {
-            const auto g = gs[c];
-            I[c] = g.x;
-            T[c] = g.y;
-        }
-    }
-}
-template <typename R>
-__global__ void k_pack(size_t n, typename Vec<R>::V4* st, typename Vec<R>::V2* gs, const R* h, const R* qx,
-                       const R* qy, const R* dmax, const R* I, const R* T) {
-    for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < n; c += size_t(gridDim.x) * blockDim.x) {
-        typename Vec<R>::V4 v;
-        v.x = h[c];
-        v.y = qx[c];
-        v.z = qy[c];
-        v.w = dmax[c];
-        st[c] = v;
-        if (gs) {
-            typename Vec<R>::V2 g;
-            g.x = I[c];
-            g.y = T[c];
-            gs[c] = g;
-        }
-    }
 }
 
 }  // namespace hp2d

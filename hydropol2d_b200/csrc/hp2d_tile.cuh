@@ -57,8 +57,16 @@ template <int ID, int NTH> __device__ __forceinline__ void bar_arrive() {
     asm volatile("barrier.arrive %0, %1;" ::"n"(ID), "n"(NTH) : "memory");
 }
 
-template <typename R, int RPT, int INF, bool MAP, bool INFL, int SCH>
-__global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB) k_tile_step(const __grid_constant__ FusedArgs<R> a, int phase) {
+// The routing step alone (Local_Inertial_Model_D4 as a call of its own, hp2d_li_step), LI: no rain,
+// clock, maxima or CFL terms, the face depths kept; buffer `phase` to the other one, with the
+// constants kc of the caller's time step.
+template <typename R> struct LiArgs {
+    StepConsts<R> kc;
+    R* hfx; R* hfy;
+};
+
+template <typename R, int RPT, int INF, bool MAP, bool INFL, int SCH, bool LI>
+__device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, const LiArgs<R>& li) {
     using V4 = typename Vec<R>::V4;
     using V2 = typename Vec<R>::V2;
     using Sh = TileShape<R, RPT>;
@@ -115,26 +123,30 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
     // fetched while warp 0 ends the step before
     place(blockIdx.x);
     fetch(next_S, a.stat, out_S);
-    step_begin<R, NT, true, true>(a, sh, phase, [&](int c) {
-        fetch(next_X, c ? a.st1 : a.st0, out_X);
-        if (a.dryflag && warp == 1) {
-            const unsigned f = flags(blockIdx.x, c);
-            if (lane == 0) s_flags[0] = f;
+    bool publish = !LI && blockIdx.x == 0 && warp == 0, next_made = LI;
+    if constexpr (LI) {
+        fetch(next_X, phase ? a.st1 : a.st0, out_X);
+    } else {
+        step_begin<R, NT, true, true>(a, sh, phase, [&](int c) {
+            fetch(next_X, c ? a.st1 : a.st0, out_X);
+            if (a.dryflag && warp == 1) {
+                const unsigned f = flags(blockIdx.x, c);
+                if (lane == 0) s_flags[0] = f;
+            }
+        });
+        if (sh.now.done) {
+            copy_wait_all();
+            if (publish) {
+                step_next(a, sh, lane);
+                step_publish<R, NT, INFL>(a, sh, phase);
+            }
+            return;
         }
-    });
-    bool publish = blockIdx.x == 0 && warp == 0, next_made = false;
-    if (sh.now.done) {
-        copy_wait_all();
-        if (publish) {
-            step_next(a, sh, lane);
-            step_publish<R, NT, INFL>(a, sh, phase);
-        }
-        return;
     }
 
-    const StepConsts<R>& K = sh.K;
-    const int cur = sh.now.cur;
-    const R clamp0 = sh.now.skip ? R(0) : R(1e-9);   // depths below are zero (Hydrological_Model.m:45-52)
+    const StepConsts<R>& K = LI ? li.kc : sh.K;
+    const int cur = LI ? phase : sh.now.cur;
+    const R clamp0 = LI ? R(0) : sh.now.skip ? R(0) : R(1e-9);   // depths below are zero (Hydrological_Model.m:45-52)
     const V4* __restrict__ sin = cur ? a.st1 : a.st0;
     V4* __restrict__ sout = cur ? a.st0 : a.st1;
     const V2* __restrict__ gin = cur ? a.gs1 : a.gs0;
@@ -158,11 +170,11 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
     const bool own_lane = lane >= 2 && lane < 30 && j < nx;
     const R first_col = j == 0 ? R(0.5) : R(1);   // refreshing_timestep.m's vel_left on the first column
     const int tile_cells = (r_end - r0) * (min(tx * OC + OC, nx) - tx * OC);
-    const unsigned fbits = a.dryflag ? s_flags[it & 1u] : 0u;
-    unsigned char* const fl_out = a.dryflag ? a.dryflag + size_t(cur ^ 1) * n_tiles + tile : nullptr;
+    const unsigned fbits = !LI && a.dryflag ? s_flags[it & 1u] : 0u;
+    unsigned char* const fl_out = !LI && a.dryflag ? a.dryflag + size_t(cur ^ 1) * n_tiles + tile : nullptr;
     const bool fo = (fbits & 1u) != 0u, fi = (fbits & 2u) != 0u;
     bool tile_skip = false;
-    if constexpr (INF == 0 && !MAP)
+    if constexpr (INF == 0 && !MAP && !LI)
         tile_skip = (fbits & 4u) && sh.now.rec < 0 && sh.p.rs.depth == R(0) && K.thr > R(0);
     const unsigned next = tile + gridDim.x;
     const bool more = next < n_tiles;
@@ -170,7 +182,7 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
         place(next);
         fetch(next_S, a.stat, out_S);
         fetch(next_X, sin, out_X);
-        if (a.dryflag && warp == 1) {
+        if (!LI && a.dryflag && warp == 1) {
             const unsigned f = flags(next, cur);
             if (lane == 0) s_flags[(it + 1u) & 1u] = f;
         }
@@ -189,6 +201,11 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
                 const size_t c = size_t(r) * nx + j;
                 const unsigned meta = meta_bits(S[i].w);
                 R hh = X[i].x;
+                if constexpr (LI) {   // the depth as it is; the fluxes see its positive part
+                    hT[i] = fmax(hh, R(0));
+                    wet = wet || hh != R(0) || (meta >> 8) != 0u;
+                    continue;
+                }
                 const bool own_cell = own_lane && warp != 0 && r >= r0 && r < r_end;
                 // a pending map record keeps the depth this step starts from
                 if (sh.now.rec >= 0 && own_cell) a.rec.snap[size_t(sh.now.rec) * (size_t(ny) * nx) + c] = hh;
@@ -231,7 +248,7 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
             }
         }
         x_h[warp][lane] = warp == 0 ? hT[0] : hT[RPT - 1];
-        const bool busy = __syncthreads_or(wet || !(K.thr > R(0))) != 0;
+        const bool busy = __syncthreads_or(wet || (!LI && !(K.thr > R(0)))) != 0;
         if (!busy) {
             // dry through: what (B)-(F) would store
             if (fo && fi) {
@@ -240,8 +257,11 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
 #pragma unroll
                 for (int i = 0; i < RPT; ++i) {
                     const int r = rw + i;
-                    if (own_lane && warp != 0 && r >= r0 && r < r_end)
-                        sout[size_t(r) * nx + j] = V4{R(0), R(0), R(0), R(0) > X[i].w ? R(0) : X[i].w};
+                    if (own_lane && warp != 0 && r >= r0 && r < r_end) {
+                        const size_t c = size_t(r) * nx + j;
+                        sout[c] = V4{R(0), R(0), R(0), !LI && R(0) > X[i].w ? R(0) : X[i].w};
+                        if (LI) li.hfx[c] = li.hfy[c] = R(0);
+                    }
                 }
                 if (fl_out && tid == 0) *fl_out = 1;
             }
@@ -354,7 +374,7 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
                 }
             }
 #pragma unroll
-            for (int i = 0; i < RPT; ++i) vu[i] = face_velocity(qyl[i], hfy[i], K);   // of the upper face
+            for (int i = 0; i < RPT; ++i) vu[i] = LI ? R(0) : face_velocity(qyl[i], hfy[i], K);   // of the upper face
             x_l[warp][lane] = qyl[0];
             x_v[warp][lane] = vu[0];
             bar_sync<2, NT>();
@@ -363,7 +383,7 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
             for (int i = 0; i < RPT; ++i) {
                 const int r = rw + i;
                 const R qxl_left = __shfl_up_sync(FULL, qxl[i], 1);
-                const R vr = face_velocity(qxl[i], hfx[i], K);
+                const R vr = LI ? R(0) : face_velocity(qxl[i], hfx[i], K);
                 if (!(own_lane && r >= r0 && r < r_end)) continue;
                 const R qyd = i + 1 < RPT ? qyl[i + 1 < RPT ? i + 1 : i] : x_l[warp + 1 < NW ? warp + 1 : 0][lane];
                 const R vb = i + 1 < RPT ? vu[i + 1 < RPT ? i + 1 : i] : x_v[warp + 1 < NW ? warp + 1 : 0][lane];
@@ -371,7 +391,7 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
                 const unsigned meta = meta_bits(S[i].w);
                 const bool mine = r >= a.own_r0 && r < a.own_r1;
                 // a control structure's transfers join the depth after the fluxes
-                R h_in = hT[i];
+                R h_in = LI ? X[i].x : hT[i];
                 if (INFL && (meta & kInflowBit)) {
                     const int ss = a.inflow.cell_struct[(meta >> 8) & 0x7FFFFFu];
                     if (ss >= 0) h_in = h_in + a.strct.extra[ss];
@@ -387,17 +407,23 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
                     a.hf3[o] = ho;
                     a.qo[o] = qq;
                     if (mine) out_acc_r.add(qq * K.dt);
-                    if (mine && !(a.ga && (meta & 255u) != 255u) &&
+                    if (!LI && mine && !(a.ga && (meta & 255u) != 255u) &&
                         hn + (MAP ? rain_at_cell(a, sh.rsn, r, j) : sh.rsn.depth) < R(-1e-11))
                         sh.negn = 1;
                 }
-                if (INFL && (meta & kInflowBit)) {   // stage hydrograph
+                if (!LI && INFL && (meta & kInflowBit)) {   // stage hydrograph
                     const int sg = a.inflow.cell_stage[(meta >> 8) & 0x7FFFFFu];
                     if (sg >= 0) {
                         const R sv = a.inflow.stage_now[sg];
                         atomicAdd(&sh.stage, double(sv) - double(hn));
                         hn = sv;
                     }
+                }
+                if constexpr (LI) {
+                    sout[c] = V4{hn, qxl[i], qyl[i], X[i].w};
+                    li.hfx[c] = hfx[i];
+                    li.hfy[c] = hfy[i];
+                    continue;
                 }
                 const R negtol = -K.tol;
                 nbad += (hn >= negtol || !mine) ? 0u : 1u;
@@ -447,15 +473,52 @@ __global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB
     if (MAP) rain_acc += rain_acc_r.value();
     if (INF) inf_acc += inf_acc_r.value();
     if (out_acc_r.any()) out_acc += out_acc_r.value();
-    step_finish<R, NT, INF, MAP, INFL, true>(a, sh, rain_acc, inf_acc, out_acc, s2max, cmaxv, nbad, false, phase, sout,
-                                             gout);
+    if constexpr (LI) {
+        if (__any_sync(FULL, out_acc != 0.0)) {
+            out_acc = warp_sum(out_acc);
+            if (lane == 0) atomicAdd(&a.sc->acc_out, out_acc);
+        }
+    } else {
+        step_finish<R, NT, INF, MAP, INFL, true>(a, sh, rain_acc, inf_acc, out_acc, s2max, cmaxv, nbad, false, phase, sout,
+                                                 gout);
+    }
+}
+
+template <typename R, int RPT, int INF, bool MAP, bool INFL, int SCH>
+__global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB)
+k_tile_step(const __grid_constant__ FusedArgs<R> a, int phase) {
+    const LiArgs<R> none{};
+    tile_body<R, RPT, INF, MAP, INFL, SCH, false>(a, phase, none);
+}
+template <typename R, int RPT, bool INFL, int SCH>
+__global__ void __launch_bounds__(TileShape<R, RPT>::NT, TileShape<R, RPT>::MINB)
+k_tile_li(const __grid_constant__ FusedArgs<R> a, int cur, const __grid_constant__ LiArgs<R> li) {
+    tile_body<R, RPT, 0, false, INFL, SCH, true>(a, cur, li);
 }
 
 // the tile step of a grid: infiltration model, rain from maps, boundary-cell variant, faces of
 // schemes 2/3 (defined in hp2d_tile_f32.cu and hp2d_tile_f64.cu)
 template <typename R> void launch_tile_step(const FusedArgs<R>& a, int inf, bool map, bool infl, bool sch, int phase, cudaStream_t st);
+// the routing step alone, from buffer `cur` to the other one (infl: control structures)
+template <typename R> void launch_tile_li(const FusedArgs<R>& a, const LiArgs<R>& li, bool infl, bool sch, int cur, cudaStream_t st);
 
 #ifdef HP2D_TILE_INSTANTIATE
+// kernels whose shared memory exceeds the default opt in, once per device; one TileOptIn per group of
+// kernels
+struct TileOptIn {
+    std::mutex mu;
+    unsigned long long done[4] = {};
+};
+template <typename K> static void tile_opt_in(K kernel, size_t smem, int v, TileOptIn* o) {
+    if (smem + 20 * 1024 <= 48 * 1024) return;   // with the static part
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(o->mu);
+    if (dev > 63 || !((o->done[v] >> dev) & 1ull)) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (dev <= 63) o->done[v] |= 1ull << dev;
+    }
+}
 template <typename R, int RPT, int INF, bool MAP>
 static void launch_tile_v(const FusedArgs<R>& a, bool infl, bool sch, int phase, cudaStream_t st) {
     constexpr int NT = TileShape<R, RPT>::NT;
@@ -463,18 +526,8 @@ static void launch_tile_v(const FusedArgs<R>& a, bool infl, bool sch, int phase,
     const unsigned grid = a.n_ctas < a.tile_grid ? a.n_ctas : a.tile_grid;
     auto* const kernel = sch ? k_tile_step<R, RPT, INF, MAP, true, 1>
                          : infl ? k_tile_step<R, RPT, INF, MAP, true, 0> : k_tile_step<R, RPT, INF, MAP, false, 0>;
-    if (smem + 20 * 1024 > 48 * 1024) {   // with the static part beyond the default: opt in, once per device
-        static std::mutex mu;
-        static unsigned long long done[3] = {};
-        const int v = sch ? 2 : infl ? 1 : 0;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        std::lock_guard<std::mutex> lock(mu);
-        if (dev > 63 || !((done[v] >> dev) & 1ull)) {
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (dev <= 63) done[v] |= 1ull << dev;
-        }
-    }
+    static TileOptIn opt;
+    tile_opt_in(kernel, smem, sch ? 2 : infl ? 1 : 0, &opt);
     launch_step(kernel, grid, NT, smem, st, a, phase);
 }
 template <typename R, int RPT>
@@ -489,6 +542,21 @@ static void launch_tile_r(const FusedArgs<R>& a, int inf, bool map, bool infl, b
         if (map) launch_tile_v<R, RPT, 0, true>(a, infl, sch, phase, st);
         else launch_tile_v<R, RPT, 0, false>(a, infl, sch, phase, st);
     }
+}
+template <typename R, int RPT>
+static void launch_li_r(const FusedArgs<R>& a, const LiArgs<R>& li, bool infl, bool sch, int cur, cudaStream_t st) {
+    constexpr int NT = TileShape<R, RPT>::NT;
+    constexpr size_t smem = 2 * sizeof(typename Vec<R>::V4) * NT * RPT;
+    const unsigned grid = a.n_ctas < a.tile_grid ? a.n_ctas : a.tile_grid;
+    auto* const kernel = sch ? (infl ? k_tile_li<R, RPT, true, 1> : k_tile_li<R, RPT, false, 1>)
+                             : (infl ? k_tile_li<R, RPT, true, 0> : k_tile_li<R, RPT, false, 0>);
+    static TileOptIn opt;
+    tile_opt_in(kernel, smem, (sch ? 2 : 0) + (infl ? 1 : 0), &opt);
+    kernel<<<grid, NT, smem, st>>>(a, cur, li);
+}
+template <typename R> void launch_tile_li(const FusedArgs<R>& a, const LiArgs<R>& li, bool infl, bool sch, int cur, cudaStream_t st) {
+    if (a.tile_rpt == 2) launch_li_r<R, 2>(a, li, infl, sch, cur, st);
+    else launch_li_r<R, 1>(a, li, infl, sch, cur, st);
 }
 template <typename R> void launch_tile_step(const FusedArgs<R>& a, int inf, bool map, bool infl, bool sch, int phase, cudaStream_t st) {
     if (a.tile_rpt == 2) launch_tile_r<R, 2>(a, inf, map, infl, sch, phase, st);

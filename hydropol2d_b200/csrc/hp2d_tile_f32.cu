@@ -4,4 +4,5 @@
 
 namespace hp2d {
 template void launch_tile_step<float>(const FusedArgs<float>&, int, bool, bool, bool, int, cudaStream_t);
+template void launch_tile_li<float>(const FusedArgs<float>&, const LiArgs<float>&, bool, bool, int, cudaStream_t);
 }

@@ -4,4 +4,5 @@
 
 namespace hp2d {
 template void launch_tile_step<double>(const FusedArgs<double>&, int, bool, bool, bool, int, cudaStream_t);
+template void launch_tile_li<double>(const FusedArgs<double>&, const LiArgs<double>&, bool, bool, int, cudaStream_t);
 }
