@@ -70,6 +70,21 @@ bool make_map_nhwc(CUtensorMap* m, const void* base, int B, int H, int W, int C,
               CU_TENSOR_MAP_INTERLEAVE_NONE, kb == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+// The output [B, H, W, Co] (pixel pitch ldy) for tiles stored by TMA: BF16 epilogues with a pitch and
+// base of whole 16 bytes.  Returns whether the kernel stages its tiles (no map: it stores rows itself).
+bool make_map_out(CUtensorMap* m, void* y, int B, int H, int W, int Co, int ldy, int epi, int box) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn || (epi != EPI_BF16_BIAS && epi != EPI_BF16_BIAS_RELU) || ldy % 8 || Co % 8 ||
+        (reinterpret_cast<uintptr_t>(y) & 15u))
+        return false;
+    cuuint64_t dims[4] = {cuuint64_t(Co), cuuint64_t(W), cuuint64_t(H), cuuint64_t(B)};
+    cuuint64_t strides[3] = {cuuint64_t(ldy) * 2, cuuint64_t(W) * ldy * 2, cuuint64_t(H) * W * ldy * 2};
+    cuuint32_t bx[4] = {cuuint32_t(box), cuuint32_t(kTX), cuuint32_t(kTY), 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, y, dims, strides, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              box == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 TileGeom tile_geom(int B, int H, int W) {
     const int tx = (W + kTX - 1) / kTX, ty = (H + kTY - 1) / kTY;
     return TileGeom{H, W, tx, ty, B * tx * ty};
@@ -225,7 +240,9 @@ hp2d_status conv_halo(const void* x, int B, int H, int W, const void* w, int ldw
     if (!n) return launched("cudaFuncSetAttribute");
     const TileGeom g = tile_geom(B, H, W);
     const int ctas = std::min(g.total, n * int(std::min<size_t>(227 * 1024 / (smem + 1024), 4)));
-    k_conv_halo<CB, BN><<<ctas, kPtThreads, smem, st>>>(mx, mw, Co, y, ldy, bias, epi, err, g);
+    CUtensorMap my{};
+    const int staged = make_map_out(&my, y, B, H, W, Co, ldy, epi, out_box<BN>());
+    k_conv_halo<CB, BN><<<ctas, kPtThreads, smem, st>>>(mx, mw, my, staged, Co, y, ldy, bias, epi, err, g);
     return launched("k_conv_halo");
 }
 template <int C, int BN>
@@ -234,12 +251,14 @@ hp2d_status conv_small(const uint16_t* x, int B, int H, int W, const void* w, in
     CUtensorMap mw;
     if (!make_map(&mw, w, Co, 64, ldw, BN)) return fail("cuTensorMapEncodeTiled rejected the weights (alignment or pitch)");
     static int sms[64] = {};
-    constexpr size_t smem = kBM * 128 + BN * 128 + 1024;
+    constexpr size_t smem = kBM * 128 + BN * 128 + out_bytes<BN>() + 1024;
     const int n = kernel_setup(k_conv_small<C, BN>, smem, sms);
     if (!n) return launched("cudaFuncSetAttribute");
     const TileGeom g = tile_geom(B, H, W);
     const int per_sm = std::min(8, 512 / BN);
-    k_conv_small<C, BN><<<std::min(g.total, n * per_sm), 128, smem, st>>>(x, mw, Co, y, ldy, bias, epi, err, g);
+    CUtensorMap my{};
+    const int staged = make_map_out(&my, y, B, H, W, Co, ldy, epi, out_box<BN>());
+    k_conv_small<C, BN><<<std::min(g.total, n * per_sm), 128, smem, st>>>(x, mw, my, staged, Co, y, ldy, bias, epi, err, g);
     return launched("k_conv_small");
 }
 template <int C>

@@ -33,26 +33,77 @@ template <int CB> __device__ __forceinline__ uint64_t row_desc(uint32_t addr, ui
     d |= uint64_t(CB == 64 ? 2u : 4u) << 61;       // 128- or 64-byte swizzle
     return d;
 }
+// ---- BF16 output tiles through shared memory -----------------------------------------------------
+// A thread holds a pixel's channels: stored straight to memory, a warp's 16-byte stores are 64 or more
+// bytes apart and each writes half a sector, and the layers' time followed their output (16 x 256^2,
+// 32 -> 32 channels 82 us, 32 -> 64 127 us).  Instead the tile is laid out in shared memory as TMA
+// stores it, rows of OB = 32 or 64 channels a pixel in the 64- or 128-byte swizzle, and one TMA copy
+// writes it; rows and columns outside the image are left out by the copy.
+template <int BN> __host__ __device__ constexpr int out_box() { return BN >= 64 ? 64 : 32; }   // channels of a box
+template <int BN> __host__ __device__ constexpr uint32_t out_bytes() { return uint32_t(kBM * BN * 2); }
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+                 : "memory");
+}
+__device__ __forceinline__ void store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// at most N of this thread's latest stores still read shared memory / are not complete
+template <int N> __device__ __forceinline__ void store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+template <int N> __device__ __forceinline__ void store_wait() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }
+template <int ID, int NTH> __device__ __forceinline__ void epi_sync() { asm volatile("barrier.sync %0, %1;" ::"n"(ID), "n"(NTH) : "memory"); }
+template <int ID, int NTH> __device__ __forceinline__ bool epi_any(bool p) {
+    int any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.red.or.pred q, %2, %3, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+                 : "=r"(any) : "r"(int(p)), "n"(ID), "n"(NTH) : "memory");
+    return any != 0;
+}
+// 32 accumulator columns (channels col0 ..) of pixel m through the epilogue into the staged tile
+template <int BN>
+__device__ __forceinline__ void stage_row32(const float (&v)[32], int col0, int Co, const float* __restrict__ bias, bool relu,
+                                            uint32_t tile, int m) {
+    constexpr int OB = out_box<BN>();
+    const uint32_t row = tile + uint32_t(col0 / OB) * uint32_t(kBM * OB * 2) + uint32_t(m) * (OB * 2);
+    const uint32_t chunk0 = uint32_t(col0 % OB) / 8u, flip = OB == 64 ? uint32_t(m & 7) : uint32_t((m >> 1) & 3);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = 8 * q + 2 * i;
+            float a = v[c] + (col0 + c < Co ? bias[col0 + c] : 0.0f);
+            float b = v[c + 1] + (col0 + c + 1 < Co ? bias[col0 + c + 1] : 0.0f);
+            if (relu) { a = fmaxf(a, 0.0f); b = fmaxf(b, 0.0f); }
+            w[i] = uint32_t(f2bf(a)) | (uint32_t(f2bf(b)) << 16);
+        }
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + 16u * ((chunk0 + uint32_t(q)) ^ flip)), "r"(w[0]),
+                     "r"(w[1]), "r"(w[2]), "r"(w[3])
+                     : "memory");
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // y[P, Co] (epilogue) = conv3x3(x[B, H, W, C]) with w[Co, >= 9C], C = CB.  One persistent CTA: the
 // weights stay in shared memory, warp 0 streams halo tiles, warp 1 issues a tile's 9 * CB/16 MMAs
 // into TMEM accumulator i % 2, warps 2-5 store accumulator i % 2 through the epilogue.  K runs over
 // taps, then channels, in steps of 16, as in the GEMMs: the results are the same bit for bit.
+// output tiles staged: two, one where the weights leave no more room
+template <int CB, int BN> __host__ __device__ constexpr int conv_outs() { return CB == 64 && BN == 128 ? 1 : 2; }
 template <int CB, int BN> __host__ __device__ constexpr int conv_stages() {
-    // as many halo tiles as fit beside the weights, at most 4; 3 where two CTAs then share an SM
-    return CB == 64 && BN == 32 ? 3
-           : int((222u * 1024u - uint32_t(9 * CB * BN * 2)) / halo_stage<CB>()) < 4
-               ? int((222u * 1024u - uint32_t(9 * CB * BN * 2)) / halo_stage<CB>()) : 4;
+    // halo tiles beside the weights and the staged outputs: 2 beside 128 x 64 channels' weights, 3 where
+    // several CTAs then share an SM, else 4
+    return CB == 64 && BN == 128 ? 2 : CB == 64 && BN == 64 ? 4 : 3;
 }
 template <int CB, int BN> __host__ __device__ constexpr size_t conv_smem() {
-    return size_t(9) * CB * BN * 2 + size_t(conv_stages<CB, BN>()) * halo_stage<CB>() + 1024;
+    return size_t(9) * CB * BN * 2 + size_t(conv_stages<CB, BN>()) * halo_stage<CB>() + conv_outs<CB, BN>() * out_bytes<BN>() + 1024;
 }
 
 template <int CB, int BN>
 __global__ void __launch_bounds__(kPtThreads, 1)
-k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, int Co, void* y, int ldy,
-            const float* __restrict__ bias, int epi, int* err, const TileGeom g) {
-    constexpr int NS = conv_stages<CB, BN>();
+k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
+            const __grid_constant__ CUtensorMap tmY, int staged, int Co, void* y, int ldy, const float* __restrict__ bias,
+            int epi, int* err, const TileGeom g) {
+    constexpr int NS = conv_stages<CB, BN>(), NO = conv_outs<CB, BN>();
     static_assert(NS >= 2, "a halo tile must load while another is used");
     constexpr uint32_t kW = CB * BN * 2;   // one tap's weights
     constexpr uint32_t kRow = CB * 2;
@@ -61,9 +112,10 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
     volatile int* fail = &s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t sW = base, sX = base + 9 * kW;   // 9 * kW is a multiple of 1024 (BN >= 32)
+    const uint32_t sY = sX + uint32_t(NS) * halo_stage<CB>();
 
     if (warp == 0) tmem_alloc(smem_addr(&s_tmem), uint32_t(2 * BN));
     if (tid == 0) {
@@ -83,7 +135,7 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     uint32_t issued = 0;
     if (warp == 0) {
@@ -104,57 +156,79 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = bf16_idesc<BN>();
-            uint32_t it = 0;
-            bool ok = bar_wait(smem_addr(&bar_w), 0u);
-            for (int t = blockIdx.x; ok && t < g.total && !pt_failed(fail); t += gridDim.x, ++it) {
-                const int s = int(it % NS), b = int(it & 1u);
-                if (it >= 2 && !bar_wait(smem_addr(&acc_empty[b]), ((it >> 1) - 1u) & 1u)) { ok = false; break; }
-                if (!bar_wait(smem_addr(&bar_full[s]), (it / NS) & 1u)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t acc = tmem + uint32_t(b * BN);
-                const uint32_t x = sX + uint32_t(s) * halo_stage<CB>();
-#pragma unroll 1
-                for (int tap = 0; tap < 9; ++tap) {
-                    const uint32_t shift = uint32_t((tap / 3) * kHX + tap % 3) * kRow;
-                    const uint64_t da = row_desc<CB>(x + shift, 16u, uint32_t(kHX) * kRow);
-                    const uint64_t db = row_desc<CB>(sW + uint32_t(tap) * kW, 16u, 8u * kRow);
+        constexpr uint32_t idesc = bf16_idesc<BN>();
+        uint32_t it = 0;
+        bool ok = bar_wait_warp(smem_addr(&bar_w), 0u);
+        for (int t = blockIdx.x; ok && t < g.total && !pt_failed_warp(fail); t += gridDim.x, ++it) {
+            const int s = int(it % NS), b = int(it & 1u);
+            if (it >= 2 && !bar_wait_warp(smem_addr(&acc_empty[b]), ((it >> 1) - 1u) & 1u)) { ok = false; break; }
+            if (!bar_wait_warp(smem_addr(&bar_full[s]), (it / NS) & 1u)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t acc = tmem + uint32_t(b * BN);
+            const uint64_t da = row_desc<CB>(sX + uint32_t(s) * halo_stage<CB>(), 16u, uint32_t(kHX) * kRow);
+            const uint64_t db = row_desc<CB>(sW, 16u, 8u * kRow);
 #pragma unroll
-                    for (int kk = 0; kk < CB / 16; ++kk)
-                        tc_mma_bf16(acc, da + uint64_t(2 * kk), db + uint64_t(2 * kk), idesc, (tap | kk) != 0 ? 1u : 0u);
-                }
-                tc_commit(smem_addr(&bar_empty[s]));
-                tc_commit(smem_addr(&acc_full[b]));
+            for (int tap = 0; tap < 9; ++tap) {   // offsets in the descriptors' 16-byte units
+                const uint64_t oa = uint64_t(uint32_t((tap / 3) * kHX + tap % 3) * kRow / 16u), ob = uint64_t(uint32_t(tap) * kW / 16u);
+#pragma unroll
+                for (int kk = 0; kk < CB / 16; ++kk)
+                    tc_mma_bf16(acc, da + (oa + uint64_t(2 * kk)), db + (ob + uint64_t(2 * kk)), idesc, (tap | kk) != 0 ? 1u : 0u);
             }
-            if (!ok) *fail = 1;
-            // every MMA this thread issued has completed before the TMEM can be released
-            tc_commit(smem_addr(&bar_done));
-            if (!bar_wait(smem_addr(&bar_done), 0u)) *fail = 1;
+            tc_commit(smem_addr(&bar_empty[s]));
+            tc_commit(smem_addr(&acc_full[b]));
         }
+        if (!ok) *fail = 1;
+        // every MMA this warp issued has completed before the TMEM can be released
+        tc_commit(smem_addr(&bar_done));
+        if (!bar_wait_warp(smem_addr(&bar_done), 0u)) *fail = 1;
     } else {
         const int q = warp & 3;   // TMEM lanes 32q .. 32q + 31 = pixels of the tile
         uint32_t it = 0;
         for (int t = blockIdx.x; t < g.total; t += gridDim.x, ++it) {
             const int b = int(it & 1u);
             const bool ready = !pt_failed(fail) && bar_wait(smem_addr(&acc_full[b]), (it >> 1) & 1u);
-            if (!__all_sync(0xffffffffu, ready)) {
-                if (lane == 0) *fail = 1;
+            if (epi_any<2, 128>(!ready)) {   // the four warps leave together (they meet at barriers below)
+                *fail = 1;
                 break;
             }
             tc_fence_after();
             int img, y0, x0;
             g.at(t, img, y0, x0);
-            const int row = g.row(img, y0, x0, q * 32 + lane);
+            const int m = q * 32 + lane;
+            if (staged) {
+                const uint32_t tile = sY + (NO == 2 ? (it & 1u) : 0u) * out_bytes<BN>();
+                // the store that used this tile has read it (thread 64 issues the stores)
+                if (tid == 64) store_wait_read<NO - 1>();
+                epi_sync<1, 128>();
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                float v[32];
-                tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(b * BN + c0), v);
-                if (row >= 0) store_row32(v, row, c0, row + 1, Co, y, ldy, bias, epi);
+                for (int c0 = 0; c0 < BN; c0 += 32) {
+                    float v[32];
+                    tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(b * BN + c0), v);
+                    stage_row32<BN>(v, c0, Co, bias, epi == EPI_BF16_BIAS_RELU, tile, m);
+                }
+                tc_fence_before();
+                mbar_arrive(smem_addr(&acc_empty[b]));
+                fence_proxy_async_smem();
+                epi_sync<1, 128>();
+                if (tid == 64) {
+                    constexpr int OB = out_box<BN>();
+                    for (int c0 = 0; c0 < BN && c0 < Co; c0 += OB)
+                        tma_store_4d(&tmY, tile + uint32_t(c0 / OB) * uint32_t(kBM * OB * 2), c0, x0, y0, img);
+                    store_commit();
+                }
+            } else {
+                const int row = g.row(img, y0, x0, m);
+#pragma unroll 1
+                for (int c0 = 0; c0 < BN; c0 += 32) {
+                    float v[32];
+                    tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(b * BN + c0), v);
+                    if (row >= 0) store_row32(v, row, c0, row + 1, Co, y, ldy, bias, epi);
+                }
+                tc_fence_before();
+                mbar_arrive(smem_addr(&acc_empty[b]));
             }
-            tc_fence_before();
-            mbar_arrive(smem_addr(&acc_empty[b]));
         }
+        if (staged && tid == 64) store_wait<0>();
     }
     __syncwarp();
     tc_fence_before();
@@ -221,16 +295,16 @@ __device__ __forceinline__ void gather_row(const uint16_t* __restrict__ x, const
 // The im2col matrix this replaces was written to and read from HBM (128 bytes a pixel each way).
 template <int C, int BN>
 __global__ void __launch_bounds__(128)
-k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap tmW, int Co, void* y, int ldy,
-             const float* __restrict__ bias, int epi, int* err, const TileGeom g) {
+k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmY,
+             int staged, int Co, void* y, int ldy, const float* __restrict__ bias, int epi, int* err, const TileGeom g) {
     constexpr uint32_t kA = kBM * 128u, kB = BN * 128u;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) unsigned long long bar_w, bar_acc;
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
-    const uint32_t sA = base, sB = base + kA;
+    const uint32_t sA = base, sB = base + kA, sY = sB + kB;
     if (warp == 0) tmem_alloc(smem_addr(&s_tmem), uint32_t(BN));
     if (tid == 0) {
         mbar_init(smem_addr(&bar_w), 1u);
@@ -241,7 +315,7 @@ k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     if (tid == 0) {
         mbar_expect_tx(smem_addr(&bar_w), kB);
         tma_load_2d(sB, &tmW, 0, 0, smem_addr(&bar_w));
@@ -255,7 +329,7 @@ k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap
         fence_proxy_async_smem();
         tc_fence_before();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0) {
             tc_fence_after();
             const uint64_t da = sw128_kmajor_desc(sA), db = sw128_kmajor_desc(sB);
 #pragma unroll
@@ -266,14 +340,34 @@ k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap
         ok = bar_wait(smem_addr(&bar_acc), it & 1u) && ok;
         if (!ok) atomicExch(&s_fail, 1);
         tc_fence_after();
-        const int row = g.row(b, y0, x0, tid);
+        if (staged) {
+            if (tid == 0) store_wait_read<0>();
+            __syncthreads();
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-            float v[32];
-            tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0), v);
-            if (ok && row >= 0) store_row32(v, row, c0, row + 1, Co, y, ldy, bias, epi);
+            for (int c0 = 0; c0 < BN; c0 += 32) {
+                float v[32];
+                tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0), v);
+                stage_row32<BN>(v, c0, Co, bias, epi == EPI_BF16_BIAS_RELU, sY, tid);
+            }
+            fence_proxy_async_smem();
+            __syncthreads();
+            if (tid == 0 && ok) {
+                constexpr int OB = out_box<BN>();
+                for (int c0 = 0; c0 < BN && c0 < Co; c0 += OB)
+                    tma_store_4d(&tmY, sY + uint32_t(c0 / OB) * uint32_t(kBM * OB * 2), c0, x0, y0, b);
+                store_commit();
+            }
+        } else {
+            const int row = g.row(b, y0, x0, tid);
+#pragma unroll 1
+            for (int c0 = 0; c0 < BN; c0 += 32) {
+                float v[32];
+                tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0), v);
+                if (ok && row >= 0) store_row32(v, row, c0, row + 1, Co, y, ldy, bias, epi);
+            }
         }
     }
+    if (staged && tid == 0) store_wait<0>();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -327,7 +421,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
     volatile int* fail = &s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const int cb = int(blockIdx.y) % ci_blocks, nb = int(blockIdx.y) / ci_blocks;
     const int n_tiles = int(blockIdx.x) < g.total ? (g.total - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
@@ -345,7 +439,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     int issued = 0;
     if (warp == 0) {
@@ -368,38 +462,40 @@ k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = bf16_idesc_mn<BN>();
-            bool ok = true;
-            for (int i = 0; i < n_tiles && !pt_failed(fail); ++i) {
-                const int s = i % NS;
-                if (!bar_wait(smem_addr(&bar_full[s]), uint32_t(i / NS) & 1u)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t sa = base + uint32_t(s) * kStage, sb = sa + kA;
-#pragma unroll 1
-                for (int kk = 0; kk < kBM / 16; ++kk) {   // 16 pixels: two rows of the tile
-                    const uint64_t db = row_desc<BN>(sb + uint32_t(16 * kk) * (BN * 2), 16u, 8u * (BN * 2));
+        constexpr uint32_t idesc = bf16_idesc_mn<BN>();
+        bool ok = true;
+        for (int i = 0; i < n_tiles && !pt_failed_warp(fail); ++i) {
+            const int s = i % NS;
+            if (!bar_wait_warp(smem_addr(&bar_full[s]), uint32_t(i / NS) & 1u)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t sa = base + uint32_t(s) * kStage, sb = sa + kA;
+            const uint64_t db = row_desc<BN>(sb, 16u, 8u * (BN * 2));
+            // the descriptor of each of the NM products; a 16-pixel step moves its start
+            uint64_t da[NM];
 #pragma unroll
-                    for (int q = 0; q < NM; ++q) {
-                        uint64_t da;
-                        if (SMALL) {
-                            da = row_desc<64>(sa + uint32_t(16 * kk) * 128u, 0u, 1024u);   // rows 64..127 repeat 0..63
-                        } else if (CB == 64) {
-                            const int t0 = 2 * q, t1 = t0 + 1;
-                            const uint32_t o0 = uint32_t((t0 / 3) * kHX + t0 % 3), o1 = uint32_t((t1 / 3) * kHX + t1 % 3);
-                            const uint32_t lead = t1 < 9 ? (o1 - o0) * kRow : kRow;
-                            da = row_desc<CB>(sa + (uint32_t(2 * kk * kHX) + o0) * kRow, lead, uint32_t(kHX) * kRow);
-                        } else {
-                            da = row_desc<CB>(sa + uint32_t((2 * kk + q) * kHX) * kRow, kRow, uint32_t(kHX) * kRow);
-                        }
-                        tc_mma_bf16(tmem + uint32_t(q * BN), da, db, idesc, (i | kk) != 0 ? 1u : 0u);
-                    }
+            for (int q = 0; q < NM; ++q) {
+                if (SMALL) {
+                    da[q] = row_desc<64>(sa, 0u, 1024u);   // rows 64..127 repeat 0..63
+                } else if (CB == 64) {
+                    const int t0 = 2 * q, t1 = t0 + 1;
+                    const uint32_t o0 = uint32_t((t0 / 3) * kHX + t0 % 3), o1 = uint32_t((t1 / 3) * kHX + t1 % 3);
+                    da[q] = row_desc<CB>(sa + o0 * kRow, t1 < 9 ? (o1 - o0) * kRow : kRow, uint32_t(kHX) * kRow);
+                } else {
+                    da[q] = row_desc<CB>(sa + uint32_t(q * kHX) * kRow, kRow, uint32_t(kHX) * kRow);
                 }
-                tc_commit(smem_addr(&bar_empty[s]));
             }
-            if (!ok) *fail = 1;
-            tc_commit(smem_addr(&bar_done));   // arrives once every MMA issued above has completed
+#pragma unroll
+            for (int kk = 0; kk < kBM / 16; ++kk) {   // 16 pixels: two rows of the tile
+                const uint64_t oa = uint64_t((SMALL ? uint32_t(16 * kk) * 128u : uint32_t(2 * kk * kHX) * kRow) / 16u);
+                const uint64_t ob = uint64_t(uint32_t(16 * kk) * (BN * 2) / 16u);
+#pragma unroll
+                for (int q = 0; q < NM; ++q)
+                    tc_mma_bf16(tmem + uint32_t(q * BN), da[q] + oa, db + ob, idesc, (i | kk) != 0 ? 1u : 0u);
+            }
+            tc_commit(smem_addr(&bar_empty[s]));
         }
+        if (!ok) *fail = 1;
+        tc_commit(smem_addr(&bar_done));   // arrives once every MMA issued above has completed
     } else if (kGather) {
         const int m = tid - 64;   // pixel of the tile
         for (int i = 0; i < n_tiles && !pt_failed(fail); ++i) {

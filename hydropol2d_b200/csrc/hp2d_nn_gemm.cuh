@@ -7,7 +7,7 @@
 //   * thread 0 streams 128 x 64 and BN x 64 tiles of A and B into a ring of kStages
 //     shared-memory stages with 2-D TMA copies (128-byte swizzle), completion counted in
 //     bytes on the stage's `full` barrier;
-//   * thread 32 issues four tcgen05.mma (M = 128, N = BN, K = 16) per stage into a TMEM
+//   * warp 1 issues four tcgen05.mma (M = 128, N = BN, K = 16) per stage into a TMEM
 //     accumulator of BN columns and frees the stage with tcgen05.commit on `empty`;
 //   * after the last stage a commit on `done` releases the epilogue: warp w reads TMEM
 //     lanes 32w..32w+31 (tile rows) with tcgen05.ld and writes its rows to global memory.
@@ -85,15 +85,23 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// The MMAs and commits are issued by one elected lane of a warp whose lanes all run the loop around
+// them: the descriptors are then uniform values, formed in uniform registers.  With one thread alone
+// in the loop each MMA waited for its descriptors' moves, about 110 cycles where a 128 x 32 x 16 MMA
+// needs 40.
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)
+        : "memory");
 }
 __device__ __forceinline__ void tc_mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
@@ -153,6 +161,11 @@ template <int BN> __device__ __forceinline__ constexpr uint32_t bf16_idesc() {
 
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
     return mbar_wait_bounded(bar, parity, kWaitLimit);
+}
+
+// the same by a whole warp that goes on (or gives up) together
+__device__ __forceinline__ bool bar_wait_warp(uint32_t bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, kWaitLimit));
 }
 
 // round-to-nearest-even FP32 -> BF16
@@ -218,7 +231,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t sA0 = base, sB0 = base + kGemmStages * kABytes;
     const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
@@ -238,7 +251,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     int issued = 0;
     if (tid == 0 && nk > 0) {
@@ -265,12 +278,12 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             tma_load_2d(sB0 + uint32_t(s) * kBBytes, &tmB, kx, n0, fb);
             issued = i + 1;
         }
-    } else if (tid == 32) {
+    } else if (warp == 1) {
         // MMA issuer
         constexpr uint32_t idesc = bf16_idesc<BN>();
         for (int i = 0; i < nk; ++i) {
             const int s = i % kGemmStages;
-            if (!bar_wait(smem_addr(&bar_full[s]), uint32_t((i / kGemmStages) & 1))) {
+            if (!bar_wait_warp(smem_addr(&bar_full[s]), uint32_t((i / kGemmStages) & 1))) {
                 atomicExch(&s_fail, 1);
                 break;
             }
@@ -321,7 +334,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 // Persistent form (grids of more tiles than SMs).  One CTA of 192 threads per SM walks the tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ... of the (m, n, split) tile grid, m fastest:
 //   * warp 0 lane 0 streams the k tiles of every tile through the same stage ring;
-//   * warp 1 lane 0 issues the MMAs of the CTA's i-th tile into TMEM accumulator i % 2 (2 x BN
+//   * warp 1 issues the MMAs of the CTA's i-th tile into TMEM accumulator i % 2 (2 x BN
 //     columns allocated) and commits `acc_full[i % 2]` after its last k tile;
 //   * warps 2-5 drain accumulator i % 2 (warp w reads TMEM lanes 32 (w % 4) ..) through the
 //     epilogue and release it on `acc_empty[i % 2]` (128 arrivals),
@@ -331,6 +344,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 constexpr int kPtThreads = 192;
 
 __device__ __forceinline__ bool pt_failed(const volatile int* f) { return *f != 0; }
+__device__ __forceinline__ bool pt_failed_warp(const volatile int* f) { return __any_sync(0xffffffffu, *f != 0); }
 
 template <int BN, int KB = kBK, bool IM2COL = false>
 __global__ void __launch_bounds__(kPtThreads, 1)
@@ -349,7 +363,7 @@ k_gemm_bf16_pt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __shared__ int s_fail;
     volatile int* fail = &s_fail;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t sA0 = base, sB0 = base + kGemmStages * kABytes;
     const int total = mtiles * ntiles * splits;
@@ -371,7 +385,7 @@ k_gemm_bf16_pt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     // tile t: rows m0.., columns n0.., k tiles kt0 .. kt0 + nk - 1
     auto tile = [&](int t, int& m0, int& n0, int& kt0, int& nk) {
@@ -414,47 +428,45 @@ k_gemm_bf16_pt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = bf16_idesc<BN>();
-            uint32_t it = 0;
-            int lt = 0;
-            for (int t = blockIdx.x; t < total && !pt_failed(fail); t += gridDim.x) {
-                int m0, n0, kt0, nk;
-                tile(t, m0, n0, kt0, nk);
-                if (nk <= 0) continue;
-                const int b = lt & 1;
-                if (lt >= 2 && !bar_wait(smem_addr(&acc_empty[b]), uint32_t((lt >> 1) - 1) & 1u)) {
-                    *fail = 1;
+        constexpr uint32_t idesc = bf16_idesc<BN>();
+        uint32_t it = 0;
+        int lt = 0;
+        for (int t = blockIdx.x; t < total && !pt_failed_warp(fail); t += gridDim.x) {
+            int m0, n0, kt0, nk;
+            tile(t, m0, n0, kt0, nk);
+            if (nk <= 0) continue;
+            const int b = lt & 1;
+            if (lt >= 2 && !bar_wait_warp(smem_addr(&acc_empty[b]), uint32_t((lt >> 1) - 1) & 1u)) {
+                *fail = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t acc = tmem + uint32_t(b * BN);
+            bool ok = true;
+            for (int i = 0; i < nk; ++i, ++it) {
+                const int s = int(it % kGemmStages);
+                if (!bar_wait_warp(smem_addr(&bar_full[s]), (it / kGemmStages) & 1u)) {
+                    ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t acc = tmem + uint32_t(b * BN);
-                bool ok = true;
-                for (int i = 0; i < nk; ++i, ++it) {
-                    const int s = int(it % kGemmStages);
-                    if (!bar_wait(smem_addr(&bar_full[s]), (it / kGemmStages) & 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint64_t da = kmajor_desc<KB>(sA0 + uint32_t(s) * kABytes);
-                    const uint64_t db = kmajor_desc<KB>(sB0 + uint32_t(s) * kBBytes);
+                const uint64_t da = kmajor_desc<KB>(sA0 + uint32_t(s) * kABytes);
+                const uint64_t db = kmajor_desc<KB>(sB0 + uint32_t(s) * kBBytes);
 #pragma unroll
-                    for (int kk = 0; kk < KB / 16; ++kk)
-                        tc_mma_bf16(acc, da + uint64_t(2 * kk), db + uint64_t(2 * kk), idesc, (i | kk) != 0 ? 1u : 0u);
-                    tc_commit(smem_addr(&bar_empty[s]));
-                }
-                if (!ok) {
-                    *fail = 1;
-                    break;
-                }
-                tc_commit(smem_addr(&acc_full[b]));
-                ++lt;
+                for (int kk = 0; kk < KB / 16; ++kk)
+                    tc_mma_bf16(acc, da + uint64_t(2 * kk), db + uint64_t(2 * kk), idesc, (i | kk) != 0 ? 1u : 0u);
+                tc_commit(smem_addr(&bar_empty[s]));
             }
-            // every MMA this thread issued has completed before the TMEM can be released
-            tc_commit(smem_addr(&bar_done));
-            if (!bar_wait(smem_addr(&bar_done), 0u)) *fail = 1;
+            if (!ok) {
+                *fail = 1;
+                break;
+            }
+            tc_commit(smem_addr(&acc_full[b]));
+            ++lt;
         }
+        // every MMA this warp issued has completed before the TMEM can be released
+        tc_commit(smem_addr(&bar_done));
+        if (!bar_wait_warp(smem_addr(&bar_done), 0u)) *fail = 1;
     } else {
         const int q = warp & 3;   // TMEM lanes 32q .. 32q + 31 = tile rows
         int lt = 0;
