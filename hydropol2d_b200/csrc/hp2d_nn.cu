@@ -70,20 +70,10 @@ bool make_map_nhwc(CUtensorMap* m, const void* base, int B, int H, int W, int C,
               CU_TENSOR_MAP_INTERLEAVE_NONE, kb == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// The output [B, H, W, Co] (pixel pitch ldy) for tiles stored by TMA: BF16 epilogues with a pitch and
-// base of whole 16 bytes.  Returns whether the kernel stages its tiles (no map: it stores rows itself).
-bool make_map_out(CUtensorMap* m, void* y, int B, int H, int W, int Co, int ldy, int epi, int box) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn || (epi != EPI_BF16_BIAS && epi != EPI_BF16_BIAS_RELU) || ldy % 8 || Co % 8 ||
-        (reinterpret_cast<uintptr_t>(y) & 15u))
-        return false;
-    cuuint64_t dims[4] = {cuuint64_t(Co), cuuint64_t(W), cuuint64_t(H), cuuint64_t(B)};
-    cuuint64_t strides[3] = {cuuint64_t(ldy) * 2, cuuint64_t(W) * ldy * 2, cuuint64_t(H) * W * ldy * 2};
-    cuuint32_t bx[4] = {cuuint32_t(box), cuuint32_t(kTX), cuuint32_t(kTY), 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, y, dims, strides, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              box == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+// whether output rows can be written in 16-byte pieces (else the kernels store them element by element)
+bool pieces_out(const void* y, int Co, int ldy, int epi) {
+    return (epi == EPI_BF16_BIAS || epi == EPI_BF16_BIAS_RELU) && ldy % 8 == 0 && Co % 8 == 0 &&
+           (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
 }
 TileGeom tile_geom(int B, int H, int W) {
     const int tx = (W + kTX - 1) / kTX, ty = (H + kTY - 1) / kTY;
@@ -229,7 +219,7 @@ template <typename K> int kernel_setup(K kernel, size_t smem, int (&sms)[64]) {
 }
 
 template <int CB, int BN>
-hp2d_status conv_halo(const void* x, int B, int H, int W, const void* w, int ldw, int Co, const float* bias, void* y,
+hp2d_status conv_halo(const uint16_t* x, int B, int H, int W, const void* w, int ldw, int Co, const float* bias, void* y,
                       int ldy, int epi, int* err, cudaStream_t st) {
     CUtensorMap mx, mw;
     if (!make_map_nhwc(&mx, x, B, H, W, CB, CB, kHX, kHY) || !make_map(&mw, w, Co, 9 * CB, ldw, BN, CB))
@@ -239,10 +229,9 @@ hp2d_status conv_halo(const void* x, int B, int H, int W, const void* w, int ldw
     const int n = kernel_setup(k_conv_halo<CB, BN>, smem, sms);
     if (!n) return launched("cudaFuncSetAttribute");
     const TileGeom g = tile_geom(B, H, W);
-    const int ctas = std::min(g.total, n * int(std::min<size_t>(227 * 1024 / (smem + 1024), 4)));
-    CUtensorMap my{};
-    const int staged = make_map_out(&my, y, B, H, W, Co, ldy, epi, out_box<BN>());
-    k_conv_halo<CB, BN><<<ctas, kPtThreads, smem, st>>>(mx, mw, my, staged, Co, y, ldy, bias, epi, err, g);
+    const int ctas = std::min(g.total, n * conv_ctas<CB, BN>());
+    k_conv_halo<CB, BN><<<ctas, conv_threads<CB, BN>(), smem, st>>>(x, mx, mw, pieces_out(y, Co, ldy, epi), Co, y, ldy, bias,
+                                                                       epi, err, g);
     return launched("k_conv_halo");
 }
 template <int C, int BN>
@@ -256,9 +245,8 @@ hp2d_status conv_small(const uint16_t* x, int B, int H, int W, const void* w, in
     if (!n) return launched("cudaFuncSetAttribute");
     const TileGeom g = tile_geom(B, H, W);
     const int per_sm = std::min(8, 512 / BN);
-    CUtensorMap my{};
-    const int staged = make_map_out(&my, y, B, H, W, Co, ldy, epi, out_box<BN>());
-    k_conv_small<C, BN><<<std::min(g.total, n * per_sm), 128, smem, st>>>(x, mw, my, staged, Co, y, ldy, bias, epi, err, g);
+    k_conv_small<C, BN><<<std::min(g.total, n * per_sm), 128, smem, st>>>(x, mw, pieces_out(y, Co, ldy, epi), Co, y, ldy, bias,
+                                                                          epi, err, g);
     return launched("k_conv_small");
 }
 template <int C>

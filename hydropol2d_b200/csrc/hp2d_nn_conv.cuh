@@ -35,22 +35,11 @@ template <int CB> __device__ __forceinline__ uint64_t row_desc(uint32_t addr, ui
 }
 // ---- BF16 output tiles through shared memory -----------------------------------------------------
 // A thread holds a pixel's channels: stored straight to memory, a warp's 16-byte stores are 64 or more
-// bytes apart and each writes half a sector, and the layers' time followed their output (16 x 256^2,
-// 32 -> 32 channels 82 us, 32 -> 64 127 us).  Instead the tile is laid out in shared memory as TMA
-// stores it, rows of OB = 32 or 64 channels a pixel in the 64- or 128-byte swizzle, and one TMA copy
-// writes it; rows and columns outside the image are left out by the copy.
-template <int BN> __host__ __device__ constexpr int out_box() { return BN >= 64 ? 64 : 32; }   // channels of a box
+// bytes apart, and the layers' time followed their output (16 x 256^2, 32 -> 32 channels 82 us,
+// 32 -> 64 127 us).  Instead the tile is laid out in shared memory, rows of BN channels a pixel with
+// their 16-byte pieces exchanged so that neither side meets bank conflicts, and written out along its
+// rows, 512 contiguous bytes a warp (written by TMA, the two layers took 57 us each, now 45 and 55).
 template <int BN> __host__ __device__ constexpr uint32_t out_bytes() { return uint32_t(kBM * BN * 2); }
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
-                     reinterpret_cast<uint64_t>(map)),
-                 "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
-}
-__device__ __forceinline__ void store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// at most N of this thread's latest stores still read shared memory / are not complete
-template <int N> __device__ __forceinline__ void store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-template <int N> __device__ __forceinline__ void store_wait() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }
 template <int ID, int NTH> __device__ __forceinline__ void epi_sync() { asm volatile("barrier.sync %0, %1;" ::"n"(ID), "n"(NTH) : "memory"); }
 template <int ID, int NTH> __device__ __forceinline__ bool epi_any(bool p) {
     int any;
@@ -58,52 +47,129 @@ template <int ID, int NTH> __device__ __forceinline__ bool epi_any(bool p) {
                  : "=r"(any) : "r"(int(p)), "n"(ID), "n"(NTH) : "memory");
     return any != 0;
 }
-// 32 accumulator columns (channels col0 ..) of pixel m through the epilogue into the staged tile
+template <int BN> __device__ __forceinline__ uint32_t staged_at(uint32_t tile, int m, uint32_t piece) {
+    const uint32_t flip = BN == 32 ? uint32_t((m >> 1) & 3) : uint32_t(m & 7);
+    return tile + uint32_t(m) * (BN * 2) + 16u * (piece ^ flip);
+}
+// 32 accumulator columns (channels col0 ..) of pixel m through the epilogue into the staged tile, two
+// channels an instruction; s_bias holds the columns' biases.  An epilogue warp has a scheduler almost
+// to itself, so its instructions are the tile's time.
 template <int BN>
-__device__ __forceinline__ void stage_row32(const float (&v)[32], int col0, int Co, const float* __restrict__ bias, bool relu,
-                                            uint32_t tile, int m) {
-    constexpr int OB = out_box<BN>();
-    const uint32_t row = tile + uint32_t(col0 / OB) * uint32_t(kBM * OB * 2) + uint32_t(m) * (OB * 2);
-    const uint32_t chunk0 = uint32_t(col0 % OB) / 8u, flip = OB == 64 ? uint32_t(m & 7) : uint32_t((m >> 1) & 3);
+__device__ __forceinline__ void stage_row32(const float (&v)[32], int col0, const float* s_bias, bool relu, uint32_t tile, int m) {
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         uint32_t w[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 4; i += 2) {
             const int c = 8 * q + 2 * i;
-            float a = v[c] + (col0 + c < Co ? bias[col0 + c] : 0.0f);
-            float b = v[c + 1] + (col0 + c + 1 < Co ? bias[col0 + c + 1] : 0.0f);
-            if (relu) { a = fmaxf(a, 0.0f); b = fmaxf(b, 0.0f); }
-            w[i] = uint32_t(f2bf(a)) | (uint32_t(f2bf(b)) << 16);
+            const float4 bb = *reinterpret_cast<const float4*>(s_bias + col0 + c);
+            __nv_bfloat162 lo = __floats2bfloat162_rn(v[c] + bb.x, v[c + 1] + bb.y);
+            __nv_bfloat162 hi = __floats2bfloat162_rn(v[c + 2] + bb.z, v[c + 3] + bb.w);
+            if (relu) {   // rounding keeps the sign, so it may come first
+                lo = __hmax2(lo, zero);
+                hi = __hmax2(hi, zero);
+            }
+            w[i] = *reinterpret_cast<uint32_t*>(&lo);
+            w[i + 1] = *reinterpret_cast<uint32_t*>(&hi);
         }
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + 16u * ((chunk0 + uint32_t(q)) ^ flip)), "r"(w[0]),
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(staged_at<BN>(tile, m, uint32_t(col0 / 8 + q))), "r"(w[0]),
                      "r"(w[1]), "r"(w[2]), "r"(w[3])
                      : "memory");
     }
 }
+// the staged tile to the output, by 128 threads (e: this thread's place among them): its pieces lie
+// whole tile rows apart
+template <int BN>
+__device__ __forceinline__ void write_tile(uint32_t tile, const TileGeom& g, int b, int y0, int x0, int Co, uint16_t* out, int ldy,
+                                           int e) {
+    constexpr int PP = BN / 8;             // 16-byte pieces of a pixel
+    constexpr int kStep = kBM / PP;        // pixels between a thread's pieces
+    const int m = e / PP, piece = e % PP;
+    const int x = x0 + m % kTX;
+    int y = y0 + m / kTX;
+    if (x >= g.W || 8 * piece >= Co) return;
+    uint16_t* p = out + (size_t(b * g.H + y) * g.W + x) * ldy + 8 * piece;
+    const size_t step = size_t(kStep / kTX) * g.W * ldy;
+    uint32_t at = staged_at<BN>(tile, m, uint32_t(piece));   // kStep is a multiple of 8: the exchange stays
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+        uint32_t w0, w1, w2, w3;
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3) : "r"(at));
+        if (y < g.H) *reinterpret_cast<uint4*>(p) = make_uint4(w0, w1, w2, w3);
+        at += uint32_t(kStep) * (BN * 2);
+        p += step;
+        y += kStep / kTX;
+    }
+}
+// the biases of BN output columns (zero beyond Co) into shared memory
+__device__ __forceinline__ void load_bias(float* s_bias, int bn, const float* __restrict__ bias, int Co, int tid, int nt) {
+    for (int c = tid; c < bn; c += nt) s_bias[c] = bias && c < Co ? bias[c] : 0.0f;
+}
+// One 10 x 18 pixel halo tile of CB channels into shared memory by the kLoaders threads of the loading
+// warps (e: this thread's place among them), 16 bytes a copy, in the layout TMA would give it: 64- or
+// 128-byte swizzle, zeros outside the image.  A thread keeps its column and piece and steps down the
+// tile.  The 32 -> 32 channel layer loads so: by TMA its tile of 180 rows of 64 bytes took as long as
+// one of 128 (16 x 256^2: 57 us by TMA, 45 us so; the layers with 64 channels on either side are
+// faster by TMA, 64 -> 32 68 against 72 us, 32 -> 64 55 against 63 us).
+constexpr int kLoaders = 160;
+template <int CB, int BN> __host__ __device__ constexpr int conv_loaders() { return CB == 32 && BN == 32 ? kLoaders : 32; }
+template <int CB> __device__ __forceinline__ void load_halo(const uint16_t* __restrict__ x, const TileGeom& g, int b, int y0, int x0,
+                                                            uint32_t stage, int e) {
+    constexpr int PP = CB / 8, kLine = kHX * PP, kStep = kLoaders / kLine;   // pieces of a line of the tile; lines a pass
+    static_assert(kLoaders % kLine == 0, "whole lines a pass");
+    const int hy0 = e / kLine, hx = (e % kLine) / PP, piece = e % PP;
+    const int xx = x0 - 1 + hx;
+    const bool in_x = xx >= 0 && xx < g.W;
+    const uint16_t* p = x + ((int64_t(b) * g.H + (y0 - 1 + hy0)) * g.W + xx) * CB + 8 * piece;
+#pragma unroll
+    for (int i = 0; i < (kHY + kStep - 1) / kStep; ++i) {
+        const int hy = hy0 + i * kStep, yy = y0 - 1 + hy;
+        if (kHY % kStep == 0 || hy < kHY) {
+            const int r = hy * kHX + hx;
+            const bool in = in_x && yy >= 0 && yy < g.H;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             stage + uint32_t(r) * (CB * 2) + 16u * uint32_t(piece ^ (CB == 64 ? r & 7 : (r >> 1) & 3))),
+                         "l"(in ? p + int64_t(i) * kStep * g.W * CB : x), "r"(in ? 16 : 0)
+                         : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
 
 // ---------------------------------------------------------------------------------------------
-// y[P, Co] (epilogue) = conv3x3(x[B, H, W, C]) with w[Co, >= 9C], C = CB.  One persistent CTA: the
-// weights stay in shared memory, warp 0 streams halo tiles, warp 1 issues a tile's 9 * CB/16 MMAs
-// into TMEM accumulator i % 2, warps 2-5 store accumulator i % 2 through the epilogue.  K runs over
-// taps, then channels, in steps of 16, as in the GEMMs: the results are the same bit for bit.
-// output tiles staged: two, one where the weights leave no more room
-template <int CB, int BN> __host__ __device__ constexpr int conv_outs() { return CB == 64 && BN == 128 ? 1 : 2; }
+// y[P, Co] (epilogue) = conv3x3(x[B, H, W, C]) with w[Co, >= 9C], C = CB.  Persistent CTAs: the weights
+// stay in shared memory, the loading warps stream halo tiles, one warp issues a tile's 9 * CB/16 MMAs
+// into TMEM accumulator i % 2, groups of four warps store the accumulators through the epilogue.  K
+// runs over taps, then channels, in steps of 16, as in the GEMMs: the results are the same bit for bit.
+// What bounds it: the shared-memory pipe, which feeds the MMAs (a 128 x 32 x 16 MMA reads 5 KB) and
+// carries the waits' polls, about 60 % each on the 64 -> 32 layer; DRAM is at 28 % there.
 template <int CB, int BN> __host__ __device__ constexpr int conv_stages() {
-    // halo tiles beside the weights and the staged outputs: 2 beside 128 x 64 channels' weights, 3 where
-    // several CTAs then share an SM, else 4
-    return CB == 64 && BN == 128 ? 2 : CB == 64 && BN == 64 ? 4 : 3;
+    // halo tiles beside the weights and the staged output: 3, or the 2 that fit beside 128 x 64 channels' weights
+    return CB == 64 && BN == 128 ? 2 : 3;
+}
+// groups of four epilogue warps, a tile each in turn, with a staged tile each (one where the weights
+// leave no more room, or three CTAs share an SM)
+template <int CB, int BN> __host__ __device__ constexpr int conv_groups() {
+    return (CB == 64 && BN == 128) || conv_loaders<CB, BN>() > 32 ? 1 : 2;
+}
+template <int CB, int BN> __host__ __device__ constexpr int conv_threads() {
+    return 32 + conv_loaders<CB, BN>() + 128 * conv_groups<CB, BN>();
 }
 template <int CB, int BN> __host__ __device__ constexpr size_t conv_smem() {
-    return size_t(9) * CB * BN * 2 + size_t(conv_stages<CB, BN>()) * halo_stage<CB>() + conv_outs<CB, BN>() * out_bytes<BN>() + 1024;
+    return size_t(9) * CB * BN * 2 + size_t(conv_stages<CB, BN>()) * halo_stage<CB>() + conv_groups<CB, BN>() * out_bytes<BN>() + 1024;
 }
-
+// CTAs an SM holds
+template <int CB, int BN> __host__ __device__ constexpr int conv_ctas() {
+    return conv_smem<CB, BN>() * 3 <= 224 * 1024 ? 3 : conv_smem<CB, BN>() * 2 <= 224 * 1024 ? 2 : 1;
+}
 template <int CB, int BN>
-__global__ void __launch_bounds__(kPtThreads, 1)
-k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
-            const __grid_constant__ CUtensorMap tmY, int staged, int Co, void* y, int ldy, const float* __restrict__ bias,
-            int epi, int* err, const TileGeom g) {
-    constexpr int NS = conv_stages<CB, BN>(), NO = conv_outs<CB, BN>();
+__global__ void __launch_bounds__(conv_threads<CB, BN>(), conv_ctas<CB, BN>())
+k_conv_halo(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
+            int staged, int Co, void* y, int ldy, const float* __restrict__ bias, int epi, int* err, const TileGeom g) {
+    constexpr int NS = conv_stages<CB, BN>(), NG = conv_groups<CB, BN>(), kLoadWarps = conv_loaders<CB, BN>() / 32;
+    constexpr bool kCopy = kLoadWarps > 1;   // halo tiles by the warps' own copies, else by TMA
+    __shared__ __align__(16) float s_bias[BN];
     static_assert(NS >= 2, "a halo tile must load while another is used");
     constexpr uint32_t kW = CB * BN * 2;   // one tap's weights
     constexpr uint32_t kRow = CB * 2;
@@ -118,9 +184,10 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     const uint32_t sY = sX + uint32_t(NS) * halo_stage<CB>();
 
     if (warp == 0) tmem_alloc(smem_addr(&s_tmem), uint32_t(2 * BN));
+    load_bias(s_bias, BN, bias, Co, tid, conv_threads<CB, BN>());
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
-            mbar_init(smem_addr(&bar_full[s]), 1u);
+            mbar_init(smem_addr(&bar_full[s]), kCopy ? uint32_t(kLoaders) : 1u);
             mbar_init(smem_addr(&bar_empty[s]), 1u);
         }
         for (int b = 0; b < 2; ++b) {
@@ -138,10 +205,31 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     uint32_t issued = 0;
-    if (warp == 0) {
-        if (lane == 0) {
-            mbar_expect_tx(smem_addr(&bar_w), 9 * kW);
-            for (int tap = 0; tap < 9; ++tap) tma_load_2d(sW + tap * kW, &tmW, tap * CB, 0, smem_addr(&bar_w));
+    if (warp < kLoadWarps) {
+        if constexpr (kCopy) {
+            // NS - 1 tiles are on their way; a tile is handed over when its copies have landed
+            uint32_t it = 0;
+            const auto landed = [&](uint32_t i) {
+                fence_proxy_async_smem();
+                mbar_arrive(smem_addr(&bar_full[i % NS]));
+            };
+            for (int t = blockIdx.x; t < g.total && !pt_failed(fail); t += gridDim.x, ++it) {
+                int b, y0, x0;
+                g.at(t, b, y0, x0);
+                const int s = int(it % NS);
+                if (it >= uint32_t(NS - 1)) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
+                    landed(it - uint32_t(NS - 1));
+                }
+                if (it >= uint32_t(NS) && !bar_wait(smem_addr(&bar_empty[s]), ((it / NS) - 1u) & 1u)) {
+                    *fail = 1;
+                    break;
+                }
+                load_halo<CB>(x, g, b, y0, x0, sX + uint32_t(s) * halo_stage<CB>(), tid);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            for (uint32_t i = it >= uint32_t(NS - 1) ? it - uint32_t(NS - 1) : 0u; i < it; ++i) landed(i);
+        } else if (lane == 0) {
             for (int t = blockIdx.x; t < g.total && !pt_failed(fail); t += gridDim.x) {
                 int b, y0, x0;
                 g.at(t, b, y0, x0);
@@ -155,7 +243,12 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
                 ++issued;
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == kLoadWarps) {
+        if (lane == 0) {
+            mbar_expect_tx(smem_addr(&bar_w), 9 * kW);
+            for (int tap = 0; tap < 9; ++tap) tma_load_2d(sW + tap * kW, &tmW, tap * CB, 0, smem_addr(&bar_w));
+        }
+        __syncwarp();
         constexpr uint32_t idesc = bf16_idesc<BN>();
         uint32_t it = 0;
         bool ok = bar_wait_warp(smem_addr(&bar_w), 0u);
@@ -183,11 +276,16 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
         if (!bar_wait_warp(smem_addr(&bar_done), 0u)) *fail = 1;
     } else {
         const int q = warp & 3;   // TMEM lanes 32q .. 32q + 31 = pixels of the tile
+        constexpr int kFirst = 1 + kLoadWarps;   // the first epilogue warp
+        const int grp = NG == 2 ? (warp - kFirst) >> 2 : 0;   // its tiles: every NG-th of the CTA's
+        const uint32_t tile = sY + uint32_t(grp) * out_bytes<BN>();
+        const int e = (warp - kFirst - 4 * grp) * 32 + lane;
         uint32_t it = 0;
         for (int t = blockIdx.x; t < g.total; t += gridDim.x, ++it) {
             const int b = int(it & 1u);
+            if (NG == 2 && b != grp) continue;
             const bool ready = !pt_failed(fail) && bar_wait(smem_addr(&acc_full[b]), (it >> 1) & 1u);
-            if (epi_any<2, 128>(!ready)) {   // the four warps leave together (they meet at barriers below)
+            if (grp == 0 ? epi_any<1, 128>(!ready) : epi_any<2, 128>(!ready)) {   // a group leaves together
                 *fail = 1;
                 break;
             }
@@ -195,27 +293,18 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
             int img, y0, x0;
             g.at(t, img, y0, x0);
             const int m = q * 32 + lane;
-            if (staged) {
-                const uint32_t tile = sY + (NO == 2 ? (it & 1u) : 0u) * out_bytes<BN>();
-                // the store that used this tile has read it (thread 64 issues the stores)
-                if (tid == 64) store_wait_read<NO - 1>();
-                epi_sync<1, 128>();
+            if (staged) {   // (the group has written its tile before out: the barrier above)
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 32) {
                     float v[32];
                     tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(b * BN + c0), v);
-                    stage_row32<BN>(v, c0, Co, bias, epi == EPI_BF16_BIAS_RELU, tile, m);
+                    stage_row32<BN>(v, c0, s_bias, epi == EPI_BF16_BIAS_RELU, tile, m);
                 }
                 tc_fence_before();
                 mbar_arrive(smem_addr(&acc_empty[b]));
-                fence_proxy_async_smem();
-                epi_sync<1, 128>();
-                if (tid == 64) {
-                    constexpr int OB = out_box<BN>();
-                    for (int c0 = 0; c0 < BN && c0 < Co; c0 += OB)
-                        tma_store_4d(&tmY, tile + uint32_t(c0 / OB) * uint32_t(kBM * OB * 2), c0, x0, y0, img);
-                    store_commit();
-                }
+                if (grp == 0) epi_sync<3, 128>();
+                else epi_sync<4, 128>();
+                write_tile<BN>(tile, g, img, y0, x0, Co, static_cast<uint16_t*>(y), ldy, e);
             } else {
                 const int row = g.row(img, y0, x0, m);
 #pragma unroll 1
@@ -228,7 +317,6 @@ k_conv_halo(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
                 mbar_arrive(smem_addr(&acc_empty[b]));
             }
         }
-        if (staged && tid == 64) store_wait<0>();
     }
     __syncwarp();
     tc_fence_before();
@@ -295,9 +383,9 @@ __device__ __forceinline__ void gather_row(const uint16_t* __restrict__ x, const
 // The im2col matrix this replaces was written to and read from HBM (128 bytes a pixel each way).
 template <int C, int BN>
 __global__ void __launch_bounds__(128)
-k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmY,
-             int staged, int Co, void* y, int ldy, const float* __restrict__ bias, int epi, int* err, const TileGeom g) {
+k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap tmW, int staged, int Co, void* y, int ldy, const float* __restrict__ bias, int epi, int* err, const TileGeom g) {
     constexpr uint32_t kA = kBM * 128u, kB = BN * 128u;
+    __shared__ __align__(16) float s_bias[BN];
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) unsigned long long bar_w, bar_acc;
     __shared__ uint32_t s_tmem;
@@ -306,6 +394,7 @@ k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t sA = base, sB = base + kA, sY = sB + kB;
     if (warp == 0) tmem_alloc(smem_addr(&s_tmem), uint32_t(BN));
+    load_bias(s_bias, BN, bias, Co, tid, 128);
     if (tid == 0) {
         mbar_init(smem_addr(&bar_w), 1u);
         mbar_init(smem_addr(&bar_acc), 1u);
@@ -341,22 +430,14 @@ k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap
         if (!ok) atomicExch(&s_fail, 1);
         tc_fence_after();
         if (staged) {
-            if (tid == 0) store_wait_read<0>();
-            __syncthreads();
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 float v[32];
                 tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0), v);
-                stage_row32<BN>(v, c0, Co, bias, epi == EPI_BF16_BIAS_RELU, sY, tid);
+                stage_row32<BN>(v, c0, s_bias, epi == EPI_BF16_BIAS_RELU, sY, tid);
             }
-            fence_proxy_async_smem();
-            __syncthreads();
-            if (tid == 0 && ok) {
-                constexpr int OB = out_box<BN>();
-                for (int c0 = 0; c0 < BN && c0 < Co; c0 += OB)
-                    tma_store_4d(&tmY, sY + uint32_t(c0 / OB) * uint32_t(kBM * OB * 2), c0, x0, y0, b);
-                store_commit();
-            }
+            __syncthreads();   // (the next tile is staged after the barrier that follows its gather)
+            if (ok) write_tile<BN>(sY, g, b, y0, x0, Co, static_cast<uint16_t*>(y), ldy, tid);
         } else {
             const int row = g.row(b, y0, x0, tid);
 #pragma unroll 1
@@ -367,7 +448,6 @@ k_conv_small(const uint16_t* __restrict__ x, const __grid_constant__ CUtensorMap
             }
         }
     }
-    if (staged && tid == 0) store_wait<0>();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
