@@ -850,15 +850,19 @@ __device__ __forceinline__ R face_momentum(bool wet, R Hf, R S, R qp, R n2c, con
 
 // ---------------- the fused steps' form of the same arithmetic -------------------------------
 // The wet path is bound by instruction issue, so these leave out what cannot change a result of the
-// fused kernels: the depths that enter are >= 0 (or NaN, next to closed faces only); a face's value
-// is selected once, at the end; closed faces and depths below the smallest normal number, rare, are
-// left to branches that whole warps skip.  Every face and cell gets the bits of face_flux,
+// fused kernels: the depths that enter are >= 0 (or NaN, next to closed faces only); whether a face is
+// open and wet needs no flag of its own (face_open, face_update); the grid's edges and face depths
+// below the smallest normal number are left to branches that whole warps skip.  The latter need the
+// depths' clamp to be off: between depths that are 0 or at least 1e-9, a positive face depth is a
+// difference of numbers that size, at least their last place.  Every face and cell gets the bits of face_flux,
 // donor_scale, limit_face and cfl_cell (up to the sign of a zero).
 //
-// face_open: the face depth and slope of an open face; returns whether it is open (a closed one's
-// depth comes from face_closed).
+// face_open: the face depth and slope of a face whose dz is finite or NaN.  A NaN dz (next to an idx_nan
+// cell) takes part in no minimum or maximum, which leaves the inside cell's depth, as the closed face has
+// it; its NaN slope makes the momentum update 0.  Faces closed by an infinite dz (the grid's edges) get
+// depth 0 from their callers, and with it flux 0.
 template <typename R, bool IS_X>
-__device__ __forceinline__ bool face_open(R ha, R hb, R dz, R& Hf, R& S, const StepConsts<R>& K) {
+__device__ __forceinline__ void face_open(R ha, R hb, R dz, R& Hf, R& S, const StepConsts<R>& K) {
     const R up = fmax(dz, R(0)), dn = fmin(dz, R(0));
     if (IS_X) {
         Hf = fmax(fmax(ha - up, hb + dn), R(0));
@@ -867,11 +871,8 @@ __device__ __forceinline__ bool face_open(R ha, R hb, R dz, R& Hf, R& S, const S
         Hf = fmax(fmax(ha + dn, hb - up), R(0));
         S = (dz + (ha - hb)) * K.inv_dx;
     }
-    return fabs(dz) <= R(3.0e38);
 }
-template <typename R> __device__ __forceinline__ R face_closed(R ha, R hb, R dz) {
-    return isnan(dz) ? fmax(fmax(ha, hb), R(0)) : R(0);
-}
+template <typename R> __device__ __forceinline__ bool face_edge(R dz) { return fabs(dz) > R(3.0e38); }
 // x^(7/3) of a normal positive number
 template <typename R> __device__ __forceinline__ R pow73_normal(R x) {
     R r = bits_seed(x);
@@ -888,16 +889,17 @@ template <typename R> __device__ __forceinline__ R pow73_normal(R x) {
 template <typename R> __device__ __noinline__ R pow73_any(R x) { return pow73_pos(x); }
 __device__ __forceinline__ bool finite_abs(float x) { return fabsf(x) <= 3.402823466e+38f; }
 __device__ __forceinline__ bool finite_abs(double x) { return fabs(x) <= 1.7976931348623157e+308; }
-// the momentum update of a face; what is not wet gets 0 (its operands may be anything)
+// the momentum update of a face.  One of depth 0 gets 0 whatever the rest: a finite quotient is cut
+// to +-10 H = 0 and any other becomes 0.
 template <typename R, int SCH = 0>
-__device__ __forceinline__ R face_update(bool wet, R H, R h73, R S, R qp, R n2c, const StepConsts<R>& K,
-                                         int flag_critical, int scheme = 1, R q_lo = R(0), R q_hi = R(0)) {
+__device__ __forceinline__ R face_update(R H, R h73, R S, R qp, R n2c, const StepConsts<R>& K, int flag_critical,
+                                         int scheme = 1, R q_lo = R(0), R q_hi = R(0)) {
     R qn = qp;
     if (SCH) qn = diffused_momentum(qp, q_lo, q_hi, H, K, scheme);
     const R num = fma(-(K.gdt * H), S, qn);
     const R den = fma(K.gdt * n2c, fabs(qp), h73);
     R qq = qdiv(num * h73, den);
-    const bool ok = wet && finite_abs(qq);
+    const bool ok = finite_abs(qq);
     if (flag_critical == 1) {
         const R crit = H * sqrt(K.g * H);
         qq = fmin(fmax(qq, -crit), crit);

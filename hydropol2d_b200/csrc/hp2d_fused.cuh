@@ -1,10 +1,11 @@
 // Fused surface-flow step: one launch = one accepted step of HydroPol2D_Main_While.m
 // :403-782 (rain + Green-Ampt + clamp, local-inertial fluxes, draining limiter,
 // continuity, outlet sink, running maximum / arrival time, CFL reductions, and the
-// timestep refresh + clock advance done by the last CTA to finish).
+// timestep refresh + clock advance, done by the next launch of a grid and by the last CTA to
+// finish an ensemble member).
 //
 // Warp-streaming layout.  Each warp owns a strip of 32*CPL columns (CPL = 1 or 2 cells per
-// lane; cell h of lane L sits at column 32h + L), of which all but two columns on each side
+// lane; cell h of lane L sits at column CPL L + h), of which all but two columns on each side
 // are its output, and walks down a block of rows.  The draining limiter makes a cell's new
 // depth depend on cells two away (face <- donor scale <- donor's four faces <- their far
 // cells); in x those neighbours come from other lanes by warp shuffles (hence the
@@ -57,6 +58,12 @@ constexpr int kRowUnroll = HP2D_ROW_UNROLL;   // row-loop unroll (register renam
 // instead), so that the CPL cells interleave: wet 2048^2 41.6 vs 40.8 GCUPS, 60-minute dam-break
 // 115.5 vs 111.8, 128-member ensemble 44.6 vs 43.0; the Green-Ampt + rain-map instantiation ran
 // 20.3 vs 21.2 with it and keeps the branch.
+// What a row of wet cells costs is its instructions (64 % of the issue slots, DRAM at 40 %), so what
+// only some rows need is decided once per row by a vote: the grid's edges, outlet and gauge cells,
+// arrivals, dry flags.  A lane's two cells are neighbours (one shuffle an exchange), columns and rows
+// outside the grid are records whose faces are closed, and no face carries a flag (wet 2048^2: 64.8 M
+// to 53.9 M warp instructions, 94 to 77 us a step; 4096 x 8192 valley 45.0 to 39.0 ms; 48 members 23.3
+// to 19.4 ms; urban 2048^2 15.0 to 14.4 ms).
 template <int INF, bool MAP> constexpr bool kFlatF = INF == 0 && !MAP;
 
 // dynamic shared memory of k_fused_step: per warp kStages x (2 records x 32*CPL cells)
@@ -179,25 +186,16 @@ template <> __device__ __forceinline__ float bits_to<float>(unsigned long long b
 template <> __device__ __forceinline__ double bits_to<double>(unsigned long long b) { return __longlong_as_double((long long)b); }
 
 // Neighbour exchange across a warp's strip of 32*CPL columns (cell h of lane L sits at
-// column 32h + L): value of the cell to the right / to the left.  With two cells per lane
-// one indexed shuffle carries the value across the boundary between the two halves.
+// column CPL L + h): value of the cell to the right / to the left, one shuffle each.
 template <typename R, int CPL>
 __device__ __forceinline__ void right_of(const R (&v)[CPL], R (&out)[CPL], int lane) {
-    if (CPL == 1) {
-        out[0] = __shfl_down_sync(0xffffffffu, v[0], 1);
-    } else {
-        out[0] = __shfl_sync(0xffffffffu, lane == 0 ? v[CPL - 1] : v[0], (lane + 1) & 31);
-        out[CPL - 1] = __shfl_down_sync(0xffffffffu, v[CPL - 1], 1);
-    }
+    out[CPL - 1] = __shfl_down_sync(0xffffffffu, v[0], 1);
+    if (CPL == 2) out[0] = v[CPL - 1];
 }
 template <typename R, int CPL>
 __device__ __forceinline__ void left_of(const R (&v)[CPL], R (&out)[CPL], int lane) {
-    if (CPL == 1) {
-        out[0] = __shfl_up_sync(0xffffffffu, v[0], 1);
-    } else {
-        out[CPL - 1] = __shfl_sync(0xffffffffu, lane == 31 ? v[0] : v[CPL - 1], (lane + 31) & 31);
-        out[0] = __shfl_up_sync(0xffffffffu, v[0], 1);
-    }
+    out[0] = __shfl_up_sync(0xffffffffu, v[CPL - 1], 1);
+    if (CPL == 2) out[CPL - 1] = v[0];
 }
 
 // resident CTAs per SM the register budget is sized for (float: 8 x 128 threads)
@@ -743,6 +741,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
     Kahan<R> rain_acc_r, inf_acc_r, out_acc_r;
     unsigned nbad = 0u;                       // own cells ending non-finite or below -tol
     unsigned dry = 0u;                        // bit i: row r-i dry across the strip
+    unsigned marks = 0u;
     R s2max = R(0);
     R cmaxv = R(-1);   // largest celerity term of a non-stagnant cell (-1: none yet)
 
@@ -755,10 +754,11 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
         bool col_ok[CPL], own_lane[CPL];
 #pragma unroll
         for (int h = 0; h < CPL; ++h) {
-            j[h] = j_first + 32 * h + lane;
+            j[h] = j_first + CPL * lane + h;
             col_ok[h] = j[h] >= 0 && j[h] < nx;
-            own_lane[h] = (h > 0 || lane >= 2) && (h < CPL - 1 || lane < 30) && j[h] < nx;
+            own_lane[h] = lane >= 2 / CPL && lane < 32 - 2 / CPL && j[h] < nx;
         }
+        const R rc_half = j[0] == 0 ? R(0.5) : R(1);   // refreshing_timestep.m's vel_left on the first column
         const int r0 = rb * a.rows_per_warp;
         const int r_end = min(r0 + a.rows_per_warp, ny);
         unsigned char* const dfl =
@@ -770,11 +770,13 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
         // lane (read once: each row's output flag changes only at that row, the input flags not
         // at all during the step)
         unsigned dfw = 0u, dfw_in = 0u;
+        bool flagged = false;   // some row of the block is flagged in either buffer
         if (dfl && r0 + 4 * lane < r_end) {
             dfw = *reinterpret_cast<const unsigned*>(dfl + r0 + 4 * lane);
             dfw_in = *reinterpret_cast<const unsigned*>(a.dryflag + (size_t(cur) * a.n_strips + strip) * size_t(a.dry_rows) +
                                                         r0 + 4 * lane);
         }
+        flagged = __any_sync(FULL, (dfw | dfw_in) != 0u);
         // The whole block of rows: when this step adds no rain and no infiltration and records
         // no map, and the flags show every input row r0-1..r_end+1 of this strip and of its
         // neighbours (the 2-column aprons) deep-dry and every output row already holding the
@@ -868,6 +870,17 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
             for (int s = 0; s < kStages; ++s) mbar_init(bar0 + 8u * s, 1u);
             mbar_fence_init();
         }
+        // the ring's columns outside the grid, which no copy reaches: cells that stay dry whatever the
+        // rain, their faces closed, that enter no maximum
+        const R inf = R(__int_as_float(0x7f800000));
+        const V4 pad_S{inf, inf, R(1), make_meta<R>(255u)}, pad_X{R(-3.0e38), R(0), R(0), inf};
+#pragma unroll
+        for (int h = 0; h < CPL; ++h)
+            if (!col_ok[h])
+                for (int s = 0; s < kStages; ++s) {
+                    ring[s * 2 * SW + CPL * lane + h] = pad_S;
+                    ring[s * 2 * SW + SW + CPL * lane + h] = pad_X;
+                }
         __syncwarp();
         if (lane < 2) {
             fence_proxy_async_smem();   // reads of the ring by an earlier item come first
@@ -879,9 +892,12 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
             const int s = k % kStages;
             // the dry flag of the output row r-2 in the buffer this step writes
             const bool frow_f = r - 2 >= r0 && r - 2 < r_end;
-            const int fri = frow_f ? r - 2 - r0 : 0;
-            const unsigned flg = frow_f ? (__shfl_sync(FULL, dfw, fri >> 2) >> (8 * (fri & 3))) & 255u : 0u;
-            const unsigned flg_in = frow_f ? (__shfl_sync(FULL, dfw_in, fri >> 2) >> (8 * (fri & 3))) & 255u : 0u;
+            unsigned flg = 0u, flg_in = 0u;
+            if (flagged && frow_f) {
+                const int fri = r - 2 - r0;
+                flg = (__shfl_sync(FULL, dfw, fri >> 2) >> (8 * (fri & 3))) & 255u;
+                flg_in = (__shfl_sync(FULL, dfw_in, fri >> 2) >> (8 * (fri & 3))) & 255u;
+            }
             const bool landed = mbar_wait_bounded(bar0 + 8u * s, uint32_t((k / kStages) & 1), a.wait_polls);
             if (__any_sync(FULL, !landed)) {   // the whole warp leaves the loop together
                 timed_out = true;
@@ -894,8 +910,8 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
             V4 S[CPL], X[CPL];
 #pragma unroll
             for (int h = 0; h < CPL; ++h) {
-                S[h] = ring[s * 2 * SW + 32 * h + lane];
-                X[h] = ring[s * 2 * SW + SW + 32 * h + lane];
+                S[h] = ring[s * 2 * SW + CPL * lane + h];
+                X[h] = ring[s * 2 * SW + SW + CPL * lane + h];
             }
             __syncwarp();
             if (lane < 2 && k + kStages <= last_k) {
@@ -904,9 +920,16 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
             }
             const bool rok = r >= 0 && r < ny;
             const bool own_row = r >= r0 && r < r_end;
+            if (!rok) {   // a row outside the grid, which no copy brings
+#pragma unroll
+                for (int h = 0; h < CPL; ++h) {
+                    S[h] = pad_S;
+                    X[h] = pad_X;
+                }
+            }
             R hT0[CPL];
             unsigned meta[CPL];
-            bool all_dry = true;
+            bool all_dry = true, marked = false;
             // rain maps: the rows of the map around this row, and per lane their interpolation at its
             // columns, made anew only when those rows change (every ny / my rows) and kept in shared
             // memory (urban 2048^2 with 64 x 64 maps: four gathers and 30 instructions less per cell)
@@ -937,13 +960,15 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                 // soil records: the row after next is brought to L1 (a register prefetch spilled)
                 if (INF && col_ok[h] && r + 2 >= 0 && r + 2 < ny) prefetch_l1(gin + (size_t(r + 2) * nx + j[h]));
                 meta[h] = meta_bits(S[h].w);
+                marked = marked || (meta[h] >> 8) != 0u;
                 // (A) hydrology of (r, j)
                 hT0[h] = R(0);
-                if (col_ok[h] && rok) {
+                if constexpr (kFlatF<INF, MAP> && !INFL) {
+                    const R hh = X[h].x + RS.depth;
+                    hT0[h] = hh < clamp0 ? R(0) : hh;
+                } else if (col_ok[h] && rok) {
                     const size_t c = size_t(r) * nx + j[h];
                     R hh = X[h].x;
-                    // a pending map record keeps the depth this step starts from
-                    if (s_rec >= 0 && own_lane[h] && own_row) a.rec.snap[size_t(s_rec) * (size_t(ny) * nx) + c] = hh;
                     const R rr = MAP ? rain_row(h) : RS.depth;
                     hh = hh + rr;
                     const bool own = own_lane[h] && own_row && r >= a.own_r0 && r < a.own_r1;
@@ -970,6 +995,14 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                 }
                 all_dry = all_dry && hT0[h] == R(0);
             }
+            // a pending map record keeps the depth this step starts from
+            if (s_rec >= 0 && own_row) {
+#pragma unroll
+                for (int h = 0; h < CPL; ++h)
+                    if (own_lane[h]) a.rec.snap[size_t(s_rec) * (size_t(ny) * nx) + size_t(r) * nx + j[h]] = X[h].x;
+            }
+            // bit i: row r-i has an outlet, inflow, stage or structure cell
+            marks = (marks << 1) | (__any_sync(FULL, marked) ? 1u : 0u);
             // rows r-2..r dry across the whole strip: every face flux of row r and r-1 is
             // zero (Hf = 0), the donor scale of row r-1 is one and its limited faces are
             // zero, so (B)-(E) are skipped; the values below are what they would compute
@@ -984,10 +1017,7 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
             // only by a non-quiet (F), and the (F) after a deep-dry row is quiet.)  A depth
             // of +0 reaches the arrival threshold only when that is not positive.
             if ((dry & 15u) == 15u && K.thr > R(0)) {
-                bool plain = true;
-#pragma unroll
-                for (int h = 0; h < CPL; ++h) plain = plain && (mt2[h] >> 8) == 0u;
-                if (__all_sync(FULL, plain)) {
+                if (!(marks & 4u)) {
                     const int rm2 = r - 2;
                     if (frow_f && flg && flg_in) {
                         // this buffer already holds the row as this step would write it: the
@@ -1049,57 +1079,50 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                 // (B) and (C) interleaved: the geometry of the 2 x CPL faces, then -- unless no
                 // lane of the warp has a wet one -- their momentum updates without branches
                 R Sx[CPL], Sy[CPL], ya[CPL], yb[CPL];
-                bool wx[CPL], wy[CPL];
-                bool any_wet = false, any_rare = false, any_out = false;
+                R hmax = R(0);
+                bool edge = false;
 #pragma unroll
                 for (int h = 0; h < CPL; ++h) {
-                    wx[h] = face_open<R, true>(hT0[h], hR[h], S[h].x, hfx0[h], Sx[h], K);
-                    wy[h] = face_open<R, false>(hT1[h], hT0[h], S[h].y, hfy0[h], Sy[h], K);
-                    any_out = any_out || !(wx[h] && wy[h] && col_ok[h]);
+                    face_open<R, true>(hT0[h], hR[h], S[h].x, hfx0[h], Sx[h], K);
+                    face_open<R, false>(hT1[h], hT0[h], S[h].y, hfy0[h], Sy[h], K);
+                    edge = edge || face_edge(fmax(fabs(S[h].x), fabs(S[h].y)));
                 }
-                if (__any_sync(FULL, any_out) || !rok || r < r0 - 1) {   // the grid's edges and idx_nan cells
+                if (__any_sync(FULL, edge)) {
 #pragma unroll
                     for (int h = 0; h < CPL; ++h) {
-                        const bool inx = col_ok[h] && rok;
-                        const bool iny = inx && r >= r0 - 1;
-                        hfx0[h] = !inx ? R(0) : wx[h] ? hfx0[h] : face_closed(hT0[h], hR[h], S[h].x);
-                        hfy0[h] = !iny ? R(0) : wy[h] ? hfy0[h] : face_closed(hT1[h], hT0[h], S[h].y);
-                        wx[h] = wx[h] && inx;
-                        wy[h] = wy[h] && iny;
+                        if (face_edge(S[h].x)) hfx0[h] = R(0);
+                        if (face_edge(S[h].y)) hfy0[h] = R(0);
                     }
                 }
 #pragma unroll
                 for (int h = 0; h < CPL; ++h) {
-                    wx[h] = wx[h] && hfx0[h] > R(0);
-                    wy[h] = wy[h] && hfy0[h] > R(0);
-                    any_wet = any_wet || wx[h] || wy[h];
-                    any_rare = any_rare || (wx[h] && below_normal(hfx0[h])) || (wy[h] && below_normal(hfy0[h]));
+                    hmax = fmax(hmax, fmax(hfx0[h], hfy0[h]));
                     ya[h] = yb[h] = R(0);
                     // schemes 2/3: the previous q_y of rows r-1 (kept from the row before) and r+1
-                    if (SCH && wy[h] && r >= 1 && r + 1 < ny) {
+                    if (SCH && col_ok[h] && r >= 1 && r + 1 < ny) {
                         ya[h] = qyp1[h];
                         yb[h] = sin[size_t(r + 1) * nx + j[h]].z;
                     }
                 }
-                if (__any_sync(FULL, any_wet)) {
+                if (__any_sync(FULL, hmax > R(0))) {
                     R px[CPL], py[CPL];   // H^(7/3)
 #pragma unroll
                     for (int h = 0; h < CPL; ++h) {
                         px[h] = pow73_normal(hfx0[h]);
                         py[h] = pow73_normal(hfy0[h]);
                     }
-                    if (__any_sync(FULL, any_rare)) {
+                    if (sh.now.skip) {   // no clamp: depths of any size
 #pragma unroll
                         for (int h = 0; h < CPL; ++h) {
-                            if (wx[h] && below_normal(hfx0[h])) px[h] = pow73_any(hfx0[h]);
-                            if (wy[h] && below_normal(hfy0[h])) py[h] = pow73_any(hfy0[h]);
+                            if (hfx0[h] > R(0) && below_normal(hfx0[h])) px[h] = pow73_any(hfx0[h]);
+                            if (hfy0[h] > R(0) && below_normal(hfy0[h])) py[h] = pow73_any(hfy0[h]);
                         }
                     }
 #pragma unroll
                     for (int h = 0; h < CPL; ++h) {
-                        qxu0[h] = face_update<R, SCH>(wx[h], hfx0[h], px[h], Sx[h], X[h].y, S[h].z, K, a.flag_critical,
+                        qxu0[h] = face_update<R, SCH>(hfx0[h], px[h], Sx[h], X[h].y, S[h].z, K, a.flag_critical,
                                                        a.scheme, SCH ? qxa[h] : R(0), SCH ? qxb[h] : R(0));
-                        qyu0[h] = face_update<R, SCH>(wy[h], hfy0[h], py[h], Sy[h], X[h].z, S[h].z, K, a.flag_critical,
+                        qyu0[h] = face_update<R, SCH>(hfy0[h], py[h], Sy[h], X[h].z, S[h].z, K, a.flag_critical,
                                                        a.scheme, ya[h], yb[h]);
                     }
                 }
@@ -1111,14 +1134,14 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
 #pragma unroll
                 for (int h = 0; h < CPL; ++h) {
                     out[h] = donor_out(qxu1[h], qxu1_left[h], qyu1[h], qyu0[h]);
-                    lim = lim || (col_ok[h] && out[h] > hT1[h] * K.dx_over_dt);
+                    lim = lim || out[h] > hT1[h] * K.dx_over_dt;
                 }
                 lim1 = drow && __any_sync(FULL, lim);
                 if (lim1) {
 #pragma unroll
                     for (int h = 0; h < CPL; ++h) {
                         const R avail = hT1[h] * K.dx_over_dt;
-                        if (col_ok[h] && out[h] > avail) sc1[h] = avail / out[h];
+                        if (out[h] > avail) sc1[h] = avail / out[h];
                     }
                 }
                 // (E) limited faces of row r-1
@@ -1157,105 +1180,134 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                 // are computed and dropped: `act` masks every store and every reduction), so that the
                 // compiler can interleave the CPL cells' arithmetic; frow is the same for the warp.
                 if (frow) {
-                    R hn_[CPL], hf3_[CPL];
-    #pragma unroll
+                    R hn[CPL], hf3[CPL];
+                    const bool marked2 = (marks & 4u) != 0u;   // the rare cells of row r-2
+#pragma unroll
                     for (int h = 0; h < CPL; ++h) {
-                        const bool act = own_lane[h];
-                        const size_t c2 = size_t(rm2) * nx + j[h];
-                        // a control structure's transfers join the depth after the fluxes
-                        // (Local_Inertial_Model_D4.m:318-344, :390)
                         R h_in = hT2[h];
-                        if (INFL && act && (mt2[h] & kInflowBit)) {
-                            const int ss = a.inflow.cell_struct[(mt2[h] >> 8) & 0x7FFFFFu];
-                            if (ss >= 0) h_in = h_in + a.strct.extra[ss];
-                        }
-                        R hn = quiet ? h_in + R(0) : continuity(h_in, qxl2_left[h], qxl2[h], qyl2[h], qyl1[h], K);
-                        const R negtol = -K.tol;
-                        R hf3 = R(0);
-                        const unsigned ord = INFL ? outlet_ord(mt2[h]) : mt2[h] >> 8;
-                        if (act && ord) {
-                            const int o = int(ord) - 1;
-                            R ho;
-                            const R qq = outlet_sink(hn, a.outlet_coef[o], a.outlet_type, K, ho);
-                            hf3 = ho;
-                            a.hf3[o] = ho;
-                            a.qo[o] = qq;
-                            if (mine) out_acc_r.add(qq * K.dt);
-                            // the next step's clamp is skipped when an outlet cell (outside the
-                            // infiltrating soils) stays negative after the next rain
-                            // (Hydrological_Model.m:45-50); only outlet cells can end negative
-                            if (mine && !(a.ga && (mt2[h] & 255u) != 255u) &&
-                                hn + (MAP ? rain_at_cell(a, s_rsn, rm2, j[h]) : s_rsn.depth) < R(-1e-11))
-                                s_negn = 1;   // rare: kept in shared memory, not a register
-                        }
-                        // stage hydrograph: the cell's depth becomes the gauge's stage
-                        // (update_spatial_BC.m:332-341, after the step's refreshing_timestep)
-                        if (INFL && act && (mt2[h] & kInflowBit)) {
-                            const int sg = a.inflow.cell_stage[(mt2[h] >> 8) & 0x7FFFFFu];
-                            if (sg >= 0) {
-                                const R sv = a.inflow.stage_now[sg];
-                                atomicAdd(&s_stage, double(sv) - double(hn));
-                                hn = sv;
+                        if (INFL && marked2) {
+                            // a control structure's transfers join the depth after the fluxes
+                            // (Local_Inertial_Model_D4.m:318-344, :390)
+                            if (own_lane[h] && (mt2[h] & kInflowBit)) {
+                                const int ss = a.inflow.cell_struct[(mt2[h] >> 8) & 0x7FFFFFu];
+                                if (ss >= 0) h_in = h_in + a.strct.extra[ss];
                             }
                         }
+                        hn[h] = INFL && quiet ? h_in + R(0) : continuity(h_in, qxl2_left[h], qxl2[h], qyl2[h], qyl1[h], K);
+                        hf3[h] = R(0);
+                    }
+                    if (marked2) {
+#pragma unroll
+                        for (int h = 0; h < CPL; ++h) {
+                            const unsigned ord = INFL ? outlet_ord(mt2[h]) : mt2[h] >> 8;
+                            if (own_lane[h] && ord) {
+                                const int o = int(ord) - 1;
+                                R ho;
+                                const R qq = outlet_sink(hn[h], a.outlet_coef[o], a.outlet_type, K, ho);
+                                hf3[h] = ho;
+                                a.hf3[o] = ho;
+                                a.qo[o] = qq;
+                                if (mine) out_acc_r.add(qq * K.dt);
+                                // the next step's clamp is skipped when an outlet cell (outside the
+                                // infiltrating soils) stays negative after the next rain
+                                // (Hydrological_Model.m:45-50); only outlet cells can end negative
+                                if (mine && !(a.ga && (mt2[h] & 255u) != 255u) && hn[h] + s_rsn.depth < R(-1e-11))
+                                    s_negn = 1;   // rare: kept in shared memory, not a register
+                            }
+                            // stage hydrograph: the cell's depth becomes the gauge's stage
+                            // (update_spatial_BC.m:332-341, after the step's refreshing_timestep)
+                            if (INFL && own_lane[h] && (mt2[h] & kInflowBit)) {
+                                const int sg = a.inflow.cell_stage[(mt2[h] >> 8) & 0x7FFFFFu];
+                                if (sg >= 0) {
+                                    const R sv = a.inflow.stage_now[sg];
+                                    atomicAdd(&s_stage, double(sv) - double(hn[h]));
+                                    hn[h] = sv;
+                                }
+                            }
+                        }
+                    }
+                    // arrival times, where a depth passes the threshold for the first time
+                    bool arrived = false;
+#pragma unroll
+                    for (int h = 0; h < CPL; ++h) arrived = arrived || (dm2[h] < K.thr && hn[h] >= K.thr);
+                    if (__any_sync(FULL, arrived)) {
+#pragma unroll
+                        for (int h = 0; h < CPL; ++h)
+                            if (own_lane[h] && dm2[h] < K.thr && hn[h] >= K.thr) a.arrival[size_t(rm2) * nx + j[h]] = t_arr;
+                    }
+                    R vras[CPL];   // velocity raster: largest |face velocity| (refreshing_timestep.m:109-111)
+#pragma unroll
+                    for (int h = 0; h < CPL; ++h) vras[h] = R(0);
+                    if (mine) {
                         // a non-finite depth (NaN walls included, counted against the run's start)
                         // or one below -depth_tolerance
-                        nbad += (hn >= negtol || !mine || !act) ? 0u : 1u;
-                        if (act && dm2[h] < K.thr && hn >= K.thr) a.arrival[c2] = t_arr;
-                        hn_[h] = hn;
-                        hf3_[h] = hf3;
+#pragma unroll
+                        for (int h = 0; h < CPL; ++h)
+                            if (!(hn[h] >= -K.tol) && own_lane[h]) ++nbad;
                     }
-                    // refreshing_timestep.m:61-89, :139-150, :181-238 for these cells
-                    R vras[CPL];   // velocity raster: largest |face velocity| (refreshing_timestep.m:109-111)
-    #pragma unroll
-                    for (int h = 0; h < CPL; ++h) vras[h] = R(0);
-                    if (!quiet && mine) {
-    #pragma unroll
+                    // refreshing_timestep.m:61-89, :139-150, :181-238 for these cells; an apron lane's
+                    // values are computed and dropped, so that the CPL cells interleave
+                    if (mine && !quiet) {
+                        R vr[CPL], vu[CPL], s2[CPL], dts[CPL];
+#pragma unroll
+                        for (int h = 0; h < CPL; ++h) vr[h] = face_velocity(qxl2[h], hfx2[h], K);
+                        if (vcar_ok) {
+#pragma unroll
+                            for (int h = 0; h < CPL; ++h) vu[h] = vcar[h];
+                        } else {
+#pragma unroll
+                            for (int h = 0; h < CPL; ++h) vu[h] = face_velocity(qyl2[h], hfy2[h], K);
+                        }
+#pragma unroll
                         for (int h = 0; h < CPL; ++h) {
-                            const bool act = own_lane[h];
-                            const R vr = face_velocity(qxl2[h], hfx2[h], K);
-                            R vu;
-                            if (vcar_ok) vu = vcar[h];
-                            else vu = face_velocity(qyl2[h], hfy2[h], K);
                             const R vb = face_velocity(qyl1[h], hfy1[h], K);
                             vcar[h] = vb;
-                            if (INFL) vras[h] = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb));
-                            const R rc = vr * (j[h] == 0 ? R(0.5) : R(1));
-                            const R uc = R(0.5) * (vu + vb);
-                            const R s2 = rc * rc + uc * uc;
-                            if (act) s2max = fmax(s2max, s2);
+                            if (INFL) vras[h] = fmax(fmax(fabs(vr[h]), fabs(vu[h])), fabs(vb));
+                            const R rc = h == 0 ? vr[h] * rc_half : vr[h];
+                            const R uc = R(0.5) * (vu[h] + vb);
+                            s2[h] = rc * rc + uc * uc;
                             // the largest depth of a moving cell; its celerity is taken at the end (the
                             // product by g is monotone)
-                            R dts = fmax(fmax(hfx2[h], hfy2[h]), hf3_[h]);
-                            if (a.adaptive != 1) {
-                                const R wc = fmax(sqrt(K.g * fmax(dts, R(0))), R(1e-10));
-                                dts = fmax(fmax(fabs(vr), fabs(vu)), fabs(vb)) + wc;
+                            dts[h] = fmax(fmax(hfx2[h], hfy2[h]), hf3[h]);
+                        }
+                        if (a.adaptive != 1) {
+#pragma unroll
+                            for (int h = 0; h < CPL; ++h) {
+                                const R wc = fmax(sqrt(K.g * fmax(dts[h], R(0))), R(1e-10));
+                                dts[h] = fmax(fmax(fabs(vr[h]), fabs(vu[h])), fabs(vcar[h])) + wc;
                             }
-                            if (act && s2 >= a.stag_s2) cmaxv = fmax(cmaxv, dts);
+                        }
+#pragma unroll
+                        for (int h = 0; h < CPL; ++h) {
+                            if (own_lane[h]) s2max = fmax(s2max, s2[h]);
+                            if (own_lane[h] && s2[h] >= a.stag_s2) cmaxv = fmax(cmaxv, dts[h]);
                         }
                     }
-    #pragma unroll
+                    V4* const row = sout + size_t(rm2) * nx;
+#pragma unroll
                     for (int h = 0; h < CPL; ++h) {
                         if (!own_lane[h]) continue;
-                        const size_t c2 = size_t(rm2) * nx + j[h];
-                        const R hn = hn_[h];
-                        const R dm = dm2[h];
                         V4 o4;
-                        o4.x = hn;
+                        o4.x = hn[h];
                         o4.y = qxl2[h];
                         o4.z = qyl2[h];
-                        o4.w = hn > dm ? hn : dm;   // save_output_maps.m:598, max(d_t, dmax)
-                        sout[c2] = o4;
-                        // running maxima of the velocity raster and of depth x velocity
-                        // (save_output_maps.m:588-604, snisb_velocity_hazard_snapshot :832-848)
-                        if (INFL && a.vmax) {
+                        o4.w = hn[h] > dm2[h] ? hn[h] : dm2[h];   // save_output_maps.m:598, max(d_t, dmax)
+                        row[j[h]] = o4;
+                    }
+                    // running maxima of the velocity raster and of depth x velocity
+                    // (save_output_maps.m:588-604, snisb_velocity_hazard_snapshot :832-848)
+                    if (INFL && a.vmax) {
+#pragma unroll
+                        for (int h = 0; h < CPL; ++h) {
+                            if (!own_lane[h]) continue;
+                            const size_t c2 = size_t(rm2) * nx + j[h];
                             const R vo = a.vmax[c2];
                             a.vmax[c2] = vras[h] > vo ? vras[h] : vo;
-                            const R hd = fmax(hn, R(0));
+                            const R hd = fmax(hn[h], R(0));
                             R hz = hd * vras[h];
                             if (hd < R(0.01) || !isfinite(hz)) hz = R(0);
                             const R ho = a.hzmax[c2];
-                            a.hzmax[c2] = isnan(hn) ? hn : (hz > ho ? hz : ho);
+                            a.hzmax[c2] = isnan(hn[h]) ? hn[h] : (hz > ho ? hz : ho);
                         }
                     }
                 }

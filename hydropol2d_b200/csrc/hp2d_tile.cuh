@@ -117,7 +117,8 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
         const unsigned b = __ballot_sync(FULL, f);
         return ((b >> 9) & 1u) | ((b >> 4) & 1u) << 1 | (b == FULL ? 4u : 0u);
     };
-    const V4 out_S{R(0), R(0), R(0), make_meta<R>(255u)}, out_X{R(0), R(0), R(0), R(0)};
+    const R inf = R(__int_as_float(0x7f800000));
+    const V4 out_S{inf, inf, R(1), make_meta<R>(255u)}, out_X{R(0), R(0), R(0), R(0)};   // closed faces
 
     // the static records do not depend on the step's scalars; the state records and the dry flags are
     // fetched while warp 0 ends the step before
@@ -278,38 +279,38 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
             } else {
             // (B, C) unlimited faces
             R hfx[RPT], hfy[RPT], qxu[RPT], qyu[RPT], Sx[RPT], Sy[RPT];
-            bool wx[RPT], wy[RPT];
-            bool any_wet = false, any_rare = false;
+            R hmax = R(0);
+            bool edge = false;
 #pragma unroll
             for (int i = 0; i < RPT; ++i) {
-                const int r = rw + i;
                 const R hR = __shfl_down_sync(FULL, hT[i], 1);
                 const R hU = i > 0 ? hT[i > 0 ? i - 1 : 0] : x_h[warp - 1][lane];
-                const bool in = col_ok && r >= 0 && r < ny;
-                const bool ox = face_open<R, true>(hT[i], hR, S[i].x, hfx[i], Sx[i], K);
-                const bool oy = face_open<R, false>(hU, hT[i], S[i].y, hfy[i], Sy[i], K);
-                if (__any_sync(FULL, !(ox && oy && in))) {   // the grid's edges and idx_nan cells
-                    hfx[i] = !in ? R(0) : ox ? hfx[i] : face_closed(hT[i], hR, S[i].x);
-                    hfy[i] = !in ? R(0) : oy ? hfy[i] : face_closed(hU, hT[i], S[i].y);
-                }
-                wx[i] = in && ox && hfx[i] > R(0);
-                wy[i] = in && oy && hfy[i] > R(0);
+                face_open<R, true>(hT[i], hR, S[i].x, hfx[i], Sx[i], K);
+                face_open<R, false>(hU, hT[i], S[i].y, hfy[i], Sy[i], K);
+                edge = edge || face_edge(fmax(fabs(S[i].x), fabs(S[i].y)));
                 qxu[i] = qyu[i] = R(0);
-                any_wet = any_wet || wx[i] || wy[i];
-                any_rare = any_rare || (wx[i] && below_normal(hfx[i])) || (wy[i] && below_normal(hfy[i]));
             }
-            if (__any_sync(FULL, any_wet)) {
+            if (__any_sync(FULL, edge)) {   // the grid's edges, cells outside it
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) {
+                    if (face_edge(S[i].x)) hfx[i] = R(0);
+                    if (face_edge(S[i].y)) hfy[i] = R(0);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) hmax = fmax(hmax, fmax(hfx[i], hfy[i]));
+            if (__any_sync(FULL, hmax > R(0))) {
                 R px[RPT], py[RPT];   // H^(7/3)
 #pragma unroll
                 for (int i = 0; i < RPT; ++i) {
                     px[i] = pow73_normal(hfx[i]);
                     py[i] = pow73_normal(hfy[i]);
                 }
-                if (__any_sync(FULL, any_rare)) {
+                if (LI || sh.now.skip) {   // no clamp: depths of any size
 #pragma unroll
                     for (int i = 0; i < RPT; ++i) {
-                        if (wx[i] && below_normal(hfx[i])) px[i] = pow73_any(hfx[i]);
-                        if (wy[i] && below_normal(hfy[i])) py[i] = pow73_any(hfy[i]);
+                        if (hfx[i] > R(0) && below_normal(hfx[i])) px[i] = pow73_any(hfx[i]);
+                        if (hfy[i] > R(0) && below_normal(hfy[i])) py[i] = pow73_any(hfy[i]);
                     }
                 }
 #pragma unroll
@@ -318,18 +319,18 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                     R xa = R(0), xb = R(0), ya = R(0), yb = R(0);
                     if (SCH) {   // previous fluxes of the neighbouring faces (interior columns / rows only)
                         const size_t c = size_t(r) * nx + j;
-                        if (wx[i] && j >= 1 && j + 1 < nx) {
+                        if (hfx[i] > R(0) && j >= 1 && j + 1 < nx) {
                             xa = sin[c - 1].y;
                             xb = sin[c + 1].y;
                         }
-                        if (wy[i] && r >= 1 && r + 1 < ny) {
+                        if (hfy[i] > R(0) && r >= 1 && r + 1 < ny) {
                             ya = sin[c - nx].z;
                             yb = sin[c + nx].z;
                         }
                     }
-                    qxu[i] = face_update<R, SCH>(wx[i], hfx[i], px[i], Sx[i], X[i].y, S[i].z, K, a.flag_critical,
+                    qxu[i] = face_update<R, SCH>(hfx[i], px[i], Sx[i], X[i].y, S[i].z, K, a.flag_critical,
                                                  a.scheme, xa, xb);
-                    qyu[i] = face_update<R, SCH>(wy[i], hfy[i], py[i], Sy[i], X[i].z, S[i].z, K, a.flag_critical,
+                    qyu[i] = face_update<R, SCH>(hfy[i], py[i], Sy[i], X[i].z, S[i].z, K, a.flag_critical,
                                                  a.scheme, ya, yb);
                 }
             }
