@@ -851,27 +851,16 @@ __device__ __forceinline__ R face_momentum(bool wet, R Hf, R S, R qp, R n2c, con
 // ---------------- the fused steps' form of the same arithmetic -------------------------------
 // The wet path is bound by instruction issue, so these leave out what cannot change a result of the
 // fused kernels: the depths that enter are >= 0 (or NaN, next to closed faces only); whether a face is
-// open and wet needs no flag of its own (face_open, face_update); the grid's edges and face depths
+// open and wet needs no flag of its own (faces_open, faces_update); the grid's edges and face depths
 // below the smallest normal number are left to branches that whole warps skip.  The latter need the
 // depths' clamp to be off: between depths that are 0 or at least 1e-9, a positive face depth is a
 // difference of numbers that size, at least their last place.  Every face and cell gets the bits of face_flux,
 // donor_scale, limit_face and cfl_cell (up to the sign of a zero).
 //
-// face_open: the face depth and slope of a face whose dz is finite or NaN.  A NaN dz (next to an idx_nan
-// cell) takes part in no minimum or maximum, which leaves the inside cell's depth, as the closed face has
-// it; its NaN slope makes the momentum update 0.  Faces closed by an infinite dz (the grid's edges) get
-// depth 0 from their callers, and with it flux 0.
-template <typename R, bool IS_X>
-__device__ __forceinline__ void face_open(R ha, R hb, R dz, R& Hf, R& S, const StepConsts<R>& K) {
-    const R up = fmax(dz, R(0)), dn = fmin(dz, R(0));
-    if (IS_X) {
-        Hf = fmax(fmax(ha - up, hb + dn), R(0));
-        S = (dz + (hb - ha)) * K.inv_dx;
-    } else {
-        Hf = fmax(fmax(ha + dn, hb - up), R(0));
-        S = (dz + (ha - hb)) * K.inv_dx;
-    }
-}
+// faces_open (below): the depths and slopes of a cell's two faces, whose dz is finite or NaN.  A NaN dz
+// (next to an idx_nan cell) takes part in no minimum or maximum, which leaves the inside cell's depth, as
+// the closed face has it; its NaN slope makes the momentum update 0.  Faces closed by an infinite dz
+// (the grid's edges) get depth 0 from the callers, and with it flux 0.
 template <typename R> __device__ __forceinline__ bool face_edge(R dz) { return fabs(dz) > R(3.0e38); }
 // x^(7/3) of a normal positive number
 template <typename R> __device__ __forceinline__ R pow73_normal(R x) {
@@ -889,24 +878,107 @@ template <typename R> __device__ __forceinline__ R pow73_normal(R x) {
 template <typename R> __device__ __noinline__ R pow73_any(R x) { return pow73_pos(x); }
 __device__ __forceinline__ bool finite_abs(float x) { return fabsf(x) <= 3.402823466e+38f; }
 __device__ __forceinline__ bool finite_abs(double x) { return fabs(x) <= 1.7976931348623157e+308; }
-// the momentum update of a face.  One of depth 0 gets 0 whatever the rest: a finite quotient is cut
-// to +-10 H = 0 and any other becomes 0.
-template <typename R, int SCH = 0>
-__device__ __forceinline__ R face_update(R H, R h73, R S, R qp, R n2c, const StepConsts<R>& K, int flag_critical,
-                                         int scheme = 1, R q_lo = R(0), R q_hi = R(0)) {
-    R qn = qp;
-    if (SCH) qn = diffused_momentum(qp, q_lo, q_hi, H, K, scheme);
-    const R num = fma(-(K.gdt * H), S, qn);
-    const R den = fma(K.gdt * n2c, fabs(qp), h73);
-    R qq = qdiv(num * h73, den);
-    const bool ok = finite_abs(qq);
-    if (flag_critical == 1) {
-        const R crit = H * sqrt(K.g * H);
-        qq = fmin(fmax(qq, -crit), crit);
+
+// Two values that go through the same operations, a cell's x and y face: in FP32 one instruction
+// does both (f32x2, each half rounded as by itself), half the issue slots of the wet path's longest
+// chains.
+template <typename R> struct Two;
+template <> struct Two<float> {
+    unsigned long long v;
+};
+template <> struct Two<double> {
+    double a, b;
+};
+__device__ __forceinline__ Two<float> two(float a, float b) {
+    Two<float> r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void split(Two<float> x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ Two<float> two_mul(Two<float> x, Two<float> y) {
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(x.v) : "l"(y.v));
+    return x;
+}
+__device__ __forceinline__ Two<float> two_add(Two<float> x, Two<float> y) {
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x.v) : "l"(y.v));
+    return x;
+}
+__device__ __forceinline__ Two<float> two_fma(Two<float> x, Two<float> y, Two<float> z) {
+    Two<float> r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(x.v), "l"(y.v), "l"(z.v));
+    return r;
+}
+__device__ __forceinline__ Two<double> two(double a, double b) { return {a, b}; }
+__device__ __forceinline__ void split(Two<double> x, double& a, double& b) { a = x.a; b = x.b; }
+__device__ __forceinline__ Two<double> two_mul(Two<double> x, Two<double> y) { return {x.a * y.a, x.b * y.b}; }
+__device__ __forceinline__ Two<double> two_add(Two<double> x, Two<double> y) { return {x.a + y.a, x.b + y.b}; }
+__device__ __forceinline__ Two<double> two_fma(Two<double> x, Two<double> y, Two<double> z) {
+    return {fma(x.a, y.a, z.a), fma(x.b, y.b, z.b)};
+}
+// pow73_normal of both; the root's iterates carry the other sign, which their rounding does not see
+__device__ __forceinline__ Two<float> pow73_normal(float a, float b) {
+    const Two<float> x = two(a, b), one = two(1.0f, 1.0f), third = two(float(1.0 / 3.0), float(1.0 / 3.0));
+    Two<float> r = two(__uint_as_float(0xD4AAAAABu - __float_as_uint(a) / 3u), __uint_as_float(0xD4AAAAABu - __float_as_uint(b) / 3u));
+#pragma unroll
+    for (int it = 0; it < RcbrtTraits<float>::iters; ++it) {
+        const Two<float> e = two_fma(two_mul(two_mul(x, r), r), r, one);
+        r = two_fma(two_mul(r, e), third, r);
     }
-    const R thr = H * R(10);
-    qq = fmin(fmax(qq, -thr), thr);
-    return ok ? qq : R(0);
+    return two_mul(two_mul(x, x), two_mul(x, two_mul(r, r)));
+}
+__device__ __forceinline__ Two<double> pow73_normal(double a, double b) { return {pow73_normal(a), pow73_normal(b)}; }
+// minus qdiv(a, d) of both
+__device__ __forceinline__ Two<float> qdiv_neg(Two<float> a, float d0, float d1) {
+    d0 = fmaxf(d0, 1.17549435e-38f);
+    d1 = fmaxf(d1, 1.17549435e-38f);
+    const Two<float> b = two(d0, d1), one = two(1.0f, 1.0f);
+    Two<float> r = two(__uint_as_float(0xFEF311C3u - __float_as_uint(d0)), __uint_as_float(0xFEF311C3u - __float_as_uint(d1)));
+#pragma unroll
+    for (int it = 0; it < 3; ++it) r = two_fma(r, two_fma(b, r, one), r);
+    const Two<float> q = two_mul(a, r);
+    return two_fma(two_fma(b, q, a), r, q);
+}
+__device__ __forceinline__ Two<double> qdiv_neg(Two<double> a, double d0, double d1) { return {-(a.a / d0), -(a.b / d1)}; }
+// depths and slopes of a cell's two faces: its depth h and its neighbours hr (right) and hu (above)
+template <typename R>
+__device__ __forceinline__ void faces_open(R h, R hr, R hu, R dzx, R dzy, R& Hx, R& Hy, Two<R>& S, const StepConsts<R>& K) {
+    const Two<R> own = two_add(two(h, h), two(fmin(-dzx, R(0)), fmin(-dzy, R(0))));
+    const Two<R> nbr = two_add(two(hr, hu), two(fmin(dzx, R(0)), fmin(dzy, R(0))));
+    R ox, oy, nx, ny;
+    split(own, ox, oy);
+    split(nbr, nx, ny);
+    Hx = fmax(fmax(ox, nx), R(0));
+    Hy = fmax(fmax(oy, ny), R(0));
+    S = two_mul(two_add(two(dzx, dzy), two(hr - h, hu - h)), two(K.inv_dx, K.inv_dx));
+}
+// The momentum update of a cell's two faces (Hx, Hy: their depths, h73 their powers 7/3, S their
+// slopes, qx, qy their fluxes before and after).  A face of depth 0 gets 0 whatever the rest: a finite
+// quotient is cut to +-10 H = 0 and any other becomes 0.
+template <typename R, int SCH = 0>
+__device__ __forceinline__ void faces_update(R Hx, R Hy, Two<R> h73, Two<R> S, R& qx, R& qy, R n2c, const StepConsts<R>& K,
+                                             int flag_critical, int scheme = 1, R x_lo = R(0), R x_hi = R(0),
+                                             R y_lo = R(0), R y_hi = R(0)) {
+    R nx = qx, ny = qy;
+    if (SCH) {
+        nx = diffused_momentum(qx, x_lo, x_hi, Hx, K, scheme);
+        ny = diffused_momentum(qy, y_lo, y_hi, Hy, K, scheme);
+    }
+    const Two<R> num = two_fma(two_mul(two(-K.gdt, -K.gdt), two(Hx, Hy)), S, two(nx, ny));
+    R px, py, vx, vy;
+    split(h73, px, py);
+    const R fr = K.gdt * n2c;
+    split(qdiv_neg(two_mul(num, h73), fma(fr, fabs(qx), px), fma(fr, fabs(qy), py)), vx, vy);
+    const bool okx = finite_abs(vx), oky = finite_abs(vy);
+    vx = -vx;
+    vy = -vy;
+    if (flag_critical == 1) {
+        const R cx = Hx * sqrt(K.g * Hx), cy = Hy * sqrt(K.g * Hy);
+        vx = fmin(fmax(vx, -cx), cx);
+        vy = fmin(fmax(vy, -cy), cy);
+    }
+    const R tx = Hx * R(10), ty = Hy * R(10);
+    qx = okx ? fmin(fmax(vx, -tx), tx) : R(0);
+    qy = oky ? fmin(fmax(vy, -ty), ty) : R(0);
 }
 // what leaves a cell and what it holds, as rates: its faces are limited when the first exceeds the
 // second (donor_scale)
@@ -923,6 +995,16 @@ __device__ __forceinline__ float face_velocity(float q, float hf, const StepCons
 }
 __device__ __forceinline__ double face_velocity(double q, double hf, const StepConsts<double>& K) {
     return q == 0.0 ? 0.0 : q / (hf < K.tol ? 1e9 : hf);
+}
+// minus the velocities of two faces
+__device__ __forceinline__ void face_velocities_neg(float qa, float ha, float qb, float hb, const StepConsts<float>& K, float& va,
+                                                    float& vb) {
+    split(qdiv_neg(two(qa, qb), ha < K.tol ? 1e9f : ha, hb < K.tol ? 1e9f : hb), va, vb);
+}
+__device__ __forceinline__ void face_velocities_neg(double qa, double ha, double qb, double hb, const StepConsts<double>& K,
+                                                    double& va, double& vb) {
+    va = -face_velocity(qa, ha, K);
+    vb = -face_velocity(qb, hb, K);
 }
 
 // outgoing rate of a cell over its four faces and its donor scale factor

@@ -1078,13 +1078,13 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                 }
                 // (B) and (C) interleaved: the geometry of the 2 x CPL faces, then -- unless no
                 // lane of the warp has a wet one -- their momentum updates without branches
-                R Sx[CPL], Sy[CPL], ya[CPL], yb[CPL];
+                Two<R> Sl[CPL];
+                R ya[CPL], yb[CPL];
                 R hmax = R(0);
                 bool edge = false;
 #pragma unroll
                 for (int h = 0; h < CPL; ++h) {
-                    face_open<R, true>(hT0[h], hR[h], S[h].x, hfx0[h], Sx[h], K);
-                    face_open<R, false>(hT1[h], hT0[h], S[h].y, hfy0[h], Sy[h], K);
+                    faces_open<R>(hT0[h], hR[h], hT1[h], S[h].x, S[h].y, hfx0[h], hfy0[h], Sl[h], K);
                     edge = edge || face_edge(fmax(fabs(S[h].x), fabs(S[h].y)));
                 }
                 if (__any_sync(FULL, edge)) {
@@ -1105,25 +1105,21 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                     }
                 }
                 if (__any_sync(FULL, hmax > R(0))) {
-                    R px[CPL], py[CPL];   // H^(7/3)
+                    Two<R> p73[CPL];   // H^(7/3)
 #pragma unroll
-                    for (int h = 0; h < CPL; ++h) {
-                        px[h] = pow73_normal(hfx0[h]);
-                        py[h] = pow73_normal(hfy0[h]);
-                    }
+                    for (int h = 0; h < CPL; ++h) p73[h] = pow73_normal(hfx0[h], hfy0[h]);
                     if (sh.now.skip) {   // no clamp: depths of any size
 #pragma unroll
-                        for (int h = 0; h < CPL; ++h) {
-                            if (hfx0[h] > R(0) && below_normal(hfx0[h])) px[h] = pow73_any(hfx0[h]);
-                            if (hfy0[h] > R(0) && below_normal(hfy0[h])) py[h] = pow73_any(hfy0[h]);
-                        }
+                        for (int h = 0; h < CPL; ++h)
+                            if ((hfx0[h] > R(0) && below_normal(hfx0[h])) || (hfy0[h] > R(0) && below_normal(hfy0[h])))
+                                p73[h] = two(pow73_any(hfx0[h]), pow73_any(hfy0[h]));
                     }
 #pragma unroll
                     for (int h = 0; h < CPL; ++h) {
-                        qxu0[h] = face_update<R, SCH>(hfx0[h], px[h], Sx[h], X[h].y, S[h].z, K, a.flag_critical,
-                                                       a.scheme, SCH ? qxa[h] : R(0), SCH ? qxb[h] : R(0));
-                        qyu0[h] = face_update<R, SCH>(hfy0[h], py[h], Sy[h], X[h].z, S[h].z, K, a.flag_critical,
-                                                       a.scheme, ya[h], yb[h]);
+                        qxu0[h] = X[h].y;
+                        qyu0[h] = X[h].z;
+                        faces_update<R, SCH>(hfx0[h], hfy0[h], p73[h], Sl[h], qxu0[h], qyu0[h], S[h].z, K, a.flag_critical,
+                                             a.scheme, SCH ? qxa[h] : R(0), SCH ? qxb[h] : R(0), ya[h], yb[h]);
                     }
                 }
                 // (D) which cells of row r-1 have their faces limited
@@ -1248,19 +1244,18 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
                     // refreshing_timestep.m:61-89, :139-150, :181-238 for these cells; an apron lane's
                     // values are computed and dropped, so that the CPL cells interleave
                     if (mine && !quiet) {
-                        R vr[CPL], vu[CPL], s2[CPL], dts[CPL];
-#pragma unroll
-                        for (int h = 0; h < CPL; ++h) vr[h] = face_velocity(qxl2[h], hfx2[h], K);
+                        R vr[CPL], vu[CPL], s2[CPL], dts[CPL];   // velocities with the other sign
                         if (vcar_ok) {
 #pragma unroll
                             for (int h = 0; h < CPL; ++h) vu[h] = vcar[h];
                         } else {
 #pragma unroll
-                            for (int h = 0; h < CPL; ++h) vu[h] = face_velocity(qyl2[h], hfy2[h], K);
+                            for (int h = 0; h < CPL; ++h) vu[h] = -face_velocity(qyl2[h], hfy2[h], K);
                         }
 #pragma unroll
                         for (int h = 0; h < CPL; ++h) {
-                            const R vb = face_velocity(qyl1[h], hfy1[h], K);
+                            R vb;
+                            face_velocities_neg(qxl2[h], hfx2[h], qyl1[h], hfy1[h], K, vr[h], vb);
                             vcar[h] = vb;
                             if (INFL) vras[h] = fmax(fmax(fabs(vr[h]), fabs(vu[h])), fabs(vb));
                             const R rc = h == 0 ? vr[h] * rc_half : vr[h];

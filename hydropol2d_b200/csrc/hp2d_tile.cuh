@@ -278,15 +278,15 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                 publish = false;
             } else {
             // (B, C) unlimited faces
-            R hfx[RPT], hfy[RPT], qxu[RPT], qyu[RPT], Sx[RPT], Sy[RPT];
+            R hfx[RPT], hfy[RPT], qxu[RPT], qyu[RPT];
+            Two<R> Sl[RPT];
             R hmax = R(0);
             bool edge = false;
 #pragma unroll
             for (int i = 0; i < RPT; ++i) {
                 const R hR = __shfl_down_sync(FULL, hT[i], 1);
                 const R hU = i > 0 ? hT[i > 0 ? i - 1 : 0] : x_h[warp - 1][lane];
-                face_open<R, true>(hT[i], hR, S[i].x, hfx[i], Sx[i], K);
-                face_open<R, false>(hU, hT[i], S[i].y, hfy[i], Sy[i], K);
+                faces_open<R>(hT[i], hR, hU, S[i].x, S[i].y, hfx[i], hfy[i], Sl[i], K);
                 edge = edge || face_edge(fmax(fabs(S[i].x), fabs(S[i].y)));
                 qxu[i] = qyu[i] = R(0);
             }
@@ -300,18 +300,14 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
 #pragma unroll
             for (int i = 0; i < RPT; ++i) hmax = fmax(hmax, fmax(hfx[i], hfy[i]));
             if (__any_sync(FULL, hmax > R(0))) {
-                R px[RPT], py[RPT];   // H^(7/3)
+                Two<R> p73[RPT];   // H^(7/3)
 #pragma unroll
-                for (int i = 0; i < RPT; ++i) {
-                    px[i] = pow73_normal(hfx[i]);
-                    py[i] = pow73_normal(hfy[i]);
-                }
+                for (int i = 0; i < RPT; ++i) p73[i] = pow73_normal(hfx[i], hfy[i]);
                 if (LI || sh.now.skip) {   // no clamp: depths of any size
 #pragma unroll
-                    for (int i = 0; i < RPT; ++i) {
-                        if (hfx[i] > R(0) && below_normal(hfx[i])) px[i] = pow73_any(hfx[i]);
-                        if (hfy[i] > R(0) && below_normal(hfy[i])) py[i] = pow73_any(hfy[i]);
-                    }
+                    for (int i = 0; i < RPT; ++i)
+                        if ((hfx[i] > R(0) && below_normal(hfx[i])) || (hfy[i] > R(0) && below_normal(hfy[i])))
+                            p73[i] = two(pow73_any(hfx[i]), pow73_any(hfy[i]));
                 }
 #pragma unroll
                 for (int i = 0; i < RPT; ++i) {
@@ -328,10 +324,10 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                             yb = sin[c + nx].z;
                         }
                     }
-                    qxu[i] = face_update<R, SCH>(hfx[i], px[i], Sx[i], X[i].y, S[i].z, K, a.flag_critical,
-                                                 a.scheme, xa, xb);
-                    qyu[i] = face_update<R, SCH>(hfy[i], py[i], Sy[i], X[i].z, S[i].z, K, a.flag_critical,
-                                                 a.scheme, ya, yb);
+                    qxu[i] = X[i].y;
+                    qyu[i] = X[i].z;
+                    faces_update<R, SCH>(hfx[i], hfy[i], p73[i], Sl[i], qxu[i], qyu[i], S[i].z, K, a.flag_critical, a.scheme,
+                                         xa, xb, ya, yb);
                 }
             }
             x_q[warp][lane] = qyu[0];
@@ -349,7 +345,7 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                 // (the rows outside the grid have no flux; the apron's outer columns are not looked at)
                 lim = lim || (out[i] > hT[i] * K.dx_over_dt && lane > 0 && r >= r0 - 1);
             }
-            R qxl[RPT], qyl[RPT], vu[RPT];
+            R qxl[RPT], qyl[RPT], vu[RPT], vr[RPT];
             if (bar_or<1, NT - 32>(lim)) {
                 R sc[RPT];
 #pragma unroll
@@ -375,7 +371,10 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                 }
             }
 #pragma unroll
-            for (int i = 0; i < RPT; ++i) vu[i] = LI ? R(0) : face_velocity(qyl[i], hfy[i], K);   // of the upper face
+            for (int i = 0; i < RPT; ++i) {   // of the upper and the right face, with the other sign
+                vu[i] = vr[i] = R(0);
+                if (!LI) face_velocities_neg(qyl[i], hfy[i], qxl[i], hfx[i], K, vu[i], vr[i]);
+            }
             x_l[warp][lane] = qyl[0];
             x_v[warp][lane] = vu[0];
             bar_sync<2, NT>();
@@ -384,7 +383,6 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
             for (int i = 0; i < RPT; ++i) {
                 const int r = rw + i;
                 const R qxl_left = __shfl_up_sync(FULL, qxl[i], 1);
-                const R vr = LI ? R(0) : face_velocity(qxl[i], hfx[i], K);
                 if (!(own_lane && r >= r0 && r < r_end)) continue;
                 const R qyd = i + 1 < RPT ? qyl[i + 1 < RPT ? i + 1 : i] : x_l[warp + 1 < NW ? warp + 1 : 0][lane];
                 const R vb = i + 1 < RPT ? vu[i + 1 < RPT ? i + 1 : i] : x_v[warp + 1 < NW ? warp + 1 : 0][lane];
@@ -432,8 +430,8 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                 if (dm < K.thr && hn >= K.thr) a.arrival[c] = R(sh.now.t_min * 60.0 + sh.now.dts);
                 R vras = R(0);   // velocity raster: largest |face velocity|
                 if (mine) {
-                    if (INFL) vras = fmax(fmax(fabs(vr), fabs(vu[i])), fabs(vb));
-                    const R rc = vr * first_col;
+                    if (INFL) vras = fmax(fmax(fabs(vr[i]), fabs(vu[i])), fabs(vb));
+                    const R rc = vr[i] * first_col;
                     const R uc = R(0.5) * (vu[i] + vb);
                     const R s2 = rc * rc + uc * uc;
                     s2max = fmax(s2max, s2);
@@ -441,7 +439,7 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                     // by g is monotone)
                     if (s2 >= a.stag_s2) {
                         if (a.adaptive != 1)
-                            dts = fmax(fmax(fabs(vr), fabs(vu[i])), fabs(vb)) + fmax(sqrt(K.g * fmax(dts, R(0))), R(1e-10));
+                            dts = fmax(fmax(fabs(vr[i]), fabs(vu[i])), fabs(vb)) + fmax(sqrt(K.g * fmax(dts, R(0))), R(1e-10));
                         cmaxv = fmax(cmaxv, dts);
                     }
                 }
