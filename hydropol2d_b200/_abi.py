@@ -200,7 +200,7 @@ def lib() -> C.CDLL:
         "hp2d_nn_conv3x3": ([vp, i32, i32, i32, i32, vp, i32, i32, vp, vp, i32, i32, vp], C.c_int),
         "hp2d_nn_conv3x3_any": ([vp, i32, i32, i32, i32, vp, i32, i32, vp, vp, i32, i32, vp], C.c_int),
         "hp2d_nn_conv3x3_wgrad": ([vp, i32, i32, i32, i32, vp, i32, vp, i32, vp], C.c_int),
-        "hp2d_nn_relu_colsum": ([vp, vp, i64, i32, vp, vp], C.c_int),
+        "hp2d_nn_relu_colsum": ([vp, i64, vp, i64, i32, vp, vp], C.c_int),
         "hp2d_nn_check": ([], C.c_int),
         "hp2d_nn_error": ([], C.c_char_p),
         "hp2d_nn_im2col3x3": ([vp, i32, i32, i32, i32, vp, i32, i32, vp], C.c_int),

@@ -659,7 +659,7 @@ __global__ void k_copy_channels_v8(const uint4* __restrict__ in, int cin8, int c
 }
 // The ReLU's mask on dy (in place, y null: none) and dy's column sums into out, in one pass: a thread
 // keeps the sums of its 8 channels over its pixels, the block adds its threads' up in shared memory.
-__global__ void __launch_bounds__(256) k_relu_colsum_v8(const uint4* __restrict__ y, uint4* __restrict__ dy, int64_t P, int C8,
+__global__ void __launch_bounds__(256) k_relu_colsum_v8(const uint4* __restrict__ y, int64_t ldy8, uint4* __restrict__ dy, int64_t P, int C8,
                                                         float* __restrict__ out) {
     extern __shared__ float s_part[];   // [256 / C8][C8 * 8]
     const int c = threadIdx.x % C8, pl = threadIdx.x / C8, per = 256 / C8;
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(256) k_relu_colsum_v8(const uint4* __restrict_
         for (int64_t p = int64_t(blockIdx.x) * per + pl; p < P; p += int64_t(gridDim.x) * per) {
             Vec8 d = load8(dy + p * C8 + c);
             if (y) {
-                const Vec8 v = load8(y + p * C8 + c);
+                const Vec8 v = load8(y + p * ldy8 + c);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     if (!(v.get(i) > 0.0f)) d.set(i, 0u);
@@ -841,16 +841,17 @@ hp2d_status hp2d_nn_colsum(const uint16_t* dz, int64_t P, int32_t C, int32_t ld,
     return launched("colsum");
 }
 
-hp2d_status hp2d_nn_relu_colsum(const uint16_t* y, uint16_t* dy, int64_t P, int32_t C, float* out, void* stream) {
-    if (!dy || !out || P <= 0 || C <= 0) return fail("relu_colsum: bad shape");
-    if (C % 8 == 0 && C <= 2048 && aligned16(dy) && (!y || aligned16(y))) {
+hp2d_status hp2d_nn_relu_colsum(const uint16_t* y, int64_t ldy, uint16_t* dy, int64_t P, int32_t C, float* out, void* stream) {
+    if (!dy || !out || P <= 0 || C <= 0 || (y && ldy < C)) return fail("relu_colsum: bad shape");
+    if (C % 8 == 0 && C <= 2048 && aligned16(dy) && (!y || (aligned16(y) && ldy % 8 == 0))) {
         const int per = 256 / std::min(C / 8, 256);
         const unsigned grid = unsigned(std::min<int64_t>((P + per - 1) / per, 148 * 4));
         k_relu_colsum_v8<<<grid, 256, size_t(per) * C * sizeof(float), S(stream)>>>(
-            reinterpret_cast<const uint4*>(y), reinterpret_cast<uint4*>(dy), P, C / 8, out);
+            reinterpret_cast<const uint4*>(y), ldy / 8, reinterpret_cast<uint4*>(dy), P, C / 8, out);
         return launched("relu_colsum");
     }
     if (y) {
+        if (ldy != C) return fail("relu_colsum: a pitch needs multiples of 8 channels", HP2D_UNSUPPORTED_FLAG);
         const hp2d_status r = hp2d_nn_relu_bwd(y, dy, P * C, stream);
         if (r != HP2D_OK) return r;
     }

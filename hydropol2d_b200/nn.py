@@ -159,8 +159,8 @@ def colsum(dz2d, out):
 def relu_colsum(y, dy2d, out):
     """``relu_bwd`` of dy2d [P, C] by y (None: no ReLU) and ``colsum`` of the result, in one pass."""
     P, Cc = dy2d.shape
-    assert dy2d.is_contiguous() and (y is None or y.is_contiguous())
-    _ok(_L().hp2d_nn_relu_colsum(_p(y), _p(dy2d), P, Cc, _p(out), _stream()))
+    assert dy2d.is_contiguous() and (y is None or (y.shape == dy2d.shape and y.stride(1) == 1))
+    _ok(_L().hp2d_nn_relu_colsum(_p(y), Cc if y is None else y.stride(0), _p(dy2d), P, Cc, _p(out), _stream()))
 
 
 def mse(pred, target, weight, scale, loss, dpred):

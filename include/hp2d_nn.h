@@ -86,7 +86,7 @@ hp2d_status hp2d_nn_relu_bwd(const uint16_t* y, uint16_t* dy, int64_t n, void* s
 /* out[c] += sum_p dz[p, c]  (dz [P, C] pitch ld) */
 hp2d_status hp2d_nn_colsum(const uint16_t* dz, int64_t P, int32_t C, int32_t ld, float* out, void* stream);
 /* hp2d_nn_relu_bwd (y null: none) and hp2d_nn_colsum of the result in one pass over dy [P, C] */
-hp2d_status hp2d_nn_relu_colsum(const uint16_t* y, uint16_t* dy, int64_t P, int32_t C, float* out, void* stream);
+hp2d_status hp2d_nn_relu_colsum(const uint16_t* y, int64_t ldy, uint16_t* dy, int64_t P, int32_t C, float* out, void* stream);
 /* masked squared error over channels 0..nch-1 of pred [P, ldp] (fp32) against target
  * [P, nch] with weights w [P, nch] (fp32): loss += sum w (pred - t)^2 * scale and
  * dpred [P, ldd] (bf16, other channels zero) = 2 w (pred - t) * scale */

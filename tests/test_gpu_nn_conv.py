@@ -98,3 +98,35 @@ def test_vector_layers_equal_torch(C):
     nn.relu_colsum(y, g, out)
     assert torch.equal(g, masked)
     assert torch.all((out.double() - 1 - masked.double().sum(0)).abs() <= (1 + masked.double().abs().sum(0)) * 2.0 ** -20)
+
+
+@pytest.mark.parametrize("c,ld", [(8, 16), (32, 64), (64, 200)])
+def test_relu_mask_from_channels_of_a_wider_tensor(c, ld):
+    from hydropol2d_b200 import nn
+    wide, g = _rand((777, ld), 11), _rand((777, c), 12)
+    y = wide[:, 8:8 + c] if ld > c + 8 else wide[:, :c]
+    a, b = g.clone(), g.clone()
+    sa, sb = torch.zeros(c, device="cuda"), torch.zeros(c, device="cuda")
+    nn.relu_colsum(y, a, sa)
+    nn.relu_colsum(y.contiguous(), b, sb)
+    assert torch.equal(a, b)
+    torch.testing.assert_close(sa, sb, rtol=1e-5, atol=1e-4)   # FP32 sums of 777 terms in another order
+
+
+def test_adam_in_one_buffer_equals_adam_by_layer():
+    from hydropol2d_b200.surrogate import UNet
+    nets = [UNet(seed=5, base=16, levels=2) for _ in range(2)]
+    for c in nets[1].layers.values():   # tensors of their own: the layers one by one
+        c.W, c.b = c.W.clone(), c.b.clone()
+    for net in nets:
+        gen = torch.Generator().manual_seed(7)
+        for _ in range(2):
+            net.zero_grad()
+            for c in net.layers.values():
+                c.gW.add_(torch.randn(c.gW.shape, generator=gen).cuda())
+                c.gb.add_(torch.randn(c.gb.shape, generator=gen).cuda())
+            net.adam_step(1e-3, 1e-2)
+    assert nets[0]._one_buffer("W") and not nets[1]._one_buffer("W")
+    for a, b in zip(nets[0].layers.values(), nets[1].layers.values()):
+        for name in ("W", "b", "mW", "vW", "mb", "vb", "W16", "gW", "gb"):
+            assert torch.equal(getattr(a, name), getattr(b, name)), name
