@@ -395,9 +395,9 @@ template <typename R> struct Impl : Base {
         if (wait_polls != kWaitPolls) return 0;   // the caller bounds the row copies that strips have
         if (tile_mode >= 0) return tile_mode;
         // Up to where the tiles measured faster than the strips, us per step, strips / tiles.  FP32:
-        // 1000^2 56 / 29 wet, 54 / 22 valley, 103 / 50 Green-Ampt and rain maps; 1300^2 59 / 47, 58 / 30,
-        // 108 / 83; 1700^2 80 / 81, 80 / 51, 155 / 133; 2048^2 99 / 118, -, 203 / 200.  FP64: 1700^2 Green-Ampt
-        // and maps 291 / 259, wet 189 / 160.
+        // 1000^2 41 / 25 wet, 38 / 19 valley, 86 / 43 Green-Ampt and rain maps; 1300^2 44 / 43, 41 / 28,
+        // 93 / 68; 1500^2 44 / 53, 42 / 35, 101 / 90; 1700^2 58 / 81, 57 / 51, 139 / 113; 2048^2 180 / 169
+        // with Green-Ampt and maps.  FP64: 1700^2 Green-Ampt and maps 255 / 234, wet 161 / 141.
         const size_t most = sizeof(R) == 8 ? 4000000 : (inf_mode() || rain.n_maps) ? 4300000 : 2500000;
         if (n > most) return 0;
         return default_tile_rpt();
