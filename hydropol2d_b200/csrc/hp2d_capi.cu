@@ -403,7 +403,7 @@ template <typename R> struct Impl : Base {
         return default_tile_rpt();
     }
     // one row per thread while the grid gives the GPU little more than one wave of tiles (256^2 wet
-    // FP32 6.5 / 7.4 us with one / two rows, 400^2 9.7 / 9.5; FP64 Green-Ampt 600^2 43 / 46,
+    // FP32 6.5 / 7.4 us with one / two rows, 450^2 10.2 / 9.9, 700^2 16.7 / 14.5; FP64 Green-Ampt 600^2 43 / 46,
     // 1000^2 103 / 103)
     int default_tile_rpt() const { return n > (sizeof(R) == 8 ? 1000000u : 200000u) ? 2 : 1; }
     bool tile_on() const { return tile_rpt() != 0; }

@@ -221,7 +221,7 @@ template <int CPL> struct FusedOcc<double, CPL> { static constexpr int minb = CP
 // The depth d_tot a step hands to its fluxes at each control structure's reservoir cell --
 // phase (A) of that cell restated: rain, infiltration, inflow, clamps, from the state and
 // soil records `st`/`gs` the step starts from -- then the structures' transfers (one thread,
-// in structure order).  The last CTA of a step runs it for the next step; k_struct_prime for
+// in structure order).  The end of a step runs it for the next step; k_struct_prime for
 // the first step of a call.
 template <typename R, int INF, bool MAP, bool INFL>
 __device__ __noinline__ void structure_prepare(const FusedArgs<R>& a, const RainStep<R>& rs, bool skip,

@@ -31,16 +31,12 @@ namespace hp2d {
 
 // A CTA's warps and the rows per thread.  Warp 0 holds the first apron row only, the others RPT
 // consecutive rows each.
-#ifndef HP2D_TILE_NW2
-#define HP2D_TILE_NW2 12
-#define HP2D_TILE_MB2 2
-#endif
 template <typename R, int RPT> struct TileShape {
-    static constexpr int NW = RPT == 1 ? (sizeof(R) == 4 ? 16 : 12) : HP2D_TILE_NW2;
+    static constexpr int NW = RPT == 1 && sizeof(R) == 4 ? 16 : 12;
     static constexpr int NT = 32 * NW;
     static constexpr int OR = 1 + (NW - 1) * RPT - 4;   // output rows
     static constexpr int OC = 28;                       // output columns
-    static constexpr int MINB = RPT == 1 ? 2 : HP2D_TILE_MB2;   // CTAs per SM
+    static constexpr int MINB = 2;   // CTAs per SM
 };
 
 // named barriers over NTH threads
