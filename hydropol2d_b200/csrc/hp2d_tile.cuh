@@ -410,7 +410,8 @@ __device__ __forceinline__ void tile_body(const FusedArgs<R>& a, int phase, cons
                 }
                 R hn = continuity(h_in, qxl_left, qxl[i], qyl[i], qyd, K);
                 R dts = fmax(hfx[i], hfy[i]);
-                const unsigned ord = INFL ? outlet_ord(meta) : meta >> 8;
+                // LI's instantiation says nothing of gauge and stage cells: it takes any meta word
+                const unsigned ord = INFL || LI ? outlet_ord(meta) : meta >> 8;
                 if (ord) {
                     const int o = int(ord) - 1;
                     R ho;
