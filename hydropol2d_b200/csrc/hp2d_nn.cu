@@ -490,6 +490,8 @@ k_mse(const float* __restrict__ pred, int ldp, const float* __restrict__ t, cons
       float scale, float* loss, uint16_t* __restrict__ dpred, int ldd) {
     __shared__ double part[16];
     __shared__ double block_sum[kMseCluster];
+    auto cluster = cooperative_groups::this_cluster();
+    auto started = cluster.barrier_arrive();   // waited for before block 0's shared memory is written
     double acc = 0.0;
     for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < P; p += int64_t(gridDim.x) * blockDim.x) {
         for (int c = 0; c < ldd; ++c) {
@@ -505,8 +507,8 @@ k_mse(const float* __restrict__ pred, int ldp, const float* __restrict__ t, cons
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
-    auto cluster = cooperative_groups::this_cluster();
     __syncthreads();
+    cluster.barrier_wait(std::move(started));
     if (threadIdx.x == 0) {
         double s = 0.0;
         for (int i = 0; i < 16; ++i) s += part[i];
