@@ -1496,12 +1496,16 @@ template <typename R> struct Impl : Base {
         }
     }
 
+    // the steps' sums, where something may have been left in them (a step that was not ended)
+    void clear_sums() { HP_CK(cudaMemsetAsync(&ctl.p->acc[0], 0, sizeof(ctl.p->acc), st())); }
+
     // set by the prologue's scan: a cell of finite elevation holds a non-finite depth
     bool bad_state = false;
     void prologue() {
         dry_for_layout(cells_per_lane);
         if (!dirty) return;
         reset_dry();
+        clear_sums();
         HP_CK(cudaMemsetAsync(&ctl.p->prep[0], 0xff, 2 * sizeof(StepPrep<R>), st()));   // NaN keys: the first step makes its own
         pull_sc();
         hs.skip_clamp = 0;
@@ -1945,6 +1949,7 @@ template <typename R> struct Impl : Base {
         if (n_out) { copy_dev(hf3.p, s.hf3s.p, n_out); copy_dev(qo.p, s.qos.p, n_out); }
         sc_changed();
         copy_dev(sc.p, s.scs.p, 1);   // after a flush: nothing pending
+        clear_sums();
         reset_dry();
         HP_CK(cudaStreamSynchronize(st()));
         pull_sc();
@@ -2407,9 +2412,15 @@ struct hp2d_ensemble {
         HP_CK(cudaMemcpyAsync(&q, queue.p, sizeof(q), cudaMemcpyDeviceToHost, stream));
         HP_CK(cudaStreamSynchronize(stream));
         for (int m = 0; m < nm; ++m) {
-            impl(m).sc_changed();
-            impl(m).pull_sc();
-            impl(m).flush_records();
+            Impl<float>& im = impl(m);
+            im.sc_changed();
+            im.pull_sc();
+            if ((im.hs.status & kStatusTimeout) && !im.hs.halted) {   // a step whose items were not all taken
+                im.hs.halted = 1;
+                im.push_sc();
+                im.dirty = true;
+            }
+            im.flush_records();
         }
         unsigned retried = 0;
         for (int m = 0; m < nm; ++m) {   // a rejected member step: its retry, as on its own

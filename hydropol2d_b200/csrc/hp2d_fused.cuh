@@ -607,7 +607,12 @@ __device__ __forceinline__ bool step_finish(const FusedArgs<R>& a, StepShared<R,
         StepAcc* const acc = a.acc + (SOLO ? ((phase + 1) & 3) : 0);
         unsigned ticket = 0u;
         if (lane == 0) {
-            if (!cta_ok) atomicOr(&acc->timeout, 1u);   // a row copy did not arrive in time
+            if (!cta_ok) {   // a row copy did not arrive in time
+                atomicOr(&acc->timeout, 1u);
+                // an ensemble's CTA takes no more items after this: when all have given up, some of
+                // the member's are left and no last ticket reports it
+                if (!SOLO) atomicOr(&a.sc->status, kStatusTimeout);
+            }
             if (bad) atomicAdd(&acc->bad, (unsigned long long)bad);
             if (scode) atomicMax(&acc->vmax, scode);
             if (cenc) atomicMax(&acc->cmax, cenc);
