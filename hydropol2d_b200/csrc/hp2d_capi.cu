@@ -1291,8 +1291,10 @@ template <typename R> struct Impl : Base {
         a.tile_grid = unsigned(n_sms * (rpt == 2 ? T2::MINB : T1::MINB));
         a.n_ctas = unsigned(a.tile_nx * ((ny + rows - 1) / rows));
     }
-    FusedArgs<R> fused_args(int cpl = 0) {
-        if (cpl <= 0) cpl = cells_per_lane;
+    // strips_cpl > 0: for strips of that many cells per lane whatever the grid's own layout (an
+    // ensemble's queue holds items of strips)
+    FusedArgs<R> fused_args(int strips_cpl = 0) {
+        const int cpl = strips_cpl > 0 ? strips_cpl : cells_per_lane;
         FusedArgs<R> a{};
         const hp2d_params& p = ctx->p;
         a.ny = ny; a.nx = nx; a.res = res;
@@ -1334,7 +1336,7 @@ template <typename R> struct Impl : Base {
         a.dry_rows = dry_rows();
         a.dryflag = dry_usable(rpw) && tb_chosen <= 1 && !slab() ? dryf.p : nullptr;
         a.tile_nx = 0;
-        if (tile_on()) {
+        if (strips_cpl <= 0 && tile_on()) {
             tile_shape(a, tile_rpt());
             a.dryflag = dry_enabled && tb_chosen <= 1 && !slab() ? dryf.p : nullptr;
         }
@@ -1483,13 +1485,15 @@ template <typename R> struct Impl : Base {
     // without them do not maintain them, so any change of layout or of flag use clears them
     bool dry_enabled = true;   // hp2d_set_dry_skip
     bool dry_usable(int rpw) const { return dry_enabled && rpw % 4 == 0 && rpw <= 128; }
-    int dry_key(int cpl) {
-        if (const int t = tile_rpt()) return dry_enabled ? 64 * t : -64 * t;   // a flag per tile
+    int dry_key(int strips_cpl) {   // as fused_args
+        const int t = strips_cpl > 0 ? 0 : tile_rpt();
+        if (t) return dry_enabled ? 64 * t : -64 * t;   // a flag per tile
+        const int cpl = strips_cpl > 0 ? strips_cpl : cells_per_lane;
         const int rpw = rpw_chosen ? rows_per_warp : default_rows(cpl);
         return dry_usable(rpw) ? cpl : -cpl;
     }
-    void dry_for_layout(int cpl) {
-        const int key = dry_key(cpl);
+    void dry_for_layout(int strips_cpl) {
+        const int key = dry_key(strips_cpl);
         if (dry_layout != key || !dryf.p) {
             reset_dry();
             dry_layout = key;
@@ -1501,8 +1505,8 @@ template <typename R> struct Impl : Base {
 
     // set by the prologue's scan: a cell of finite elevation holds a non-finite depth
     bool bad_state = false;
-    void prologue() {
-        dry_for_layout(cells_per_lane);
+    void prologue(int strips_cpl = 0) {
+        dry_for_layout(strips_cpl);
         if (!dirty) return;
         reset_dry();
         clear_sums();
@@ -2345,16 +2349,11 @@ struct hp2d_ensemble {
                 im.rpw_chosen = true;
                 im.invalidate_graph();
             }
-            if (im.tile_mode != 0) {   // the queue's items are strips
-                im.tile_mode = 0;
-                im.invalidate_graph();
-            }
-            im.prologue();
+            im.prologue(cells_per_lane);
             if (im.bad_state) {
                 err = "member " + std::to_string(m) + ": " + (im.bad_state_error(), members[m]->err);
                 return HP2D_NUMERICAL;
             }
-            im.dry_for_layout(cells_per_lane);   // the ensemble's layout may differ from the member's
             HP_CK(cudaStreamSynchronize(im.st()));
             host[m] = im.fused_args(cells_per_lane);
         }
