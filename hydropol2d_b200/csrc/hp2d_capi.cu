@@ -394,17 +394,23 @@ template <typename R> struct Impl : Base {
     int tile_rpt() const {
         if (wait_polls != kWaitPolls) return 0;   // the caller bounds the row copies that strips have
         if (tile_mode >= 0) return tile_mode;
-        // Up to where the tiles measured faster than the strips, us per step, strips / tiles.  FP32:
-        // 1000^2 41 / 25 wet, 38 / 19 valley, 86 / 43 Green-Ampt and rain maps; 1300^2 44 / 43, 41 / 28,
-        // 93 / 68; 1500^2 44 / 53, 42 / 35, 101 / 90; 1700^2 58 / 81, 57 / 51, 139 / 113; 2048^2 180 / 169
-        // with Green-Ampt and maps.  FP64: 1700^2 Green-Ampt and maps 255 / 234, wet 161 / 141.
-        const size_t most = sizeof(R) == 8 ? 4000000 : (inf_mode() || rain.n_maps) ? 4300000 : 2500000;
+        // Up to where the tiles are the faster form, us per step, strips / tiles of two rows, on square grids.
+        // FP32 with soil and rain maps 2048^2 180 / 163, 2300^2 222 / 193, 2600^2 319 / 244 (larger ones were
+        // not measured); with one of the two 1600^2 101 / 86 soil and 103 / 82 maps, 1800^2 101 / 110 and
+        // 103 / 106 wet but 91 / 77 and 101 / 92 in a partly dry valley, 2048^2 125 / 147, 134 / 167, 116 / 123
+        // and 132 / 159; with neither the wet grid turns first (1300^2 43 / 41, 1450^2 46 / 55, 1600^2 63 / 69,
+        // 1800^2 58 / 77), the valley last (43 / 36, 57 / 42, 57 / 51 at the latter three, 2048^2 73 / 93), and at
+        // the limit their differences are about equal.  FP64 2000^2 274 / 193 wet, 166 / 125 valley, 433 / 316
+        // soil and maps; 2300^2 296 / 271, 165 / 156, 455 / 409; 2600^2 399 / 318, 173 / 195, 601 / 516.  Long
+        // and flat grids of as many cells turn alike (FP32 250 x 8000 wet 45 / 55, soil and maps 98 / 83).
+        const bool soil = inf_mode() != 0, maps_on = rain.n_maps > 0;
+        const size_t most = sizeof(R) == 8 ? 5400000 : soil && maps_on ? 6800000 : soil || maps_on ? 3300000 : 2500000;
         if (n > most) return 0;
         return default_tile_rpt();
     }
     // one row per thread while the grid gives the GPU little more than one wave of tiles (256^2 wet
-    // FP32 6.5 / 7.4 us with one / two rows, 450^2 10.2 / 9.9, 700^2 16.7 / 14.5; FP64 Green-Ampt 600^2 43 / 46,
-    // 1000^2 103 / 103)
+    // FP32 6.5 / 7.4 us with one / two rows, 450^2 10.2 / 9.9, 700^2 16.7 / 14.5; FP64 soil and maps 600^2
+    // 43 / 46, 800^2 61 / 63, 1000^2 92 / 93, 1300^2 147 / 138, though wet without them 800^2 44 / 38)
     int default_tile_rpt() const { return n > (sizeof(R) == 8 ? 1000000u : 200000u) ? 2 : 1; }
     bool tile_on() const { return tile_rpt() != 0; }
     cudaGraphExec_t graph = nullptr;
