@@ -488,7 +488,7 @@ template <int BN> __device__ __forceinline__ constexpr uint32_t bf16_idesc_mn() 
 template <int CB, int BN, int SMALL, bool BSMALL>
 __global__ void __launch_bounds__(kPtThreads, 1)
 k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmD, const uint16_t* __restrict__ x,
-        const uint16_t* __restrict__ dy, int Ci, int Co, float* gW, int ldw, int* err, const TileGeom g, int ci_blocks) {
+        const uint16_t* __restrict__ dy, int Ci, int Co, float* gW, int ldw, int* err, const TileGeom g, int ci_blocks, int halves) {
     constexpr int NS = wgrad_stages<CB, BN, SMALL>();
     constexpr int NM = wgrad_mmas<CB, SMALL>();
     constexpr uint32_t kA = wgrad_a<CB, SMALL>(), kB = kBM * BN * 2, kStage = kA + kB;
@@ -504,7 +504,11 @@ k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const int cb = int(blockIdx.y) % ci_blocks, nb = int(blockIdx.y) / ci_blocks;
-    const int n_tiles = int(blockIdx.x) < g.total ? (g.total - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
+    // the CTA's work items: tiles, or half tiles (halves = 2: the product runs over half of the pixels)
+    const int items = g.total * halves;
+    const int n_tiles = int(blockIdx.x) < items ? (items - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
+    const auto item = [&](int i) { return int(blockIdx.x) + i * int(gridDim.x); };
+    const auto tile_of = [&](int i) { return halves == 2 ? item(i) >> 1 : item(i); };
 
     if (warp == 0) tmem_alloc(smem_addr(&s_tmem), kCols);
     if (tid == 0) {
@@ -526,7 +530,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
         if (lane == 0) {
             for (int i = 0; i < n_tiles && !pt_failed(fail); ++i) {
                 int b, y0, x0;
-                g.at(int(blockIdx.x) + i * int(gridDim.x), b, y0, x0);
+                g.at(tile_of(i), b, y0, x0);
                 const int s = i % NS;
                 const uint32_t fb = smem_addr(&bar_full[s]);
                 if (i >= NS && !bar_wait(smem_addr(&bar_empty[s]), uint32_t((i / NS) - 1) & 1u)) {
@@ -564,13 +568,17 @@ k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
                     da[q] = row_desc<CB>(sa + uint32_t(q * kHX) * kRow, kRow, uint32_t(kHX) * kRow);
                 }
             }
+            const int half = item(i) & 1;
+            bool first = i == 0;
 #pragma unroll
             for (int kk = 0; kk < kBM / 16; ++kk) {   // 16 pixels: two rows of the tile
+                if (halves == 2 && kk / (kBM / 32) != half) continue;
                 const uint64_t oa = uint64_t((SMALL ? uint32_t(16 * kk) * 128u : uint32_t(2 * kk * kHX) * kRow) / 16u);
                 const uint64_t ob = uint64_t(uint32_t(16 * kk) * (BN * 2) / 16u);
 #pragma unroll
                 for (int q = 0; q < NM; ++q)
-                    tc_mma_bf16(tmem + uint32_t(q * BN), da[q] + oa, db + ob, idesc, (i | kk) != 0 ? 1u : 0u);
+                    tc_mma_bf16(tmem + uint32_t(q * BN), da[q] + oa, db + ob, idesc, first ? 0u : 1u);
+                first = false;
             }
             tc_commit(smem_addr(&bar_empty[s]));
         }
@@ -580,7 +588,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
         const int m = tid - 64;   // pixel of the tile
         for (int i = 0; i < n_tiles && !pt_failed(fail); ++i) {
             int b, y0, x0;
-            g.at(int(blockIdx.x) + i * int(gridDim.x), b, y0, x0);
+            g.at(tile_of(i), b, y0, x0);
             const int s = i % NS;
             if (i >= NS && !bar_wait(smem_addr(&bar_empty[s]), uint32_t((i / NS) - 1) & 1u)) {
                 *fail = 1;
