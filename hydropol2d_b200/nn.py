@@ -67,6 +67,13 @@ def conv3x3(x: torch.Tensor, w16: torch.Tensor, Co: int, out: torch.Tensor, epil
                              EPI[epilogue], _stream()))
 
 
+def aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t``, or a copy where it is not contiguous from a 16-byte boundary (slices of a batch of small
+    or odd images), as the convolutions read it."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def conv_any_ok(ci: int, co: int, ldw: int) -> bool:
     """Whether ``conv3x3_any`` takes these channel counts (weights of row pitch ``ldw``)."""
     return (ci in (1, 2, 4) and co <= 128 and ldw >= 64) or ci % 32 == 0

@@ -97,7 +97,7 @@ class Conv3x3:
             y = out.as_strided((P, self.co), (out.stride(2), 1))
         epi = "f32_bias" if head else ("bf16_bias_relu" if self.relu else "bf16_bias")
         if nn.conv_any_ok(self.ci, self.co, self.kp):
-            nn.conv3x3_any(x.contiguous(), self.W16, self.co, y, epi, bias=self.b)
+            nn.conv3x3_any(nn.aligned(x), self.W16, self.co, y, epi, bias=self.b)
         else:
             nn.gemm(nn.im2col3x3(x, self.kp), self.W16, y, epi, bias=self.b)
         if keep:
@@ -110,9 +110,11 @@ class Conv3x3:
         B, H, W, _ = x.shape
         P = B * H * W
         dy2 = dy.reshape(P, self.co)
+        if not self.relu:   # nothing is written to dy
+            dy2 = dy2.contiguous()
         nn.relu_colsum(self.y if self.relu else None, dy2, self.gb)
         if nn.wgrad_ok(self.ci, self.co):
-            nn.conv3x3_wgrad(x.contiguous(), dy2.view(B, H, W, self.co), self.gW)
+            nn.conv3x3_wgrad(nn.aligned(x), nn.aligned(dy2).view(B, H, W, self.co), self.gW)
         else:
             dyT = nn.transpose(dy2)
             colsT = nn.im2col3x3(x, self.kp, transpose=True)
@@ -125,7 +127,7 @@ class Conv3x3:
         dx = torch.empty(P, self.ci, dtype=torch.bfloat16, device=x.device)
         dyv = dy2.view(B, H, W, self.co)
         if nn.conv_any_ok(self.co, self.ci, self.kp2):
-            nn.conv3x3_any(dyv, wt, self.ci, dx, "bf16_bias", bias=self.zero_ci)
+            nn.conv3x3_any(nn.aligned(dyv), wt, self.ci, dx, "bf16_bias", bias=self.zero_ci)
         else:
             nn.gemm(nn.im2col3x3(dyv, self.kp2), wt, dx, "bf16_bias", bias=self.zero_ci)
         return dx.view(B, H, W, self.ci)
