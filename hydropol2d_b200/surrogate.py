@@ -63,22 +63,41 @@ def layer_level(name: str) -> int:
     return int(name[3])
 
 
-class Conv3x3:
-    """One 3x3, stride-1, zero-padded convolution (+ bias, optional ReLU)."""
+def parameters(spec, gen: torch.Generator, device):
+    """The parameters of a list of layers (as ``unet_spec`` gives them): weights W (initialised from
+    ``gen``, layer by layer), their gradients gW, moments mW, vW and BF16 copies W16 in one buffer each,
+    the biases b, gb, mb, vb likewise; and per layer the views of them."""
+    shapes = [(co, ceil64(9 * ci)) for _, ci, co, _ in spec]
+    at = [0]
+    for co, kp in shapes:
+        at.append(at[-1] + co * kp)   # multiples of 64 elements
+    W = torch.zeros(at[-1])
+    for (_, ci, co, relu), a, shape in zip(spec, at, shapes):
+        std = math.sqrt((2.0 if relu else 1.0) / (9 * ci))
+        W[a:a + shape[0] * shape[1]].view(shape)[:, :9 * ci] = torch.randn(co, 9 * ci, generator=gen) * std
+    flat = {"W": W.to(device)}
+    flat |= {name: torch.zeros(at[-1], device=device) for name in ("gW", "mW", "vW")}
+    flat["W16"] = nn.to_bf16(flat["W"])
+    bat = [0]
+    for co, _ in shapes:
+        bat.append(bat[-1] + ceil64(co))
+    flat |= {name: torch.zeros(bat[-1], device=device) for name in ("b", "gb", "mb", "vb")}
+    views = [{name: t[b:b + shape[0]] if name.endswith("b") else t[a:a + shape[0] * shape[1]].view(shape)
+              for name, t in flat.items()} for a, b, shape in zip(at, bat, shapes)]
+    return flat, views
 
-    def __init__(self, name, ci, co, relu, gen: torch.Generator, device):
+
+class Conv3x3:
+    """One 3x3, stride-1, zero-padded convolution (+ bias, optional ReLU).  ``views``: its parameters,
+    where a network holds them (``parameters``)."""
+
+    def __init__(self, name, ci, co, relu, gen: torch.Generator, device, views: dict | None = None):
         self.name, self.ci, self.co, self.relu = name, ci, co, relu
         self.kp, self.kp2 = ceil64(9 * ci), ceil64(9 * co)
-        std = math.sqrt((2.0 if relu else 1.0) / (9 * ci))
-        W = torch.zeros(co, self.kp)
-        W[:, :9 * ci] = torch.randn(co, 9 * ci, generator=gen) * std
-        self.W = W.to(device)
-        self.b = torch.zeros(co, device=device)
-        self.gW = torch.zeros_like(self.W)
-        self.gb = torch.zeros_like(self.b)
-        self.mW, self.vW = torch.zeros_like(self.W), torch.zeros_like(self.W)
-        self.mb, self.vb = torch.zeros_like(self.b), torch.zeros_like(self.b)
-        self.W16 = nn.to_bf16(self.W)
+        if views is None:
+            _, (views,) = parameters([(name, ci, co, relu)], gen, device)
+        for key, t in views.items():
+            setattr(self, key, t)
         self.zero_ci = torch.zeros(ci, device=device)
         self.x = self.y = None
 
@@ -143,25 +162,13 @@ class UNet:
         g = torch.Generator().manual_seed(seed)
         self.levels = levels
         self.spec = unet_spec(base, levels, in_ch, out_ch)
-        self.layers = {name: Conv3x3(name, ci, co, relu, g, device) for name, ci, co, relu in self.spec}
-        self.step_count = 0
-        self.loss_buf = torch.zeros(1, device=device)
         # all weights, and all biases, with their gradients and moments, each in one buffer that the
         # layers hold views of: clearing the gradients and Adam are one launch a buffer, not one a
         # layer (72 launches of a 16 x 256^2 step, 0.2 of its 3.3 ms)
-        self._flat = {}
-        for names in (("W", "gW", "mW", "vW", "W16"), ("b", "gb", "mb", "vb")):
-            for name in names:
-                parts = [getattr(c, name) for c in self.layers.values()]
-                sizes = [ceil64(t.numel()) for t in parts]
-                flat = torch.zeros(sum(sizes), dtype=parts[0].dtype, device=device)
-                at = 0
-                for c, t, size in zip(self.layers.values(), parts, sizes):
-                    view = flat[at:at + t.numel()].view(t.shape)
-                    view.copy_(t)
-                    setattr(c, name, view)
-                    at += size
-                self._flat[name] = flat
+        self._flat, views = parameters(self.spec, g, device)
+        self.layers = {layer[0]: Conv3x3(*layer, g, device, v) for layer, v in zip(self.spec, views)}
+        self.step_count = 0
+        self.loss_buf = torch.zeros(1, device=device)
 
     def _one_buffer(self, *names) -> bool:
         """Whether the layers' tensors of these names are (still) the views of their one buffer."""
