@@ -1,9 +1,10 @@
 // Device-side arithmetic of the surface-flow step, shared by the fused and the unfused
 // kernels.  Every function here is the per-cell or per-face form of a reference line:
-//   face_flux      Local_Inertial_Model_D4.m:31-44, :89-142 (split slope), :198,
+//   face_geom, face_momentum and their paired form faces_open, faces_update
+//                  Local_Inertial_Model_D4.m:31-44, :89-142 (split slope), :198,
 //                  Inertial_Solver.m:24-25, LIM_D4.m:264, :272-275, :292-294
-//   donor_scale    apply_coarse_draining_limiter, LIM_D4.m:814-829
-//   limit_face     LIM_D4.m:831-857
+//   donor_scale_finite, donor_out    apply_coarse_draining_limiter, LIM_D4.m:814-829
+//   limit_face_finite, limit_by      LIM_D4.m:831-857
 //   continuity     LIM_D4.m:313-315, :389-393, :415
 //   outlet_sink    LIM_D4.m:417-498
 //   green_ampt     HydroPol2D_Main_While_Ensemble.m:274-298 with Infiltration_Module.m
@@ -160,7 +161,6 @@ struct StepScalars {
     int pad2;
     double inflow_vol;     // cumulative inflow-hydrograph volume [m^3]
     double stage_vol;      // cumulative volume the stage overwrites added [m^3]
-    double acc_stage;      // step sum [m] (times cell area later)
     // map records (save_output_maps.m:25-27, :160-166): index of the last record time below
     // t_save, records taken, and whether the next step's input depth is to be recorded
     long long rec_count;
@@ -739,7 +739,7 @@ __device__ __forceinline__ R vg_infiltration(R& hh, R& Ic, R zwt, const SoilClas
     return fd;
 }
 
-// momentum term of schemes 2 and 3 for a face with Hf > 0 (see face_flux)
+// momentum term of schemes 2 and 3 for a face with Hf > 0 (see face_geom)
 template <typename R>
 __device__ __forceinline__ R diffused_momentum(R qp, R q_lo, R q_hi, R Hf, const StepConsts<R>& K, int scheme) {
     const R th = R(1) - K.dt_over_dx * fmin(qdiv(fabs(qp), Hf), sqrt(K.g * Hf));
@@ -755,8 +755,6 @@ __device__ __forceinline__ R diffused_momentum(R qp, R q_lo, R q_hi, R Hf, const
 // domain (idx_nan, NaN elevation).  There MATLAB's max ignores the NaN, so the face depth
 // is the inside cell's depth (:133-134) while the NaN slope sends q to 0 (:264); that
 // depth still enters the wave celerity of refreshing_timestep.
-// Faces that carry no water leave early: whole warps of them skip the power and the
-// division, which matters on wet/dry fronts.
 //
 // SCH = 0: Bates (flag_numerical_scheme 1, Inertial_Solver.m:23-26).  SCH = 1: the schemes
 // with numerical diffusion chosen at run time by `scheme` (Inertial_Solver.m:29-121): the
@@ -769,48 +767,11 @@ __device__ __forceinline__ R diffused_momentum(R qp, R q_lo, R q_hi, R Hf, const
 // (x: columns j-1, j+1; y: rows i-1, i+1), zero on the first and last column (x) or row
 // (y), as the reference's interior ranges 2:(end-1) leave them.  The friction term keeps
 // |q_p| (total_flux = q_p, :31, :101).
-template <typename R, bool IS_X, int SCH = 0>
-__device__ __forceinline__ void face_flux(R ha, R hb, R dz, R qp, R n2c, const StepConsts<R>& K,
-                                          int flag_critical, R& Hf, R& q, int scheme = 1, R q_lo = R(0),
-                                          R q_hi = R(0)) {
-    if (!(fabs(dz) <= R(3.0e38))) {
-        // NaN dz: MATLAB's max over the two sides skips the NaN one
-        Hf = isnan(dz) ? fmax(fmax(ha, hb), R(0)) : R(0);
-        q = R(0);
-        return;
-    }
-    ha = fmax(ha, R(0));
-    hb = fmax(hb, R(0));
-    R S;
-    if (IS_X) {
-        Hf = fmax(fmax(ha - fmax(dz, R(0)), hb + fmin(dz, R(0))), R(0));
-        S = (dz + (hb - ha)) * K.inv_dx;
-    } else {
-        Hf = fmax(fmax(ha + fmin(dz, R(0)), hb - fmax(dz, R(0))), R(0));
-        S = (dz + (ha - hb)) * K.inv_dx;
-    }
-    if (!(Hf > R(0))) { q = R(0); return; }
-    R qn = qp;
-    if (SCH) qn = diffused_momentum(qp, q_lo, q_hi, Hf, K, scheme);
-    R num = fma(-(K.gdt * Hf), S, qn);   // one rounding for qn - (g dt Hf) S
-    R h73 = pow73_pos(Hf);
-    R den = fma(K.gdt * n2c, fabs(qp), h73);
-    R qq = qdiv(num * h73, den);
-    if (!isfinite(qq)) qq = R(0);
-    if (flag_critical == 1) {
-        R crit = Hf * sqrt(K.g * Hf);
-        qq = fmin(fmax(qq, -crit), crit);
-    }
-    R thr = Hf * R(10);
-    q = fmin(fmax(qq, -thr), thr);
-}
-
-// face_flux split in two for the fused kernel's interleaved faces: face_geom gives the face
-// depth Hf, the slope S and whether the face carries water (open and Hf > 0); face_momentum is
-// the update of a wet face, written without branches so that the independent faces of a row
-// (two directions, CPL cells per lane) can be interleaved.  For a wet face the two together
-// perform the same operations on the same values as face_flux; a face that is not wet is given
-// q = 0 (its momentum is evaluated on harmless operands and discarded).
+//
+// In two parts, so that the independent faces of a row can be interleaved: face_geom gives the face
+// depth Hf, the slope S and whether the face carries water (open and Hf > 0); face_momentum is the
+// update of a wet face without branches (a face that is not wet is given q = 0: its momentum is
+// evaluated on harmless operands and discarded).
 template <typename R, bool IS_X>
 __device__ __forceinline__ bool face_geom(R ha, R hb, R dz, R& Hf, R& S, const StepConsts<R>& K) {
     const bool open = fabs(dz) <= R(3.0e38);
@@ -854,8 +815,9 @@ __device__ __forceinline__ R face_momentum(bool wet, R Hf, R S, R qp, R n2c, con
 // open and wet needs no flag of its own (faces_open, faces_update); the grid's edges and face depths
 // below the smallest normal number are left to branches that whole warps skip.  The latter need the
 // depths' clamp to be off: between depths that are 0 or at least 1e-9, a positive face depth is a
-// difference of numbers that size, at least their last place.  Every face and cell gets the bits of face_flux,
-// donor_scale, limit_face and cfl_cell (up to the sign of a zero).
+// difference of numbers that size, at least their last place.  Every face and cell gets the bits of
+// face_geom and face_momentum, donor_scale_finite, limit_face_finite and cfl_cell (up to the sign of a
+// zero).
 //
 // faces_open (below): the depths and slopes of a cell's two faces, whose dz is finite or NaN.  A NaN dz
 // (next to an idx_nan cell) takes part in no minimum or maximum, which leaves the inside cell's depth, as
@@ -981,7 +943,7 @@ __device__ __forceinline__ void faces_update(R Hx, R Hy, Two<R> h73, Two<R> S, R
     qy = oky ? fmin(fmax(vy, -ty), ty) : R(0);
 }
 // what leaves a cell and what it holds, as rates: its faces are limited when the first exceeds the
-// second (donor_scale)
+// second (donor_scale_finite)
 template <typename R> __device__ __forceinline__ R donor_out(R qR, R qL, R qU, R qD) {
     R out = fmax(qR, R(0));
     out = out + fmax(-qL, R(0));
@@ -1007,23 +969,9 @@ __device__ __forceinline__ void face_velocities_neg(double qa, double ha, double
     vb = -face_velocity(qb, hb, K);
 }
 
-// outgoing rate of a cell over its four faces and its donor scale factor
-template <typename R>
-__device__ __forceinline__ R donor_scale(R qR, R qL, R qU, R qD, R hc, const StepConsts<R>& K) {
-    R out = fmax(qR, R(0));
-    out = out + fmax(-qL, R(0));
-    out = out + fmax(qU, R(0));
-    out = out + fmax(-qD, R(0));
-    R avail = fmax(hc, R(0)) * K.dx_over_dt;
-    R s = R(1);
-    if (out > avail && out > R(0)) s = avail / out;
-    if (!isfinite(s)) s = R(0);
-    return fmax(fmin(s, R(1)), R(0));
-}
-
-// donor_scale without the checks that cannot fire when the four faces are finite:
-// avail >= 0, so out > avail implies out > 0 and 0 <= avail/out <= 1 (a finite value
-// that the clamps and the NaN test of donor_scale leave unchanged)
+// outgoing rate of a cell over its four finite faces and its donor scale factor: avail >= 0, so
+// out > avail implies out > 0 and 0 <= avail / out <= 1 (the reference's clamps and its NaN test
+// leave that unchanged)
 template <typename R>
 __device__ __forceinline__ R donor_scale_finite(R qR, R qL, R qU, R qD, R hc, const StepConsts<R>& K) {
     R out = fmax(qR, R(0));
@@ -1033,19 +981,11 @@ __device__ __forceinline__ R donor_scale_finite(R qR, R qL, R qU, R qD, R hc, co
     const R avail = fmax(hc, R(0)) * K.dx_over_dt;
     return out > avail ? avail / out : R(1);
 }
-// limit_face for a finite q and scales in [0, 1] (the product is finite)
+// a finite face limited by the scale of its donor cell, s_pos = donor when q > 0; scales in [0, 1]
+// (the product is finite)
 template <typename R>
 __device__ __forceinline__ R limit_face_finite(R q, R s_pos, R s_neg) {
     return q > R(0) ? q * s_pos : (q < R(0) ? q * s_neg : q);
-}
-
-// face limited by the scale of its donor cell; s_pos = donor when q > 0
-template <typename R>
-__device__ __forceinline__ R limit_face(R q, R s_pos, R s_neg) {
-    if (q > R(0)) q = q * s_pos;
-    else if (q < R(0)) q = q * s_neg;
-    if (!isfinite(q)) q = R(0);
-    return q;
 }
 
 template <typename R>

@@ -42,7 +42,6 @@
 
 namespace hp2d {
 
-constexpr int kStripOut = 28;   // output columns of a 32-lane strip (lanes 2..29)
 #ifndef HP2D_STAGES
 #define HP2D_STAGES 4
 #endif
@@ -51,19 +50,16 @@ constexpr int kStages = HP2D_STAGES;   // shared-memory ring depth of the row pi
 #define HP2D_ROW_UNROLL 1
 #endif
 constexpr int kRowUnroll = HP2D_ROW_UNROLL;   // row-loop unroll (register renaming of the window)
-// The faces of a row are interleaved, branch-free momentum updates (face_open + face_update)
-// rather than one face_flux after the other: measured faster on every workload (wet 2048^2 40.2
-// vs 39.1 GCUPS, 60-minute dam-break 98.3 vs 96.3, Green-Ampt + rain maps 21.4 vs 21.0).
 // Phase (F) without a per-lane branch around each cell's body (stores and reductions masked
-// instead), so that the CPL cells interleave: wet 2048^2 41.6 vs 40.8 GCUPS, 60-minute dam-break
-// 115.5 vs 111.8, 128-member ensemble 44.6 vs 43.0; the Green-Ampt + rain-map instantiation ran
-// 20.3 vs 21.2 with it and keeps the branch.
-// What a row of wet cells costs is its instructions (64 % of the issue slots, DRAM at 40 %), so what
-// only some rows need is decided once per row by a vote: the grid's edges, outlet and gauge cells,
-// arrivals, dry flags.  A lane's two cells are neighbours (one shuffle an exchange), columns and rows
-// outside the grid are records whose faces are closed, and no face carries a flag (wet 2048^2: 64.8 M
-// to 53.9 M warp instructions, 94 to 77 us a step; 4096 x 8192 valley 45.0 to 39.0 ms; 48 members 23.3
-// to 19.4 ms; urban 2048^2 15.0 to 14.4 ms).
+// instead), so that the CPL cells interleave: 3 % faster on the plain instantiations (60-minute
+// dam-break 115.5 vs 111.8 GCUPS when it was introduced); the Green-Ampt + rain-map instantiation,
+// at its register cap, ran 20.3 vs 21.2 with it and keeps the branch.
+// What a row of wet cells costs is its instructions (wet 2048^2, 73 us a step: 61 % of the issue
+// slots, 11.6 warp instructions a cell, DRAM at 40 %), so what only some rows need is
+// decided once per row by a vote: the grid's edges, outlet and gauge cells, arrivals, dry flags.  A
+// lane's two cells are neighbours (one shuffle an exchange), columns and rows outside the grid are
+// records whose faces are closed, no face carries a flag, and a cell's two faces share one FP32x2
+// instruction (faces_open, faces_update).
 template <int INF, bool MAP> constexpr bool kFlatF = INF == 0 && !MAP;
 
 // dynamic shared memory of k_fused_step: per warp kStages x (2 records x 32*CPL cells)
@@ -735,7 +731,6 @@ __device__ __forceinline__ bool fused_item(const FusedArgs<R>& a, const unsigned
     V2* __restrict__ gout = cur ? a.gs0 : a.gs1;
     const V4* __restrict__ stat = a.stat;
     const R t_arr = R(sh.now.t_min * 60.0 + sh.now.dts);
-    const R NaNR = R(__int_as_float(0x7fc00000));
 
     const int lane = tid & 31, warp = tid >> 5;
     const int wg = int(blk) * (NT / 32) + warp;

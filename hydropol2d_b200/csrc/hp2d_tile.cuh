@@ -12,8 +12,8 @@
 // same bit for bit.
 //
 // Why: a strip's warp takes about 2.4 us per row (one warp's dependent chain of ~1000
-// instructions), so a small grid is bound by rows per warp, not by work: 256 x 256 FP32 ran at
-// 49 us and 200 x 200 FP64 at 169 us per step.
+// instructions), so a small grid of strips is bound by rows per warp, not by work: us per step,
+// strips / tiles, 200 x 200 FP64 155 / 7.7, 512 x 512 FP32 46 / 10, 1000 x 1000 wet FP32 43 / 29.
 //
 // Dry tiles: a flag per tile and state buffer records that the tile's whole output was written as
 // dry records there.  A tile whose depths are all zero after (A), two-cell apron included, and
