@@ -271,26 +271,31 @@ hp2d_status wgrad(const uint16_t* x, int B, int H, int W, int Ci, const uint16_t
     const int ci_blocks = SMALL ? 1 : Ci / CB, units = ci_blocks * ((Co + BN - 1) / BN);
     // A unit's tiles are split over the SMs, each part adds its sums into gW once.  The tensor core
     // truncates its sums, so an accumulator's error grows with its chain (2^-24 of it a step of 16 pixels),
-    // and every part's addition rounds once more.  So the parts follow those of the split-K GEMM over
-    // pixels that this replaces (296 parts over its 128 x 256 output tiles, in k tiles of 64 pixels): none
-    // holds more pixels; short ones hold as many, in half tiles where whole ones do not divide them; longer
-    // ones become shorter where that fills whole waves.  gW's distance from 64 bits (RMS) over that GEMM's,
-    // all layers at 16 x 256^2, 16 x 128^2, 4 x 128^2 and 8 x 224 x 160: 0.4 to 1.03; with the parts by the
-    // SMs alone up to 1.98 (16 x 128^2, 4 -> 32 channels), though 8 us less where this takes a second wave
-    // (16 x 256^2, 128 -> 128 at a quarter of the resolution 38 us for 30).
+    // and every part's addition rounds once more.  So no part is longer than those of the split-K GEMM over
+    // pixels that this replaces (296 parts over its 128 x 256 output tiles, in k tiles of 64 pixels): long
+    // ones fill the SMs once, or the number of the GEMM's parts, or else as many waves as keep them short
+    // enough; short ones are the GEMM's, in half tiles where whole ones do not divide them.  gW's distance
+    // from 64 bits (RMS) over that GEMM's, all layers at 16 x 256^2, 16 x 128^2, 4 x 128^2 and
+    // 8 x 224 x 160: 0.6 to 1.03 (the two-channel layer 1.08); with the parts by the SMs alone up to 1.98
+    // (16 x 128^2, 4 -> 32 channels), though 8 us less where this takes a second wave (16 x 256^2,
+    // 128 -> 128 at a quarter of the resolution 38 us for 30).
     const int kp = (9 * Ci + 63) / 64 * 64;
     const int gemm_tiles = ((Co + 127) / 128) * (kp > 128 ? (kp + 255) / 256 : 1);
     const int64_t P = int64_t(B) * H * W;
-    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(P / 64, 2 * n / gemm_tiles));
-    const int64_t k_tiles = ((P + 63) / 64 + parts - 1) / parts;   // of a part of the GEMM
+    const int64_t gemm_parts = std::max<int64_t>(1, std::min<int64_t>(P / 64, 2 * n / gemm_tiles));
+    const int64_t k_tiles = ((P + 63) / 64 + gemm_parts - 1) / gemm_parts;   // of a part of the GEMM
     const bool is_short = k_tiles < 8;
     const int halves = is_short && k_tiles % 2 ? 2 : 1;
     // P / items pixels each, on average: ragged images pad their tiles, and a part takes a fifth more then
     const int64_t items = int64_t(g.total) * halves;
     const int64_t most = std::max<int64_t>(1, std::min(k_tiles * 64 * items / P, k_tiles * halves * 3 / 5));
-    const int64_t wave = is_short ? 1 : std::max(1, n / units);
-    const int64_t need = (items + most - 1) / most;
-    const int splits = int(std::min(items, (need + wave - 1) / wave * wave));
+    const int64_t need = (items + most - 1) / most, wave = std::max(1, n / units);
+    int64_t parts = need;
+    if (!is_short) {
+        parts = P > wave * 128 * 16 ? std::max(1, 2 * n / gemm_tiles) : wave;
+        if ((items + parts - 1) / parts * 2 > k_tiles + 1) parts = (need + wave - 1) / wave * wave;
+    }
+    const int splits = int(std::min(items, parts));
     k_wgrad<CB, BN, SMALL, BSMALL><<<dim3(splits, units), kPtThreads, smem, st>>>(mx, md, x, dy, Ci, Co, gW, ldw, err, g,
                                                                                  ci_blocks, halves);
     return launched("k_wgrad");
@@ -298,7 +303,8 @@ hp2d_status wgrad(const uint16_t* x, int B, int H, int W, int Ci, const uint16_t
 template <int CB, int SMALL>
 hp2d_status wgrad_n(const uint16_t* x, int B, int H, int W, int Ci, const uint16_t* dy, int Co, float* gW, int ldw, int* err,
                     cudaStream_t st) {
-    // 64 -> 32 channels as two units of 32: their 2 x 148 parts at full resolution fill the GPU two to an SM
+    // 64 -> 32 channels as two units of 32: their 2 x 98 parts at full resolution fill the GPU two to an
+    // SM, where 98 parts of 64 channels left a third of it idle
     if constexpr (CB == 64 && SMALL == 0)
         if (Ci == 64 && Co == 32) return wgrad<32, 32, 0, false>(x, B, H, W, Ci, dy, Co, gW, ldw, err, st);
     if (Co % 64 == 0) return wgrad<CB, 64, SMALL, false>(x, B, H, W, Ci, dy, Co, gW, ldw, err, st);
