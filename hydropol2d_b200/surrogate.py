@@ -63,27 +63,29 @@ def layer_level(name: str) -> int:
     return int(name[3])
 
 
+def initial_weight(ci: int, co: int, relu: bool, gen: torch.Generator) -> torch.Tensor:
+    """A layer's weights [co, 9 ci] on the host: normal, He's scale with the ReLU."""
+    return torch.randn(co, 9 * ci, generator=gen) * math.sqrt((2.0 if relu else 1.0) / (9 * ci))
+
+
 def parameters(spec, gen: torch.Generator, device):
-    """The parameters of a list of layers (as ``unet_spec`` gives them): weights W (initialised from
+    """The parameters of a network's layers (as ``unet_spec`` gives them): weights W (initialised from
     ``gen``, layer by layer), their gradients gW, moments mW, vW and BF16 copies W16 in one buffer each,
     the biases b, gb, mb, vb likewise; and per layer the views of them."""
     shapes = [(co, ceil64(9 * ci)) for _, ci, co, _ in spec]
-    at = [0]
-    for co, kp in shapes:
-        at.append(at[-1] + co * kp)   # multiples of 64 elements
-    W = torch.zeros(at[-1])
-    for (_, ci, co, relu), a, shape in zip(spec, at, shapes):
-        std = math.sqrt((2.0 if relu else 1.0) / (9 * ci))
-        W[a:a + shape[0] * shape[1]].view(shape)[:, :9 * ci] = torch.randn(co, 9 * ci, generator=gen) * std
+    sizes, bsizes = [co * kp for co, kp in shapes], [ceil64(co) for co, _ in shapes]   # multiples of 64 elements
+    W = torch.zeros(sum(sizes))
+    for (_, ci, co, relu), part, shape in zip(spec, W.split(sizes), shapes):
+        part.view(shape)[:, :9 * ci] = initial_weight(ci, co, relu, gen)
     flat = {"W": W.to(device)}
-    flat |= {name: torch.zeros(at[-1], device=device) for name in ("gW", "mW", "vW")}
+    flat |= {name: torch.zeros(sum(sizes), device=device) for name in ("gW", "mW", "vW")}
     flat["W16"] = nn.to_bf16(flat["W"])
-    bat = [0]
-    for co, _ in shapes:
-        bat.append(bat[-1] + ceil64(co))
-    flat |= {name: torch.zeros(bat[-1], device=device) for name in ("b", "gb", "mb", "vb")}
-    views = [{name: t[b:b + shape[0]] if name.endswith("b") else t[a:a + shape[0] * shape[1]].view(shape)
-              for name, t in flat.items()} for a, b, shape in zip(at, bat, shapes)]
+    flat |= {name: torch.zeros(sum(bsizes), device=device) for name in ("b", "gb", "mb", "vb")}
+    views = [{} for _ in spec]
+    for name, t in flat.items():
+        bias = name.endswith("b")
+        for v, part, shape in zip(views, t.split(bsizes if bias else sizes), shapes):
+            v[name] = part[:shape[0]] if bias else part.view(shape)
     return flat, views
 
 
@@ -95,9 +97,16 @@ class Conv3x3:
         self.name, self.ci, self.co, self.relu = name, ci, co, relu
         self.kp, self.kp2 = ceil64(9 * ci), ceil64(9 * co)
         if views is None:
-            _, (views,) = parameters([(name, ci, co, relu)], gen, device)
-        for key, t in views.items():
-            setattr(self, key, t)
+            W = torch.zeros(co, self.kp)
+            W[:, :9 * ci] = initial_weight(ci, co, relu, gen)
+            self.W = W.to(device)
+            self.b = torch.zeros(co, device=device)
+            self.gW, self.mW, self.vW = (torch.zeros_like(self.W) for _ in range(3))
+            self.gb, self.mb, self.vb = (torch.zeros_like(self.b) for _ in range(3))
+            self.W16 = nn.to_bf16(self.W)
+        else:
+            for key, t in views.items():
+                setattr(self, key, t)
         self.zero_ci = torch.zeros(ci, device=device)
         self.x = self.y = None
 
